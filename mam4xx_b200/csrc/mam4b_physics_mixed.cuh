@@ -260,36 +260,28 @@ __device__ __forceinline__ double rcp(double d) {
 }
 }  // namespace mx
 
+// Skipped modes are cleared before the first pass (soa_clear_skipped), so a
+// pass has no branch per mode.
 __device__ __forceinline__ bool soa_step_mx(SoaState &st) {
-  if (!(st.tcur < st.dtfull - 1.0e-3))
+  if (!soa_more(st))
     return false;
-  st.niter++;
-  if (st.niter > 1000)
-    return false;
-  double g_soa = dmax(st.g, 0.0);
-  double tot_soa = g_soa;
-  double a_soa[NMODE], sat[NMODE], g_star[NMODE];
-  bool skip[NMODE];
+  const double g = dmax(st.g, 0.0);
+  double tot = g, a[NMODE], sat[NMODE], g_star[NMODE], tmpb = 0.0;
 #pragma unroll
   for (int n = 0; n < NMODE; ++n) {
-    skip[n] = !(st.uptk[n] > 1.0e-15);
-    a_soa[n] = skip[n] ? 0.0 : dmax(st.a[n], 0.0);
-    tot_soa += a_soa[n];
-  }
-  double tmpb = 0.0;
-#pragma unroll
-  for (int n = 0; n < NMODE; ++n) {
-    if (skip[n])
-      continue;
+    a[n] = dmax(st.a[n], 0.0);
+    tot += a[n];
     // both denominators are at least 1e-20: normal numbers
-    sat[n] = st.g0 * mx::rcp(dmax(st.opoa[n] + a_soa[n], 1.0e-20));
-    g_star[n] = sat[n] * a_soa[n];
-    const double phi = (g_soa - g_star[n]) * mx::rcp(dmax(g_soa, dmax(g_star[n], 1.0e-20)));
+    sat[n] = st.g0 * mx::rcp(dmax(st.opoa[n] + a[n], 1.0e-20));
+    g_star[n] = sat[n] * a[n];
+  }
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    const double phi = (g - g_star[n]) * mx::rcp(dmax(g, dmax(g_star[n], 1.0e-20)));
     tmpb = __fma_rn(st.uptk[n], fabs(phi), tmpb);
   }
-  const double tmpa = dmax(0.0, tmpb);
+  const double tmpa = dmax(0.0, tmpb), dtmax = st.dtfull - st.tcur;
   double dtcur;
-  const double dtmax = st.dtfull - st.tcur;
   if (dtmax * tmpa <= 0.05) {
     dtcur = dtmax;
     st.tcur = st.dtfull;
@@ -301,22 +293,19 @@ __device__ __forceinline__ bool soa_step_mx(SoaState &st) {
   double beta[NMODE], r[NMODE], ta = 0.0, tb = 0.0;
 #pragma unroll
   for (int n = 0; n < NMODE; ++n) {
-    if (skip[n])
-      continue;
     beta[n] = dtcur * st.uptk[n];
-    const double del_g = g_soa - g_star[n];
-    if (del_g > 0.0)
-      sat[n] = st.g0 * mx::rcp(dmax(st.opoa[n] + __fma_rn(beta[n], del_g, a_soa[n]), 1.0e-20));
+    const double del_g = g - g_star[n];
+    const double s2 =
+        st.g0 * mx::rcp(dmax(st.opoa[n] + __fma_rn(beta[n], del_g, a[n]), 1.0e-20));
     // 1 + beta sat >= 1
-    r[n] = mx::rcp(__fma_rn(beta[n], sat[n], 1.0));
-    ta = __fma_rn(a_soa[n], r[n], ta);
+    r[n] = mx::rcp(__fma_rn(beta[n], del_g > 0.0 ? s2 : sat[n], 1.0));
+    ta = __fma_rn(a[n], r[n], ta);
     tb = __fma_rn(beta[n], r[n], tb);
   }
-  g_soa = dmax(0.0, (tot_soa - ta) * mx::rcp(1.0 + tb));
+  st.g = dmax(0.0, (tot - ta) * mx::rcp(1.0 + tb));
 #pragma unroll
   for (int n = 0; n < NMODE; ++n)
-    st.a[n] = skip[n] ? 0.0 : __fma_rn(beta[n], g_soa, a_soa[n]) * r[n];
-  st.g = g_soa;
+    st.a[n] = __fma_rn(beta[n], st.g, a[n]) * r[n];
   return true;
 }
 

@@ -63,6 +63,9 @@ struct StepArgs {
   unsigned *counters;
   int *npass;        // [ncell] or null: passes of each slot's loop (adjoint only)
   int mixed;         // the mode/pair stages ran in FP32 (MAM4B_MIXED, _FAST)
+  double long_steps;    // a loop is long (soa_kernel runs it first) when its
+                        // first sub-step is shorter than dt / long_steps
+  int quads;            // long loops run four lanes to a loop (soa_long_loops)
   double inline_scale;  // pre_kernel<.., FUSE>: cells whose first SOA sub-step
                         // is at least 1/inline_scale of the step finish in pre
 };
@@ -83,14 +86,10 @@ enum { SOA_G = 0, SOA_A = 1, SOA_OPOA = 5, SOA_UPTK = 9, SOA_G0 = 13, SOA_FIELDS
 // per-particle H2SO4 uptake rate of each mode
 // and the 12 coagulation coefficients (coag_all_coefs order)
 enum { AUX_RH = 0, AUX_GDIFF = 1, AUX_FPATH = 2, AUX_RATE = 3, AUX_COAG = 7, AUX_FIELDS = 19 };
-// queue counters: queued slots, slots handed to the solver, long and short
-// loops in the order list
+// queue counters: queued slots, long and short loops in the order list,
+// short and long loops handed to the solver
 enum { CNT_QUEUED = 0, CNT_TAKEN = 1, CNT_LONG = 2, CNT_SHORT = 3, CNT_TAKEN_ADJ = 4,
-       CNT_WORDS = 8 };
-// A loop is started early when its first sub-step is shorter than
-// dt / kLongLoopSteps, i.e. when it is expected to take at least about that
-// many sub-steps (the SOA loop's step is 0.05 / sum(uptake * |phi|)).
-constexpr double kLongLoopSteps = 300.0;
+       CNT_TAKEN_LONG = 5, CNT_WORDS = 8 };
 
 // ----------------------------------------------------- per-cell amicphys
 struct Diag {
@@ -1054,7 +1053,7 @@ struct FinishRegs {
   __device__ double soag() const { return soag_; }
 };
 template <int SOA, class State>
-__device__ __forceinline__ bool soa_pass(State &st);
+__device__ __forceinline__ bool soa_pass(State &st, bool fast);
 
 template <bool CHEM, bool MIXED = false, bool FUSE = false>
 __device__ __forceinline__ void cell_pre(const StepArgs &a, const ChemArgs &ch,
@@ -1122,7 +1121,8 @@ __device__ __forceinline__ void cell_pre(const StepArgs &a, const ChemArgs &ch,
     // runs here and the cell finishes without the hand-off, with the same
     // arithmetic as the solver and post kernels
     if (first_rate <= 0.05 * a.inline_scale) {
-      while (soa_pass<MIXED ? 1 : 0>(st)) {
+      const bool fast = soa_begin(st);
+      while (soa_pass<MIXED ? 1 : 0>(st, fast)) {
       }
       if (st.niter > 1000)
         atomicOr(a.flags, MAM4B_FLAG_SOA_NITER_LIMIT);
@@ -1136,7 +1136,7 @@ __device__ __forceinline__ void cell_pre(const StepArgs &a, const ChemArgs &ch,
       return;
     }
   }
-  const bool long_loop = first_rate > 0.05 * kLongLoopSteps;
+  const bool long_loop = first_rate > 0.05 * a.long_steps;
   // warp-aggregated appends: the slot (in discovery order, which keeps the
   // post kernel's cell accesses coalesced) and the solver order entry
   const unsigned m = __activemask();
@@ -1617,39 +1617,272 @@ __global__ void __maxnreg__(R) post_kernel(const __grid_constant__ StepArgs a) {
   }
 }
 
-// SOA sub-stepping of the queued cells. Persistent warps; every lane owns
-// one cell's loop and, as soon as that loop ends, takes the next queued
-// cell (one atomic per warp for all lanes that need work), so a warp never
-// idles behind one cell that needs hundreds of sub-steps. Cells are taken
-// long loops first, so that the last ones handed out are short. The loop
-// is bound by FP64 division latency: 4 blocks of 256 per SM (64 registers)
-// hide more of it than the unconstrained 93-register build.
-// With MIXED the loop runs in single precision (f32::soa_step).
-// Launched with any block size that is a multiple of 32 and one grid of
-// persistent blocks (SMs x blocks per SM).
+// SOA sub-stepping of the queued cells.
 constexpr int kSoaBlock = 256;
 template <int SOA, class State>
-__device__ __forceinline__ bool soa_pass(State &st) {
-  if constexpr (SOA == 1)
+__device__ __forceinline__ bool soa_pass(State &st, bool fast) {
+  if constexpr (SOA == 0)
+    return soa_step(st, fast);
+  else if constexpr (SOA == 1)
     return f32::soa_step_mx(st);
   else
-    return soa_step(st);
+    return f32::soa_step(st);
 }
 
+// One loop on four lanes, one mode each (lanes 4 k + mode of a warp): the
+// values of the loop state that belong to a mode are the lane's, the others
+// are the same on the four lanes. A pass is the arithmetic of soa_step
+// (SOA 0), f32::soa_step_mx (1) or f32::soa_step (2), value by value: the
+// sums over the modes are taken by every lane in mode order, a skipped
+// mode adding nothing. What it changes is the length of the chain: a
+// thread that owns a whole loop issues four modes' divisions one after the
+// other, so a loop of 1,000 passes, which nothing else can shorten, takes
+// four times as long.
+template <class T>
+struct SoaQuad {
+  T g, a, opoa, uptk, g0;
+  double tcur, dtfull;
+  int niter;
+};
+template <class T>
+struct ModeVals {
+  T v[NMODE];
+};
+template <class T>
+__device__ __forceinline__ ModeVals<T> of_modes(T x, int base) {
+  ModeVals<T> r;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n)
+    r.v[n] = __shfl_sync(0xffffffffu, x, base + n);
+  return r;
+}
+// The pass itself, by all lanes of a warp together; lanes of loops that
+// have ended (or of no loop) take part with no uptake and no SOA. Skipped
+// modes are cleared (soa_clear_skipped) before the first pass.
+template <bool FAST>
+__device__ __forceinline__ void soa_quad_fp64(SoaQuad<double> &st, int base) {
+  auto quot = [](double x, double y) { return FAST ? quot_in_range(x, y) : x / y; };
+  const double g = dmax(st.g, 0.0), a = dmax(st.a, 0.0);
+  double sat = quot(st.g0, dmax(st.opoa + a, 1.0e-20));
+  const double g_star = sat * a;
+  const double part = st.uptk * fabs(quot(g - g_star, dmax(g, dmax(g_star, 1.0e-20))));
+  const ModeVals<double> all_a = of_modes(a, base), all_part = of_modes(part, base);
+  double tot = g, tmpb = 0.0;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    tot += all_a.v[n];
+    tmpb += all_part.v[n];
+  }
+  const double tmpa = dmax(0.0, tmpb), dtmax = st.dtfull - st.tcur;
+  const bool last = dtmax * tmpa <= 0.05;
+  const double dtcur = last ? dtmax : quot(0.05, tmpa);
+  st.tcur = last ? st.dtfull : st.tcur + dtcur;
+  const double beta = dtcur * st.uptk, del_g = g - g_star;
+  if (del_g > 0.0)
+    sat = quot(st.g0, dmax(st.opoa + (a + beta * del_g), 1.0e-20));
+  const double den = 1.0 + beta * sat;
+  const Divisor d(den);
+  auto over_den = [&](double x) { return FAST ? d.under(x) : x / den; };
+  const ModeVals<double> all_qa = of_modes(over_den(a), base),
+                         all_qb = of_modes(over_den(beta), base);
+  double ta = 0.0, tb = 0.0;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    ta += all_qa.v[n];
+    tb += all_qb.v[n];
+  }
+  st.g = dmax(0.0, quot(tot - ta, 1.0 + tb));
+  st.a = over_den(a + beta * st.g);
+}
+__device__ __noinline__ void soa_quad_exact(SoaQuad<double> &st, int base) {
+  soa_quad_fp64<false>(st, base);
+}
+// fast: the lane's own parameters allow quot_in_range (soa_params_moderate);
+// one form for the whole warp, whose lanes exchange values
+__device__ __forceinline__ void soa_quad_pass(SoaQuad<double> &st, bool fast, int base,
+                                              std::integral_constant<int, 0>) {
+  if (__all_sync(0xffffffffu, fast && zero_or_moderate(st.g) && zero_or_moderate(st.a))) {
+    soa_quad_fp64<true>(st, base);
+  } else {
+    SoaQuad<double> t = st;
+    soa_quad_exact(t, base);
+    st = t;
+  }
+}
+__device__ __forceinline__ void soa_quad_pass(SoaQuad<double> &st, bool, int base,
+                                              std::integral_constant<int, 1>) {
+  const double g = dmax(st.g, 0.0);
+  const double a = dmax(st.a, 0.0), uptk = st.uptk;
+  double sat = st.g0 * f32::mx::rcp(dmax(st.opoa + a, 1.0e-20));
+  const double g_star = sat * a;
+  const double aphi = fabs((g - g_star) * f32::mx::rcp(dmax(g, dmax(g_star, 1.0e-20))));
+  const ModeVals<double> all_a = of_modes(a, base), all_phi = of_modes(aphi, base),
+                         all_u = of_modes(uptk, base);
+  double tot = g, tmpb = 0.0;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    tot += all_a.v[n];
+    tmpb = __fma_rn(all_u.v[n], all_phi.v[n], tmpb);
+  }
+  const double tmpa = dmax(0.0, tmpb);
+  const double dtmax = st.dtfull - st.tcur;
+  double dtcur;
+  if (dtmax * tmpa <= 0.05) {
+    dtcur = dtmax;
+    st.tcur = st.dtfull;
+  } else {
+    dtcur = 0.05 * f32::mx::rcp(tmpa);
+    st.tcur += dtcur;
+  }
+  const double beta = dtcur * uptk, del_g = g - g_star;
+  if (del_g > 0.0)
+    sat = st.g0 * f32::mx::rcp(dmax(st.opoa + __fma_rn(beta, del_g, a), 1.0e-20));
+  const double r = f32::mx::rcp(__fma_rn(beta, sat, 1.0));
+  const ModeVals<double> all_r = of_modes(r, base);
+  double ta = 0.0, tb = 0.0;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    ta = __fma_rn(all_a.v[n], all_r.v[n], ta);
+    tb = __fma_rn(dtcur * all_u.v[n], all_r.v[n], tb);
+  }
+  st.g = dmax(0.0, (tot - ta) * f32::mx::rcp(1.0 + tb));
+  st.a = __fma_rn(beta, st.g, a) * r;
+}
+__device__ __forceinline__ void soa_quad_pass(SoaQuad<float> &st, bool, int base,
+                                              std::integral_constant<int, 2>) {
+  using f32::fmx;
+  const float g = fmx(st.g, 0.0f);
+  const float a = fmx(st.a, 0.0f), uptk = st.uptk;
+  float sat = __fdividef(st.g0, fmx(st.opoa + a, 1.0e-20f));
+  const float g_star = sat * a;
+  const float phi = __fdividef(g - g_star, fmx(g, fmx(g_star, 1.0e-20f)));
+  const ModeVals<float> all_a = of_modes(a, base),
+                        all_part = of_modes(uptk * fabsf(phi), base);
+  float tot = g, tmpb = 0.0f;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    tot += all_a.v[n];
+    tmpb += all_part.v[n];
+  }
+  const double dtmax = st.dtfull - st.tcur;
+  float dtcur;
+  if (dtmax * (double)tmpb <= 0.05) {
+    dtcur = (float)dtmax;
+    st.tcur = st.dtfull;
+  } else {
+    dtcur = __fdividef(0.05f, tmpb);
+    st.tcur += (double)dtcur;
+  }
+  const float beta = dtcur * uptk, del_g = g - g_star;
+  if (del_g > 0.0f)
+    sat = __fdividef(st.g0, fmx(st.opoa + (a + beta * del_g), 1.0e-20f));
+  const float den = __fdividef(1.0f, 1.0f + beta * sat);
+  const ModeVals<float> all_ta = of_modes(a * den, base), all_tb = of_modes(beta * den, base);
+  float ta = 0.0f, tb = 0.0f;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    ta += all_ta.v[n];
+    tb += all_tb.v[n];
+  }
+  st.g = fmx(0.0f, __fdividef(tot - ta, 1.0f + tb));
+  st.a = (a + beta * st.g) * den;
+}
+
+// The long loops of the queue, four lanes to a loop, with work stealing as
+// in soa_kernel (eight loops per warp).
+template <int SOA, class T>
+__device__ __forceinline__ void soa_long_loops(const StepArgs &a) {
+  const unsigned nlong = a.counters[CNT_LONG];
+  const int lane = threadIdx.x & 31, mode = lane & 3, base = lane & ~3;
+  const size_t n = (size_t)a.ncell;
+  SoaQuad<T> st = {};
+  unsigned slot = 0;
+  bool active = false, want = nlong > 0, fast = true;
+  while (true) {
+    const unsigned need = __ballot_sync(0xffffffffu, want);
+    if (need) {
+      const int leader = __ffs(need) - 1;
+      unsigned first = 0;
+      if (lane == leader)
+        first = atomicAdd(&a.counters[CNT_TAKEN_LONG], (unsigned)__popc(need) / 4u);
+      first = __shfl_sync(0xffffffffu, first, leader);
+      if (want) {
+        const unsigned t = first + __popc(need & ((1u << base) - 1)) / 4u;
+        want = false;
+        if (t < nlong) {
+          slot = (unsigned)a.order[t];
+          const double *q = a.soa + slot;
+          st.g = q[SOA_G * n];
+          st.a = q[(SOA_A + mode) * n];
+          st.opoa = q[(SOA_OPOA + mode) * n];
+          st.uptk = q[(SOA_UPTK + mode) * n];
+          st.g0 = q[SOA_G0 * n];
+          st.tcur = 0.0;
+          st.dtfull = (double)(int)(a.dt / 1);
+          st.niter = 0;
+          // a skipped mode takes no part (soa_clear_skipped)
+          if (!(st.uptk > (T)1.0e-15) && 0.0 < st.dtfull - 1.0e-3)
+            st.uptk = st.a = st.opoa = (T)0.0;
+          if constexpr (SOA == 0)
+            fast = zero_or_moderate(st.g0) && st.g0 != 0.0 && zero_or_moderate(st.dtfull) &&
+                   zero_or_moderate(st.opoa) && zero_or_moderate(st.uptk);
+          active = true;
+        }
+      }
+    }
+    if (!__any_sync(0xffffffffu, active))
+      return;
+    // passes until a loop of the warp ends
+    bool more;
+    while (true) {
+      more = active && soa_more(st);
+      if (__any_sync(0xffffffffu, active && !more))
+        break;
+      soa_quad_pass(st, fast, base, std::integral_constant<int, SOA>());
+    }
+    if (active && !more) {
+      double *q = a.soa + slot;
+      if (mode == 0) {
+        q[SOA_G * n] = st.g;
+        if (st.niter > 1000)
+          atomicOr(a.flags, MAM4B_FLAG_SOA_NITER_LIMIT);
+        if (a.npass)
+          a.npass[slot] = st.niter > 1000 ? 1000 : st.niter;
+      }
+      q[(SOA_A + mode) * n] = st.a;
+      active = false;
+      want = true;
+      fast = true;
+      st.g = st.a = st.uptk = (T)0.0;
+    }
+    if (more)
+      --st.niter;  // counted again when this pass runs
+  }
+}
+
+// Persistent warps. The long loops of the queue (StepArgs::long_steps) run
+// first, four lanes to a loop; then every lane owns one short loop and, as
+// soon as that loop ends, takes the next queued cell (one atomic per warp
+// for all lanes that need work), so a warp never idles behind one cell.
 // SOA: 0 the FP64 loop (soa_step), 1 FP64 state with FP32 step control
 // (f32::soa_step_mx, MAM4B_MIXED), 2 the FP32 loop (f32::soa_step,
 // MAM4B_MIXED_FAST).
+// Launched with any block size that is a multiple of 32 and one grid of
+// persistent blocks (SMs x blocks per SM).
 template <int SOA, int R>
 __global__ void __maxnreg__(R) soa_kernel(const __grid_constant__ StepArgs a) {
   constexpr bool F32 = SOA == 2;
+  if (a.quads)
+    soa_long_loops<SOA, typename std::conditional<F32, float, double>::type>(a);
   using State = typename std::conditional<F32, f32::SoaStateF, SoaState>::type;
-  const unsigned ntask = a.counters[CNT_QUEUED];
-  const unsigned nlong = a.counters[CNT_LONG];
+  // the loops left, long ones first
+  const unsigned nlong = a.quads ? 0 : a.counters[CNT_LONG];
+  const unsigned ntask = nlong + a.counters[CNT_SHORT];
   const int lane = threadIdx.x & 31;
   const size_t n = (size_t)a.ncell;
   State st;
   unsigned slot = 0;
-  bool active = false, want = true;
+  bool active = false, want = true, fast = false;
   while (true) {
     const unsigned need = __ballot_sync(0xffffffffu, want);
     if (need) {
@@ -1675,13 +1908,20 @@ __global__ void __maxnreg__(R) soa_kernel(const __grid_constant__ StepArgs a) {
           st.tcur = 0.0;
           st.dtfull = (double)(int)(a.dt / 1);
           st.niter = 0;
+          if constexpr (SOA != 2)
+            fast = soa_begin(st);
           active = true;
         }
       }
     }
     if (!__any_sync(0xffffffffu, active))
       break;
-    if (active && !soa_pass<SOA>(st)) {
+    // passes until a loop of the warp ends
+    bool ran;
+    do {
+      ran = active && soa_pass<SOA>(st, fast);
+    } while (!__any_sync(0xffffffffu, active && !ran));
+    if (active && !ran) {
       double *q = a.soa + slot;
       q[SOA_G * n] = st.g;
 #pragma unroll
@@ -1959,11 +2199,11 @@ __host__ __device__ constexpr int adj_soa_slots(int ck) {
 }
 
 template <bool FAST>
-__device__ __forceinline__ bool adj_soa_pass(SoaState &st) {
+__device__ __forceinline__ bool adj_soa_pass(SoaState &st, bool fast) {
   if constexpr (FAST)
     return f32::soa_step_mx(st);
   else
-    return soa_step(st);
+    return soa_step(st, fast);
 }
 
 template <int CK, bool FAST>
@@ -2025,12 +2265,13 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
     st.tcur = 0.0;
     st.dtfull = (double)(int)(a.dt / 1);
     st.niter = 0;
+    const bool fast = soa_begin(st);
     // forward: k passes (the states before passes 0..k-1 are reversed)
     int k = 0;
     while (true) {
       if (CK == 1 || k % CK == 0)
         put(k / CK, st);
-      if (!adj_soa_pass<FAST>(st))
+      if (!adj_soa_pass<FAST>(st, fast))
         break;
       ++k;
     }
@@ -2059,7 +2300,7 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
         st.niter = 0;
         put(kBlock, st);
         for (int j = 1; j < nb; ++j) {
-          adj_soa_pass<FAST>(st);
+          adj_soa_pass<FAST>(st, fast);
           put(kBlock + j, st);
         }
         for (int j = nb - 1; j >= 0; --j) {
@@ -3400,6 +3641,20 @@ cudaError_t ensure_solver_scratch(mam4b_ctx *ctx, size_t ncell) {
   return e;
 }
 
+// How the solver treats long loops. A batch with fewer cells than about
+// 3,500 per SM is bound by its longest loops (up to 1,000 passes of about
+// 400 ns with one lane per loop, about 700 ns when the SM is full): those
+// run four lanes to a loop, 520 ns a pass alone. Larger batches are bound by
+// throughput, where one lane per loop does more work per instruction, and
+// only start their longest loops early. FP64 step, 1..1,000 sub-steps per
+// cell, four lanes / one lane: 37 k cells 0.78 / 1.34 ms, 295 k cells 2.17 /
+// 2.40 ms, 590 k cells 3.70 / 3.60 ms, 2.4 M cells 13.2 / 10.7 ms. Loops
+// below 150 expected passes end before the long ones either way.
+void set_solver(StepArgs &a, int sms) {
+  a.quads = a.ncell < 3500LL * sms;
+  a.long_steps = a.quads ? 150.0 : 300.0;
+}
+
 void set_step_config(const mam4b_ctx *ctx, StepArgs &a, long long ncell, int nlev, double dt) {
   a.flags = ctx->d_flags;
   a.ncell = ncell;
@@ -3411,6 +3666,7 @@ void set_step_config(const mam4b_ctx *ctx, StepArgs &a, long long ncell, int nle
   a.do_coag = ctx->cfg.do_coag;
   a.optaa = ctx->cfg.gaexch_h2so4_uptake_optaa;
   a.nmono = ctx->cfg.n_so4_monolayers_pcage;
+  set_solver(a, ctx->sms);
 }
 
 // Pipeline scratch of the cells [c0, c0 + a.ncell) of a batch (one host
@@ -3876,8 +4132,8 @@ void mam4b_default_tuning(mam4b_tuning *t) {
   t->pre_regs = 255;
   t->post_block = 128;
   t->post_regs = 128;
-  t->soa_block = 256;
-  t->soa_regs = 64;
+  t->soa_block = 128;
+  t->soa_regs = 128;
   t->soa_blocks_per_sm = 4;
   t->cells_per_thread = 1;
   t->inline_scale = 0;
@@ -4595,6 +4851,7 @@ mam4b_status mam4b_step_slab_noalloc(const mam4b_config *cfg, const double *in_s
   a.do_coag = c.do_coag;
   a.optaa = c.gaexch_h2so4_uptake_optaa;
   a.nmono = c.n_so4_monolayers_pcage;
+  set_solver(a, nd.sms);
   cudaStream_t s = (cudaStream_t)stream;
   // the counters (and the spare flag word) must start every step at zero
   e = cudaMemsetAsync(tail, 0, (CNT_WORDS + 1) * sizeof(unsigned), s);
