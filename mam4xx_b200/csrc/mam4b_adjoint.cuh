@@ -1319,34 +1319,20 @@ struct SoaBar {
   double opoa[NMODE], uptk[NMODE], g0;
 };
 
-// x / d (FP64 arithmetic of the step), or x * mx::rcp(d) with FAST (the
-// mixed-precision loop's arithmetic, f32::soa_step_mx); on the host always
-// x / d.
-template <bool FAST>
-MAM4B_HD double qdiv(double x, double d) {
+// 1 / d for a positive normal d: cotangents need not round as the forward
+// does, so each reciprocal is taken once.
+MAM4B_HD double recip(double d) {
 #ifdef __CUDA_ARCH__
-  if constexpr (FAST)
-    return x * f32::mx::rcp(d);
+  return Divisor(d).y;
+#else
+  return 1.0 / d;
 #endif
-  return x / d;
-}
-// x * y + z, rounded once with FAST, twice (as the FP64 step) without
-template <bool FAST>
-MAM4B_HD double fmadd(double x, double y, double z) {
-  if constexpr (FAST)
-    return fma(x, y, z);
-  return z + x * y;
 }
 
-// The forward values of the pass are recomputed with the arithmetic of the
-// loop being reversed, so that every branch (skip, last sub-step, del > 0,
-// the clips) is the forward's: FAST = false the FP64 loop's (soa_step),
-// FAST = true f32::soa_step_mx's, the mixed-precision step's loop (every
-// quotient x / d as x * mx::rcp(d), the sums fused; the mixed-precision
-// adjoint). The cotangent sweep takes each reciprocal once, as
-// mx::rcp(d), in both: cotangents need not round as the forward does.
-template <bool FAST>
-MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
+// The forward values of the pass are recomputed with the FP64 loop's
+// arithmetic (soa_pass_exact), so that every branch (skip, last sub-step,
+// del > 0, the clips) is the forward's.
+MAM4B_HD void soa_step_rev(const SoaState &st, SoaBar &b) {
   const double g_prev = st.g;
   const double g = dmax(g_prev, 0.0);
   double tot = g;
@@ -1367,16 +1353,16 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
     if (skip[n])
       continue;
     aoa[n] = st.opoa[n] + a[n];
-    sat[n] = qdiv<FAST>(st.g0, dmax(aoa[n], 1.0e-20));
+    sat[n] = st.g0 / dmax(aoa[n], 1.0e-20);
     gs[n] = sat[n] * a[n];
     M1[n] = dmax(g, dmax(gs[n], 1.0e-20));
-    phi[n] = qdiv<FAST>(g - gs[n], M1[n]);
-    tmpb = fmadd<FAST>(st.uptk[n], fabs(phi[n]), tmpb);
+    phi[n] = (g - gs[n]) / M1[n];
+    tmpb = tmpb + st.uptk[n] * fabs(phi[n]);
   }
   const double tmpa = dmax(0.0, tmpb);
   const double dtmax = st.dtfull - st.tcur;
   const bool last = dtmax * tmpa <= 0.05;
-  const double dtcur = last ? dtmax : qdiv<FAST>(0.05, tmpa);
+  const double dtcur = last ? dtmax : 0.05 / tmpa;
   double beta[NMODE], del[NMODE], sat2[NMODE], den[NMODE];
   double ta = 0.0, tbs = 0.0;
 #pragma unroll
@@ -1387,28 +1373,22 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
     del[n] = g - gs[n];
     sat2[n] = sat[n];
     if (del[n] > 0.0) {
-      const double a_tmp = fmadd<FAST>(beta[n], del[n], a[n]);
-      sat2[n] = qdiv<FAST>(st.g0, dmax(st.opoa[n] + a_tmp, 1.0e-20));
+      const double a_tmp = a[n] + beta[n] * del[n];
+      sat2[n] = st.g0 / dmax(st.opoa[n] + a_tmp, 1.0e-20);
     }
-    den[n] = fmadd<FAST>(beta[n], sat2[n], 1.0);
-    if constexpr (FAST) {
-      const double rd = qdiv<FAST>(1.0, den[n]);
-      ta = fmadd<FAST>(a[n], rd, ta);
-      tbs = fmadd<FAST>(beta[n], rd, tbs);
-    } else {
-      ta += a[n] / den[n];
-      tbs += beta[n] / den[n];
-    }
+    den[n] = 1.0 + beta[n] * sat2[n];
+    ta += a[n] / den[n];
+    tbs += beta[n] / den[n];
   }
-  const double q = qdiv<FAST>(tot - ta, 1.0 + tbs);
+  const double q = (tot - ta) / (1.0 + tbs);
   const double gn = dmax(0.0, q);
   // ---- reverse (reciprocals taken once: the cotangents need not round as
   // the forward does)
   double rden[NMODE];
 #pragma unroll
   for (int n = 0; n < NMODE; ++n)
-    rden[n] = skip[n] ? 0.0 : qdiv<true>(1.0, den[n]);
-  const double r1 = qdiv<true>(1.0, 1.0 + tbs);
+    rden[n] = skip[n] ? 0.0 : recip(den[n]);
+  const double r1 = recip(1.0 + tbs);
   double gnb = b.g, ab_[NMODE], betab[NMODE], denb[NMODE], sat2b[NMODE], satb[NMODE], gsb[NMODE];
   double gb = 0.0, totb = 0.0, tab = 0.0, tbb = 0.0, dtcurb = 0.0, tcurb = 0.0;
 #pragma unroll
@@ -1429,7 +1409,7 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
   for (int n = 0; n < NMODE; ++n) {
     if (skip[n])
       continue;  // a'[n] = 0
-    const double an = fmadd<FAST>(beta[n], gn, a[n]) * rden[n];
+    const double an = (a[n] + beta[n] * gn) * rden[n];
     const double numb = b.a[n] * rden[n];
     denb[n] -= numb * an;
     ab_[n] += numb;
@@ -1451,9 +1431,9 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
     betab[n] += denb[n] * sat2[n];
     sat2b[n] += denb[n] * beta[n];
     if (del[n] > 0.0) {
-      const double a_tmp = fmadd<FAST>(beta[n], del[n], a[n]);
+      const double a_tmp = a[n] + beta[n] * del[n];
       const double aoa2 = st.opoa[n] + a_tmp;
-      const double rM2 = qdiv<true>(1.0, dmax(aoa2, 1.0e-20));
+      const double rM2 = recip(dmax(aoa2, 1.0e-20));
       b.g0 += sat2b[n] * rM2;
       const double M2b = -sat2b[n] * sat2[n] * rM2;
       const double aoa2b = maxxc_rev(aoa2, 1.0e-20, M2b);
@@ -1474,7 +1454,7 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
   if (last)
     tcurb -= dtcurb;  // dtcur = dtfull - tcur
   else
-    tmpab -= qdiv<true>(dtcurb * dtcur, tmpa);
+    tmpab -= dtcurb * dtcur * recip(tmpa);
   const double tmpbb = maxc_rev(0.0, tmpb, tmpab);
 #pragma unroll
   for (int n = 0; n < NMODE; ++n) {
@@ -1482,7 +1462,7 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
       continue;
     b.uptk[n] += tmpbb * fabs(phi[n]);
     const double phib = tmpbb * st.uptk[n] * (phi[n] < 0.0 ? -1.0 : 1.0);
-    const double rM1 = qdiv<true>(1.0, M1[n]);
+    const double rM1 = recip(M1[n]);
     gb += phib * rM1;
     gsb[n] -= phib * rM1;
     const double M1b = -phib * phi[n] * rM1;
@@ -1497,7 +1477,7 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
     satb[n] += gsb[n] * a[n];
     ab_[n] += gsb[n] * sat[n];
     // sat = g0 / dmax(aoa, 1e-20)
-    const double rM = qdiv<true>(1.0, dmax(aoa[n], 1.0e-20));
+    const double rM = recip(dmax(aoa[n], 1.0e-20));
     b.g0 += satb[n] * rM;
     const double Mb = -satb[n] * sat[n] * rM;
     const double aoab = maxxc_rev(aoa[n], 1.0e-20, Mb);
@@ -1519,7 +1499,163 @@ MAM4B_HD void soa_step_rev_t(const SoaState &st, SoaBar &b) {
   b.tcur = tcurb;
 }
 
-MAM4B_HD void soa_step_rev(const SoaState &st, SoaBar &b) { soa_step_rev_t<false>(st, b); }
+#ifdef __CUDACC__
+// The reverse of a pass for the solver kernel: W modes per lane, W = 4 the
+// whole loop on one lane, W = 1 one mode on each of four consecutive lanes
+// (values without a mode index are then the same on the four, but for
+// LoopBar::g0, of which each lane holds its mode's part). It linearises the
+// pass at the stored state with the division-free arithmetic of
+// f32::soa_step_mx, one reciprocal per denominator; the state is the
+// forward's exactly, so its derivative is computed to rounding (a branch
+// that sits within rounding of its threshold may be taken the other way,
+// like a finite difference across it). Skipped modes are cleared
+// (soa_clear_skipped) and keep zero cotangents, so there is no branch per
+// mode and their chains overlap. The sums over the modes are taken in mode
+// order in both forms: in a cell near equilibrium the cotangents cancel, and
+// another order moves its gradient by far more than rounding.
+template <int W>
+struct LoopState {
+  double g, a[W], tcur, opoa[W], uptk[W], g0, dtfull;
+};
+template <int W>
+struct LoopBar {
+  double g, a[W], tcur, opoa[W], uptk[W], g0;
+};
+// the value of every mode
+template <int W>
+__device__ __forceinline__ void all_modes(const double (&x)[W], double (&v)[NMODE]) {
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    if constexpr (W == 1)
+      v[n] = __shfl_sync(0xffffffffu, x[0], ((threadIdx.x & 31) & ~3) + n);
+    else
+      v[n] = x[n];
+  }
+}
+template <int W>
+__device__ __forceinline__ double sum_modes(double s, const double (&x)[W]) {
+  double v[NMODE];
+  all_modes(x, v);
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n)
+    s += v[n];
+  return s;
+}
+
+template <int W>
+__device__ __forceinline__ void soa_pass_rev(const LoopState<W> &st, LoopBar<W> &b) {
+  using f32::mx::rcp;
+  const double g = dmax(st.g, 0.0);
+  double a[W], aoa[W], rM[W], sat[W], gs[W], rM1[W], phi[W], aphi[W];
+#pragma unroll
+  for (int n = 0; n < W; ++n) {
+    a[n] = dmax(st.a[n], 0.0);
+    aoa[n] = st.opoa[n] + a[n];
+    rM[n] = rcp(dmax(aoa[n], 1.0e-20));
+    sat[n] = st.g0 * rM[n];
+    gs[n] = sat[n] * a[n];
+    rM1[n] = rcp(dmax(g, dmax(gs[n], 1.0e-20)));
+    phi[n] = (g - gs[n]) * rM1[n];
+    aphi[n] = fabs(phi[n]);
+  }
+  double all_a[NMODE], all_phi[NMODE], all_u[NMODE], all_r[NMODE];
+  all_modes(a, all_a);
+  all_modes(aphi, all_phi);
+  all_modes(st.uptk, all_u);
+  double tot = g, tmpb = 0.0;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    tot += all_a[n];
+    tmpb = fma(all_u[n], all_phi[n], tmpb);
+  }
+  const double tmpa = dmax(0.0, tmpb), dtmax = st.dtfull - st.tcur;
+  const bool last = dtmax * tmpa <= 0.05;
+  const double rt = rcp(last ? 1.0 : tmpa);
+  const double dtcur = last ? dtmax : 0.05 * rt;
+  double beta[W], del[W], aoa2[W], rM2[W], sat2[W], rden[W];
+#pragma unroll
+  for (int n = 0; n < W; ++n) {
+    beta[n] = dtcur * st.uptk[n];
+    del[n] = g - gs[n];
+    aoa2[n] = st.opoa[n] + fma(beta[n], del[n], a[n]);
+    rM2[n] = rcp(dmax(aoa2[n], 1.0e-20));
+    sat2[n] = del[n] > 0.0 ? st.g0 * rM2[n] : sat[n];
+    rden[n] = rcp(fma(beta[n], sat2[n], 1.0));
+  }
+  all_modes(rden, all_r);
+  double ta = 0.0, tbs = 0.0;
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n) {
+    ta = fma(all_a[n], all_r[n], ta);
+    tbs = fma(dtcur * all_u[n], all_r[n], tbs);
+  }
+  const double r1 = rcp(1.0 + tbs);
+  const double q = (tot - ta) * r1, gn = dmax(0.0, q);
+  // ---- reverse: particle update and the gas
+  double numb[W], part[W];
+#pragma unroll
+  for (int n = 0; n < W; ++n) {
+    numb[n] = b.a[n] * rden[n];
+    part[n] = numb[n] * beta[n];
+  }
+  const double qr = maxc_rev(0.0, q, sum_modes(b.g, part)) * r1;
+  const double tbb = -qr * q;  // cotangent of 1 + tbs; of tot qr, of ta -qr
+  double ab[W], gsb[W], satb[W], delb[W];
+#pragma unroll
+  for (int n = 0; n < W; ++n) {
+    const double an = fma(beta[n], gn, a[n]) * rden[n];
+    const double denb = -(numb[n] * an) - (tbb * beta[n] - qr * a[n]) * (rden[n] * rden[n]);
+    const double sat2b = denb * beta[n];
+    double betab = (numb[n] * gn + tbb * rden[n]) + denb * sat2[n];
+    const bool up = del[n] > 0.0;
+    const double aoa2b =
+        up ? maxxc_rev(aoa2[n], 1.0e-20, -sat2b * sat2[n] * rM2[n]) : 0.0;
+    ab[n] = (numb[n] - qr * rden[n]) + aoa2b;
+    betab += aoa2b * del[n];
+    delb[n] = aoa2b * beta[n];
+    gsb[n] = -delb[n];
+    satb[n] = up ? 0.0 : sat2b;
+    b.g0 += up ? sat2b * rM2[n] : 0.0;
+    b.opoa[n] += aoa2b;
+    b.uptk[n] += betab * dtcur;
+    part[n] = betab * st.uptk[n];
+  }
+  // sub-step: dtfull - tcur in the last pass, 0.05 / tmpa otherwise
+  const double dtcurb = sum_modes(last ? 0.0 : b.tcur, part);
+  const double tmpbb = last ? 0.0 : maxc_rev(0.0, tmpb, -(dtcurb * dtcur) * rt);
+  double gb = sum_modes(0.0, delb), phir[W], M1g[W];
+#pragma unroll
+  for (int n = 0; n < W; ++n) {
+    b.uptk[n] += tmpbb * aphi[n];
+    const double phib = tmpbb * st.uptk[n] * (phi[n] < 0.0 ? -1.0 : 1.0);
+    phir[n] = phib * rM1[n];
+    gsb[n] -= phir[n];
+    // the denominator of phi: dmax(g, dmax(gs, 1e-20))
+    const double M1b = -phib * phi[n] * rM1[n];
+    const bool of_g = !(g < dmax(gs[n], 1.0e-20));
+    M1g[n] = of_g ? M1b : 0.0;
+    gsb[n] += of_g ? 0.0 : maxxc_rev(gs[n], 1.0e-20, M1b);
+    // gs = sat a, sat = g0 / dmax(aoa, 1e-20)
+    satb[n] += gsb[n] * a[n];
+    b.g0 += satb[n] * rM[n];
+    const double aoab = maxxc_rev(aoa[n], 1.0e-20, -satb[n] * sat[n] * rM[n]);
+    b.opoa[n] += aoab;
+    const bool live = st.uptk[n] > 1.0e-15;
+    ab[n] = (ab[n] + gsb[n] * sat[n]) + aoab;
+    b.a[n] = live ? maxxc_rev(st.a[n], 0.0, ab[n] + qr) : 0.0;
+    b.uptk[n] = live ? b.uptk[n] : 0.0;
+  }
+  double all_p[NMODE], all_m[NMODE];
+  all_modes(phir, all_p);
+  all_modes(M1g, all_m);
+#pragma unroll
+  for (int n = 0; n < NMODE; ++n)
+    gb = (gb + all_p[n]) + all_m[n];
+  b.g = maxxc_rev(st.g, 0.0, gb + qr);
+  b.tcur = last ? -dtcurb : b.tcur;
+}
+#endif
+
 
 // soa_init (gasaerexch_soaexch.hpp:155-170): g0 from T (p fixed); opoa
 // from POM; initial g, a from the subarea

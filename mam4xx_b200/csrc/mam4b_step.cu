@@ -89,7 +89,7 @@ enum { AUX_RH = 0, AUX_GDIFF = 1, AUX_FPATH = 2, AUX_RATE = 3, AUX_COAG = 7, AUX
 // queue counters: queued slots, long and short loops in the order list,
 // short and long loops handed to the solver
 enum { CNT_QUEUED = 0, CNT_TAKEN = 1, CNT_LONG = 2, CNT_SHORT = 3, CNT_TAKEN_ADJ = 4,
-       CNT_TAKEN_LONG = 5, CNT_WORDS = 8 };
+       CNT_TAKEN_LONG = 5, CNT_TAKEN_ADJ_LONG = 6, CNT_WORDS = 8 };
 
 // ----------------------------------------------------- per-cell amicphys
 struct Diag {
@@ -1788,6 +1788,16 @@ __device__ __forceinline__ void soa_quad_pass(SoaQuad<float> &st, bool, int base
   st.a = (a + beta * st.g) * den;
 }
 
+// soa_begin for one lane: clears a skipped mode and returns whether the
+// lane's parameters allow quot_in_range.
+template <class T>
+__device__ __forceinline__ bool soa_quad_begin(SoaQuad<T> &st) {
+  if (!(st.uptk > (T)1.0e-15) && 0.0 < st.dtfull - 1.0e-3)
+    st.uptk = st.a = st.opoa = (T)0.0;
+  return zero_or_moderate(st.g0) && st.g0 != (T)0.0 && zero_or_moderate(st.dtfull) &&
+         zero_or_moderate(st.opoa) && zero_or_moderate(st.uptk);
+}
+
 // The long loops of the queue, four lanes to a loop, with work stealing as
 // in soa_kernel (eight loops per warp).
 template <int SOA, class T>
@@ -1820,12 +1830,7 @@ __device__ __forceinline__ void soa_long_loops(const StepArgs &a) {
           st.tcur = 0.0;
           st.dtfull = (double)(int)(a.dt / 1);
           st.niter = 0;
-          // a skipped mode takes no part (soa_clear_skipped)
-          if (!(st.uptk > (T)1.0e-15) && 0.0 < st.dtfull - 1.0e-3)
-            st.uptk = st.a = st.opoa = (T)0.0;
-          if constexpr (SOA == 0)
-            fast = zero_or_moderate(st.g0) && st.g0 != 0.0 && zero_or_moderate(st.dtfull) &&
-                   zero_or_moderate(st.opoa) && zero_or_moderate(st.uptk);
+          fast = soa_quad_begin(st);
           active = true;
         }
       }
@@ -2184,19 +2189,20 @@ __global__ void __launch_bounds__(256) adj_sort_kernel(const __grid_constant__ A
 // (the recomputed passes are the forward's arithmetic on the same state);
 // CK > 1 needs about 1/CK of the memory and recomputes up to CK - 1 passes
 // per block. The forward loop is the step's: soa_step (FP64), or with FAST
-// f32::soa_step_mx (the mixed-precision adjoint). The reverse of each pass
-// linearises it at the stored state with the division-free arithmetic of
-// f32::soa_step_mx (adj::soa_step_rev_t<true>): the trajectory is the
-// forward's exactly, its local derivative is computed to rounding (a
-// branch that sits within rounding of its threshold may be taken the other
-// way, like a finite difference across it). 2 blocks per SM (128
-// registers, some spilled to L1): the extra warps hide more FP64 latency
-// than the unconstrained 255-register build (10 % faster).
+// f32::soa_step_mx (the mixed-precision adjoint); the reverse of a pass is
+// adj::soa_pass_rev. Long loops of small batches (StepArgs::quads) go first,
+// four lanes to a loop (adj_long_loops). 2 blocks per SM (128 registers,
+// some spilled to L1): the extra warps hide more FP64 latency than the
+// unconstrained 255-register build (10 % faster).
 constexpr int kAdjSoaStates = 1001;  // states before passes 0..1000 (passes <= 1000)
 // states kept per solver thread: checkpoints plus, with CK > 1, one block
 __host__ __device__ constexpr int adj_soa_slots(int ck) {
   return ck == 1 ? kAdjSoaStates : (kAdjSoaStates + ck - 1) / ck + ck;
 }
+// rows of a thread's column of p.ck that adj_long_loops uses: one SOA value
+// per pass, and g or tcur of every other pass
+constexpr int kAdjQuadRows = kAdjSoaStates + (kAdjSoaStates + 1) / 2;
+static_assert(kAdjQuadRows <= 6 * adj_soa_slots(4), "the quads' states fit either form's columns");
 
 template <bool FAST>
 __device__ __forceinline__ bool adj_soa_pass(SoaState &st, bool fast) {
@@ -2206,10 +2212,108 @@ __device__ __forceinline__ bool adj_soa_pass(SoaState &st, bool fast) {
     return soa_step(st, fast);
 }
 
+// The loops of at least kAdjLongPasses passes (the head of the sorted order
+// list), eight per warp and four lanes each, with the state before every
+// pass kept in the four lanes' columns: row i of a lane its mode's SOA
+// before pass i, rows kAdjSoaStates + i / 2 of lanes 2 (i % 2) and 2 (i % 2)
+// + 1 g and tcur. The chain of a 1,000-pass loop, forward and reverse, is
+// what bounds a small batch.
+constexpr int kAdjLongPasses = 64;
+template <bool FAST>
+__device__ __forceinline__ void adj_long_loops(const AdjPipeArgs &p, unsigned nlong) {
+  const StepArgs &a = p.s;
+  const int lane = threadIdx.x & 31, mode = lane & 3, base = lane & ~3;
+  const size_t n = (size_t)a.ncell;
+  const size_t nthreads = (size_t)gridDim.x * blockDim.x;
+  double *own = p.ck + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  double *group = own - mode;
+  auto pair_row = [&](int i) {
+    return group + (size_t)(kAdjSoaStates + (i >> 1)) * nthreads + 2 * (i & 1);
+  };
+  while (true) {
+    unsigned first = 0;
+    if (lane == 0)
+      first = atomicAdd(&a.counters[CNT_TAKEN_ADJ_LONG], 8u);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (first >= nlong)
+      return;
+    const unsigned t = first + lane / 4;
+    const bool valid = t < nlong;
+    const unsigned slot = (unsigned)a.order[valid ? t : nlong - 1];
+    const double *h = a.hand + slot;
+    const double *q = a.soa + slot;
+    constexpr int kSoaSlot[NMODE] = {K::aer_slot(0, 0), K::aer_slot(0, 1), K::aer_slot(0, 2), -1};
+    const int soa_slot = mode == 0 ? kSoaSlot[0] : mode == 1 ? kSoaSlot[1] : kSoaSlot[2];
+    SoaQuad<double> st;
+    st.g = h[H_SOAG0 * n];
+    st.a = mode < 3 ? h[(H_POP + soa_slot) * n] : 0.0;
+    st.opoa = q[(SOA_OPOA + mode) * n];
+    st.uptk = q[(SOA_UPTK + mode) * n];
+    st.g0 = q[SOA_G0 * n];
+    st.tcur = 0.0;
+    st.dtfull = (double)(int)(a.dt / 1);
+    st.niter = 0;
+    const bool fast = soa_quad_begin(st);
+    const SoaQuad<double> init = st;
+    int k = 0;
+    bool go = valid;
+    while (true) {
+      if (go) {
+        own[(size_t)k * nthreads] = st.a;
+        if (mode < 2)
+          pair_row(k)[mode] = mode == 0 ? st.g : st.tcur;
+        go = soa_more(st);
+      }
+      if (!__any_sync(0xffffffffu, go))
+        break;
+      soa_quad_pass(st, fast, base, std::integral_constant<int, FAST ? 1 : 0>());
+      k += go;
+    }
+    __syncwarp();  // the group reads g and tcur where its other lanes stored them
+    adj::LoopState<1> x;
+    x.opoa[0] = init.opoa;
+    x.uptk[0] = init.uptk;
+    x.g0 = init.g0;
+    x.dtfull = init.dtfull;
+    adj::LoopBar<1> b;
+    b.g = q[SOA_G * n];
+    // a pass leaves a skipped mode no SOA, so nothing passes back through it
+    b.a[0] = k == 0 || init.uptk > 1.0e-15 ? q[(SOA_A + mode) * n] : 0.0;
+    b.tcur = b.opoa[0] = b.uptk[0] = b.g0 = 0.0;
+    for (int i = __reduce_max_sync(0xffffffffu, k) - 1; i >= 0; --i) {
+      const int j = min(i, max(k - 1, 0));  // loops with fewer passes wait
+      x.a[0] = own[(size_t)j * nthreads];
+      x.g = pair_row(j)[0];
+      x.tcur = pair_row(j)[1];
+      adj::LoopBar<1> nb = b;
+      adj::soa_pass_rev(x, nb);
+      if (i < k)
+        b = nb;
+    }
+    const double g0b[1] = {b.g0};
+    const double g0_sum = adj::sum_modes(0.0, g0b);
+    if (valid) {
+      double *lb = p.lbar + a.task[slot];
+      if (mode == 0) {
+        lb[LB_G * n] = b.g;
+        lb[LB_G0 * n] = g0_sum;
+      }
+      lb[(LB_A + mode) * n] = b.a[0];
+      lb[(LB_OPOA + mode) * n] = b.opoa[0];
+      lb[(LB_UPTK + mode) * n] = b.uptk[0];
+    }
+    __syncwarp();  // before the next loops' states overwrite these
+  }
+}
+
 template <int CK, bool FAST>
 __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_constant__ AdjPipeArgs p) {
   const StepArgs &a = p.s;
   const unsigned ntask = a.counters[CNT_QUEUED];
+  // loops of at least kAdjLongPasses passes: where adj_sort_kernel left off
+  // in their last bin
+  const unsigned nlong = a.quads ? p.bins[kPassBins + 1000 - kAdjLongPasses] : 0u;
+  adj_long_loops<FAST>(p, nlong);
   const int lane = threadIdx.x & 31;
   const size_t n = (size_t)a.ncell;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
@@ -2222,7 +2326,7 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
       e[(1 + j) * nthreads] = x.a[j];
     e[5 * nthreads] = x.tcur;
   };
-  auto get = [&](int idx, SoaState &x) {
+  auto get = [&](int idx, auto &x) {
     const double *e = ck + (size_t)6 * idx * nthreads;
     x.g = e[0];
 #pragma unroll
@@ -2233,7 +2337,7 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
   while (true) {
     unsigned base = 0;
     if (lane == 0)
-      base = atomicAdd(&a.counters[CNT_TAKEN_ADJ], 32u);
+      base = nlong + atomicAdd(&a.counters[CNT_TAKEN_ADJ], 32u);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= ntask)
       break;
@@ -2275,21 +2379,26 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
         break;
       ++k;
     }
-    adj::SoaBar b;
+    adj::LoopState<NMODE> x;
+    adj::LoopBar<NMODE> b;
     b.g = q[SOA_G * n];
 #pragma unroll
     for (int j = 0; j < NMODE; ++j) {
-      b.a[j] = q[(SOA_A + j) * n];
+      x.opoa[j] = st.opoa[j];
+      x.uptk[j] = st.uptk[j];
+      b.a[j] = k == 0 || st.uptk[j] > 1.0e-15 ? q[(SOA_A + j) * n] : 0.0;
       b.opoa[j] = 0.0;
       b.uptk[j] = 0.0;
     }
+    x.g0 = st.g0;
+    x.dtfull = st.dtfull;
     b.tcur = 0.0;
     b.g0 = 0.0;
     if constexpr (CK == 1) {
       while (k > 0) {
         --k;
-        get(k, st);
-        adj::soa_step_rev_t<true>(st, b);
+        get(k, x);
+        adj::soa_pass_rev(x, b);
       }
     } else {
       constexpr int kBlock = (kAdjSoaStates + CK - 1) / CK;  // first state of the block slice
@@ -2304,8 +2413,8 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
           put(kBlock + j, st);
         }
         for (int j = nb - 1; j >= 0; --j) {
-          get(kBlock + j, st);
-          adj::soa_step_rev_t<true>(st, b);
+          get(kBlock + j, x);
+          adj::soa_pass_rev(x, b);
         }
       }
     }

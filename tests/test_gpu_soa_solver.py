@@ -73,3 +73,35 @@ def test_small_and_large_batches_agree(cuda_device, precision):
                 precision)
     ctx.close()
     assert torch.equal(big, small.repeat(1, times))
+
+
+def _adjoint(ctx, x, pb, ybar, ncol, nlev, dt, precision):
+    xb = torch.full((native.NIN, x.shape[1]), float("nan"), dtype=torch.float64, device="cuda")
+    ctx.adjoint_slab(x.data_ptr(), pb.data_ptr(), ybar.data_ptr(), xb.data_ptr(), x.shape[1],
+                     ncol, nlev, dt, precision=precision)
+    torch.cuda.synchronize()
+    return xb
+
+
+@pytest.mark.parametrize("precision", [native.FP64, native.MIXED])
+@pytest.mark.parametrize("interval", [1, 4])
+def test_adjoint_of_small_and_large_batches_agrees(cuda_device, precision, interval):
+    """Loops reversed on four lanes and on one. Every sum that feeds the
+    reverse sweep is taken in the same order, so all gradients are equal but
+    the temperature's, whose equilibrium-gas part is added up mode by mode
+    and then over the modes: a reordered sum of at most 8,000 terms, within
+    8,000 eps of the terms' size (2e-12), here against the row's norm."""
+    w = make_workload("c2", ncol=24, seed=81)
+    x, pb = torch.from_numpy(w["in_slab"]).cuda(), torch.from_numpy(w["pblh"]).cuda()
+    n, sms = x.shape[1], torch.cuda.get_device_properties(0).multi_processor_count
+    ybar = torch.from_numpy(np.random.default_rng(82).standard_normal((native.NOUT, n))).cuda()
+    times = 3500 * sms // n + 1
+    ctx = native.Context()
+    ctx.set_adjoint_checkpoint(interval)
+    small = _adjoint(ctx, x, pb, ybar, w["ncol"], w["nlev"], w["dt"], precision)
+    big = _adjoint(ctx, x.repeat(1, times), pb.repeat(times), ybar.repeat(1, times),
+                   w["ncol"] * times, w["nlev"], w["dt"], precision)[:, -n:]
+    ctx.close()
+    assert torch.equal(small[1:], big[1:])
+    d = float(torch.linalg.norm(small[0] - big[0]) / torch.linalg.norm(big[0]))
+    assert d <= 2e-12
