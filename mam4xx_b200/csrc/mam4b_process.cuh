@@ -73,9 +73,9 @@ MAM4B_HD void calcsize_process_cell(const StepConsts &C, const CalcSizeArgs &a, 
       T.n_c[m][c] = tc;
     }
     diameter_from_num(vi, num_i[m], C.n2v_min[m], C.n2v_max[m], K::dmin(m), K::dmax(m),
-                      C.log_sig[m], dgi[m]);
+                      C.diam_fac[m], dgi[m]);
     diameter_from_num(vc, num_c[m], C.n2v_min[m], C.n2v_max[m], K::dmin(m), K::dmax(m),
-                      C.log_sig[m], dgc[m]);
+                      C.diam_fac[m], dgc[m]);
   }
   if (a.do_aitacc_transfer) {
     const double v2n_ait = C.n2v_nom[1], v2n_acc = C.n2v_nom[0];
@@ -158,13 +158,13 @@ MAM4B_HD void calcsize_process_cell(const StepConsts &C, const CalcSizeArgs &a, 
       const double vdc = (dv_c[1] * xv_ait2acc - (dv_c[0] - noxf_c) * xv_acc2ait) * a.dt;
       const double vc_ait = dmax(0.0, dv_c[1] - vdc), vc_acc = dmax(0.0, dv_c[0] + vdc);
       dgi[1] = size_after_transfer(vi_ait, ni_ait, C.n2v_min[1], C.n2v_max[1], K::dmax(1),
-                                   K::dmin(1), K::dnom(1), C.log_sig[1]);
+                                   K::dmin(1), K::dnom(1), C.diam_fac[1]);
       dgc[1] = size_after_transfer(vc_ait, nc_ait, C.n2v_min[1], C.n2v_max[1], K::dmax(1),
-                                   K::dmin(1), K::dnom(1), C.log_sig[1]);
+                                   K::dmin(1), K::dnom(1), C.diam_fac[1]);
       dgi[0] = size_after_transfer(vi_acc, ni_acc, C.n2v_min[0], C.n2v_max[0], K::dmax(0),
-                                   K::dmin(0), K::dnom(0), C.log_sig[0]);
+                                   K::dmin(0), K::dnom(0), C.diam_fac[0]);
       dgc[0] = size_after_transfer(vc_acc, nc_acc, C.n2v_min[0], C.n2v_max[0], K::dmax(0),
-                                   K::dmin(0), K::dnom(0), C.log_sig[0]);
+                                   K::dmin(0), K::dnom(0), C.diam_fac[0]);
       // update_tends_flx (calcsize.hpp:529-590): common species of the two
       // modes, accumulation SO4 SOA NaCl MOM <-> aitken SO4 SOA NaCl MOM
       constexpr int acc_s[4] = {0, 2, 5, 6};

@@ -54,14 +54,14 @@ struct StepArgs {
   unsigned nmono;
   // SOA solver hand-off (see soa_kernel): per-cell loop state, the list of
   // queued cells, the solver's order and counters (CNT_*)
-  double *soa;       // [SOA_FIELDS][ncell], indexed by queue slot
-  double *hand;      // [H_FIELDS][ncell], indexed by queue slot
-  int *task;         // [ncell]: cell of each queue slot
-  int *order;        // [ncell]: slots in solver order, long loops from the
+  double *soa;       // [SOA_FIELDS][ncell]
+  double *hand;      // [H_FIELDS][ncell]
+  int *done;         // [ncell]: cells that pre_kernel<.., FUSE> finished
+  int *order;        // [ncell]: cells in solver order, long loops from the
                      // front, short ones from the back
   double *aux;       // [AUX_FIELDS][ncell], indexed by cell (size/mode kernels)
   unsigned *counters;
-  int *npass;        // [ncell] or null: passes of each slot's loop (adjoint only)
+  int *npass;        // [ncell] or null: passes of each cell's loop (adjoint only)
   int mixed;         // the mode/pair stages ran in FP32 (MAM4B_MIXED, _FAST)
   double long_steps;    // a loop is long (soa_kernel runs it first) when its
                         // first sub-step is shorter than dt / long_steps
@@ -71,25 +71,30 @@ struct StepArgs {
 };
 
 // The step runs as a pipeline of six kernels when condensation is on and
-// no diagnostics are asked for: size_kernel, mode_kernel and pair_kernel
-// compute calcsize, water uptake, uptake rates and coagulation coefficients
-// into `aux` and the size outputs; pre_kernel runs each cell up to the SOA
-// condensation loop of its clear subarea, writes the loop's initial state
-// and the rest of the cell's state at that point to slot-indexed scratch
-// and queues the cell (cloudy cells finish there); soa_kernel runs the
-// queued loops with per-lane work stealing; post_kernel finishes the queued
-// cells from the hand-off and the loop result. Otherwise full_kernel runs
+// no diagnostics are asked for: front_kernel runs calcsize, the humidity of
+// water uptake, the subarea set-up and the cloudy subarea, and leaves the
+// clear subarea at its SOA condensation loop in slot-indexed scratch (cloudy
+// cells finish there); mode_kernel and pair_kernel compute water uptake,
+// uptake rates and coagulation coefficients; pre_kernel adds the uptake
+// rates and orders the loops; soa_kernel runs them with per-lane work
+// stealing; post_kernel finishes the queued cells from the hand-off and the
+// loop result. With chemistry, which runs between calcsize's update and the
+// subareas, size_kernel takes the place of front_kernel and pre_chem_kernel
+// does the rest of its work with pre_kernel's. Otherwise full_kernel runs
 // each cell start to end in one thread.
 enum { SOA_G = 0, SOA_A = 1, SOA_OPOA = 5, SOA_UPTK = 9, SOA_G0 = 13, SOA_FIELDS = 14 };
-// per-cell values from size_kernel and mode_kernel for the pre kernel:
+// per-cell values from the first two stages for the later ones:
 // relative humidity for water uptake, H2SO4 diffusivity and mean free path,
 // per-particle H2SO4 uptake rate of each mode
 // and the 12 coagulation coefficients (coag_all_coefs order)
 enum { AUX_RH = 0, AUX_GDIFF = 1, AUX_FPATH = 2, AUX_RATE = 3, AUX_COAG = 7, AUX_FIELDS = 19 };
-// queue counters: queued slots, long and short loops in the order list,
-// short and long loops handed to the solver
-enum { CNT_QUEUED = 0, CNT_TAKEN = 1, CNT_LONG = 2, CNT_SHORT = 3, CNT_TAKEN_ADJ = 4,
-       CNT_TAKEN_LONG = 5, CNT_TAKEN_ADJ_LONG = 6, CNT_WORDS = 8 };
+// queue counters: long and short loops in the order list, short and long
+// loops handed to the solver, and to the adjoint's
+enum { CNT_TAKEN = 0, CNT_LONG = 1, CNT_SHORT = 2, CNT_TAKEN_ADJ = 3, CNT_TAKEN_LONG = 4,
+       CNT_TAKEN_ADJ_LONG = 5, CNT_WORDS = 8 };
+// Cells with a cloud fraction above this are cloudy throughout: they have no
+// clear subarea and no SOA loop.
+constexpr double kCloudy = 0.999;
 
 // ----------------------------------------------------- per-cell amicphys
 struct Diag {
@@ -103,8 +108,8 @@ __device__ __forceinline__ int pop_to_i31(int p) { return 6 + p; }
 // amicphys tracer index of the number of mode m (mam4_amicphys.hpp:36)
 __device__ __forceinline__ int num_i31(int m) { return m == 0 ? 13 : m == 1 ? 18 : m == 2 ? 26 : 30; }
 
-// Hand-off of a queued cell from the pre to the post kernel: one double per
-// field and queue slot ([field][slot], coalesced in both kernels).
+// Hand-off of a cell with a clear subarea from the first stage to the later
+// ones: one double per field and cell.
 enum {
   H_GAS1 = 0,      // H2SO4 of the clear subarea at the loop
   H_POP = 1,       // 25 numbers/masses of the clear subarea at the loop
@@ -374,11 +379,11 @@ __device__ __forceinline__ void store_cloudborne(const StepArgs &a, long long c,
                                                  const double (&oc)[NPOP],
                                                  const double (&ac)[NPOP]) {
   const StepConsts &C = c_k;
-  const double dt = a.dt;
+  const GuardedDivisor per_dt(a.dt);
   double *const *out = a.out;
 #pragma unroll
   for (int p = 0; p < NPOP; ++p)
-    out[MAM4B_OUT_TEND + 27 + p][c] = (oc[p] * C.to_mmr[2 + p] - ac[p]) / dt;
+    out[MAM4B_OUT_TEND + 27 + p][c] = per_dt.under(oc[p] * C.to_mmr[2 + p] - ac[p]);
 }
 
 // Tendencies of the gases and the 25 interstitial populations.
@@ -387,13 +392,13 @@ __device__ __forceinline__ void store_interstitial(const StepArgs &a, long long 
                                                    double h2so4, double soag,
                                                    const double (&ai)[NPOP]) {
   const StepConsts &C = c_k;
-  const double dt = a.dt;
+  const GuardedDivisor per_dt(a.dt);
   double *const *out = a.out;
-  out[MAM4B_OUT_TEND + 0][c] = (o_h2so4 * C.to_mmr[0] - h2so4) / dt;
-  out[MAM4B_OUT_TEND + 1][c] = (o_soag * C.to_mmr[1] - soag) / dt;
+  out[MAM4B_OUT_TEND + 0][c] = per_dt.under(o_h2so4 * C.to_mmr[0] - h2so4);
+  out[MAM4B_OUT_TEND + 1][c] = per_dt.under(o_soag * C.to_mmr[1] - soag);
 #pragma unroll
   for (int p = 0; p < NPOP; ++p)
-    out[MAM4B_OUT_TEND + 2 + p][c] = (oi[p] * C.to_mmr[2 + p] - ai[p]) / dt;
+    out[MAM4B_OUT_TEND + 2 + p][c] = per_dt.under(oi[p] * C.to_mmr[2 + p] - ai[p]);
 }
 
 __device__ __forceinline__ void store_outputs(const StepArgs &a, long long c, double o_h2so4,
@@ -414,6 +419,17 @@ struct Front {
   double g_h2so4, g_soag;             // gases (vmr)
   double relhumgcm;
 };
+
+// Relative humidity of the cell as amicphys diagnoses it
+// (mam4_amicphys.hpp:2199-2205)
+__device__ __forceinline__ double relhum_gcm(double qv, double temp, double pmid) {
+  const double epsqs = 0.018016 / 0.028966;
+  const double tc = temp - 273.15;
+  const double ew = 610.94 * exp(quot(17.625 * tc, 234.04 + tc));
+  const double ev_sat = 1.00071 * exp(4.5e-8 * pmid) * ew;
+  const double qv_sat = quot(epsqs * ev_sat, pmid - (1 - epsqs) * ev_sat);
+  return dmax(0.0, dmin(1.0, quot(qv, qv_sat)));
+}
 
 // Loads the cell, checks it, runs calcsize and water uptake, writes the
 // size outputs and prepares the amicphys inputs: the part of
@@ -477,12 +493,7 @@ __device__ __forceinline__ void cell_front(const StepArgs &a, const long long c,
 #pragma unroll
   for (int m = 0; m < NMODE; ++m)
     f.wetdens[m] = dmax(1000.0, wetdens_wu[m]);
-  const double epsqs = 0.018016 / 0.028966;
-  const double tc = f.temp - 273.15;
-  const double ew = 610.94 * exp(17.625 * tc / (234.04 + tc));
-  const double ev_sat = 1.00071 * exp(4.5e-8 * f.pmid) * ew;
-  const double qv_sat = epsqs * ev_sat / (f.pmid - (1 - epsqs) * ev_sat);
-  f.relhumgcm = dmax(0.0, dmin(1.0, f.qv / qv_sat));
+  f.relhumgcm = relhum_gcm(f.qv, f.temp, f.pmid);
 }
 
 // Renaming of a cloudy (sub)area, interstitial si and cloud-borne sc,
@@ -664,7 +675,7 @@ __device__ __forceinline__ void cell_step(const StepArgs &a, const long long c) 
   const bool map_gas = a.do_cond || a.do_newnuc;
   const double qgas1[2] = {f.g_soag * fsoag, f.g_h2so4 * 1.0};
 
-  if (f.cld > 0.999) {
+  if (f.cld > kCloudy) {
     cloudy_cell<DIAG>(a, f, o_h2so4, o_soag, oi, oc, dg);
   } else if (f.cld < 1.0e-5) {
     // clear grid cell: the subarea is the grid mean
@@ -977,16 +988,6 @@ __device__ __forceinline__ void run_chemistry(const StepArgs &a, const ChemArgs 
   }
 }
 
-// First half of the pipelined step (condensation on, no diagnostics): the
-// cell's front; cloudy cells finish here; every other cell sets up its
-// clear subarea (and, when partly cloudy, runs the cloudy one), runs the
-// clear subarea up to the SOA loop and hands the state at that point to the
-// solver and the post kernel. The clear-subarea part runs converged for
-// clear and partly cloudy cells alike.
-// With CHEM the cell's chemistry runs between its front and amicphys
-// (run_chemistry), and the subarea set-up takes the pre-chemistry states;
-// the post kernel needs nothing else, as everything it reads of the cell's
-// state comes through the hand-off.
 // The per-particle H2SO4 uptake rate of mode M of cell c as the FP64 step
 // computes it: FP64 water uptake of the mode from the cell's inputs, the
 // calcsize dry diameter and the relative humidity of the size stage, then
@@ -1020,19 +1021,32 @@ __device__ __noinline__ double rate_fp64(const StepArgs &a, const long long c, i
 // (relative error well below 1e-5) a rate within 1e-4 of that threshold may
 // fall on the other side of it than the FP64 step's, so such modes take
 // the FP64 rate instead (a few cells in 10^4).
-__device__ __forceinline__ void guard_soa_threshold(const StepArgs &a, const long long c,
-                                                    double temp, double pmid, const Sub &s,
-                                                    double (&rate)[NMODE], ClearMid &cm,
-                                                    double (&uptk0)[NMODE]) {
-  const double aircon = pmid / (8314.46759100000 * temp);
-#pragma unroll
-  for (int k = 0; k < NMODE; ++k) {
-    if (fabs(uptk0[k] - 1.0e-15) <= 1.0e-4 * 1.0e-15) {
-      rate[k] = rate_fp64(a, c, k);
-      cm.uptk1[k] = rate[k] * (s.num[k] * aircon);
-      uptk0[k] = cm.uptk1[k] * 0.81;
-    }
+__device__ __forceinline__ bool at_soa_threshold(double uptk0) {
+  return fabs(uptk0 - 1.0e-15) <= 1.0e-4 * 1.0e-15;
+}
+
+// Appends cell c's SOA loop to the solver's order list, one append per warp;
+// first_rate: the loop time over its first sub-step, times 0.05.
+__device__ __forceinline__ void append_loop(const StepArgs &a, long long c, double first_rate) {
+  const bool long_loop = first_rate > 0.05 * a.long_steps;
+  const unsigned m = __activemask();
+  const int lane = threadIdx.x & 31;
+  const int leader = __ffs(m) - 1;
+  const unsigned m_long = __ballot_sync(m, long_loop), m_short = m & ~m_long;
+  unsigned b_long = 0, b_short = 0;
+  if (lane == leader) {
+    if (m_long)
+      b_long = atomicAdd(&a.counters[CNT_LONG], (unsigned)__popc(m_long));
+    if (m_short)
+      b_short = atomicAdd(&a.counters[CNT_SHORT], (unsigned)__popc(m_short));
   }
+  b_long = __shfl_sync(m, b_long, leader);
+  b_short = __shfl_sync(m, b_short, leader);
+  const unsigned below = (1u << lane) - 1;
+  if (long_loop)
+    a.order[b_long + __popc(m_long & below)] = (int)c;
+  else
+    a.order[a.ncell - 1 - (b_short + __popc(m_short & below))] = (int)c;
 }
 
 template <class Src>
@@ -1040,38 +1054,30 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
                                             double pmid, double zm, double cld, double pblh,
                                             double relhum, double dgn_pc, Sub &s, ClearMid &cm,
                                             const Src &src);
-// cell_finish's late inputs held in registers (the fused path of pre)
-struct FinishRegs {
-  const double (&ci_)[NPOP];
-  const double (&cg_)[2];
-  const double (&ai_)[NPOP];
-  double h2so4_, soag_;
-  __device__ double ci(int p) const { return ci_[p]; }
-  __device__ double cg(int g) const { return cg_[g]; }
-  __device__ double ai(int p) const { return ai_[p]; }
-  __device__ double h2so4() const { return h2so4_; }
-  __device__ double soag() const { return soag_; }
-};
 template <int SOA, class State>
 __device__ __forceinline__ bool soa_pass(State &st, bool fast);
 
-template <bool CHEM, bool MIXED = false, bool FUSE = false>
-__device__ __forceinline__ void cell_pre(const StepArgs &a, const ChemArgs &ch,
-                                         const long long c) {
+// The pre stage of the step with chemistry: the cell's front (wet sizes
+// from the mode stage), its chemistry (run_chemistry), then cloudy cells
+// finish here; every other cell sets up its clear subarea with the
+// pre-chemistry states (and, when partly cloudy, runs the cloudy one), runs
+// the clear subarea up to the SOA loop and hands the state at that point to
+// the solver and the post kernel. The clear-subarea part runs converged for
+// clear and partly cloudy cells alike. Nothing later needs more, as
+// everything the post kernel reads of the cell's state comes through the
+// hand-off.
+__device__ __forceinline__ void cell_pre_chem(const StepArgs &a, const ChemArgs &ch,
+                                              const long long c) {
   const StepConsts &C = c_k;
   Front f;
   cell_front<false>(a, c, f);
   ChemPre cp;
-  if constexpr (CHEM)
-    run_chemistry(a, ch, c, f, cp);
+  run_chemistry(a, ch, c, f, cp);
   const double dt = a.dt;
   const double fsoag = C.fcvt_soag;
-  if (f.cld > 0.999) {
+  if (f.cld > kCloudy) {
     double o_h2so4, o_soag, oi[NPOP], oc[NPOP];
-    if constexpr (CHEM)
-      cloudy_cell_chem(a, f, cp, o_h2so4, o_soag, oi, oc);
-    else
-      cloudy_cell<false>(a, f, o_h2so4, o_soag, oi, oc, nullptr);
+    cloudy_cell_chem(a, f, cp, o_h2so4, o_soag, oi, oc);
     store_outputs(a, c, o_h2so4, o_soag, oi, oc, f.h2so4, f.soag, f.ai, f.ac);
     return;
   }
@@ -1091,78 +1097,23 @@ __device__ __forceinline__ void cell_pre(const StepArgs &a, const ChemArgs &ch,
       oc[p] = f.qc[p];
   } else {
     double gcl[2];
-    if constexpr (CHEM)
-      partly_cloudy_setup_chem(a, f, cp, s, gcl, rh, ci, cg, oc);
-    else
-      partly_cloudy_setup<false>(a, f, s, gcl, rh, ci, cg, oc, nullptr);
+    partly_cloudy_setup_chem(a, f, cp, s, gcl, rh, ci, cg, oc);
   }
-  double qgas1[2] = {f.g_soag * fsoag, f.g_h2so4 * 1.0};
-  if constexpr (CHEM) {
-    qgas1[0] = cp.g1[0] * fsoag;
-    qgas1[1] = cp.g1[1] * 1.0;
-  }
+  const double qgas1[2] = {cp.g1[0] * fsoag, cp.g1[1] * 1.0};
   ClearMid cm;
   double uptk0[NMODE], rate[NMODE];
 #pragma unroll
   for (int k = 0; k < NMODE; ++k)
     rate[k] = a.aux[(AUX_RATE + k) * (size_t)a.ncell + c];
   clear_prefix<false>(a, dt, f.temp, f.pmid, rate, qgas1, s, cm, uptk0);
-  if constexpr (MIXED) {
-    if (a.do_cond)
-      guard_soa_threshold(a, c, f.temp, f.pmid, s, rate, cm, uptk0);
-  }
 
   // queue the cell: solver state and hand-off at the start of the SOA loop
   SoaState st;
   soa_init(st, (double)(int)(dt / 1), f.temp, f.pmid, s, uptk0);
   const double first_rate = soa_first_rate(st) * st.dtfull;
-  if constexpr (FUSE) {
-    // a short loop (first sub-step at least 1/inline_scale of the step)
-    // runs here and the cell finishes without the hand-off, with the same
-    // arithmetic as the solver and post kernels
-    if (first_rate <= 0.05 * a.inline_scale) {
-      const bool fast = soa_begin(st);
-      while (soa_pass<MIXED ? 1 : 0>(st, fast)) {
-      }
-      if (st.niter > 1000)
-        atomicOr(a.flags, MAM4B_FLAG_SOA_NITER_LIMIT);
-      s.gas[0] = st.g;
-#pragma unroll
-      for (int k = 0; k < NMODE; ++k)
-        s.aer[0][k] = st.a[k];
-      store_cloudborne(a, c, oc, f.ac);
-      const FinishRegs src{ci, cg, f.ai, f.h2so4, f.soag};
-      cell_finish(a, c, f.temp, f.pmid, f.zm, f.cld, f.pblh, rh, f.dgn_a[3], s, cm, src);
-      return;
-    }
-  }
-  const bool long_loop = first_rate > 0.05 * a.long_steps;
-  // warp-aggregated appends: the slot (in discovery order, which keeps the
-  // post kernel's cell accesses coalesced) and the solver order entry
-  const unsigned m = __activemask();
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(m) - 1;
-  const unsigned m_long = __ballot_sync(m, long_loop), m_short = m & ~m_long;
-  unsigned base = 0, b_long = 0, b_short = 0;
-  if (lane == leader) {
-    base = atomicAdd(&a.counters[CNT_QUEUED], (unsigned)__popc(m));
-    if (m_long)
-      b_long = atomicAdd(&a.counters[CNT_LONG], (unsigned)__popc(m_long));
-    if (m_short)
-      b_short = atomicAdd(&a.counters[CNT_SHORT], (unsigned)__popc(m_short));
-  }
-  base = __shfl_sync(m, base, leader);
-  b_long = __shfl_sync(m, b_long, leader);
-  b_short = __shfl_sync(m, b_short, leader);
-  const unsigned below = (1u << lane) - 1;
-  const unsigned slot = base + __popc(m & below);
-  a.task[slot] = (int)c;
-  if (long_loop)
-    a.order[b_long + __popc(m_long & below)] = (int)slot;
-  else
-    a.order[a.ncell - 1 - (b_short + __popc(m_short & below))] = (int)slot;
+  append_loop(a, c, first_rate);
   const size_t n = (size_t)a.ncell;
-  double *q = a.soa + slot;
+  double *q = a.soa + c;
   q[SOA_G * n] = st.g;
 #pragma unroll
   for (int k = 0; k < NMODE; ++k) {
@@ -1171,7 +1122,7 @@ __device__ __forceinline__ void cell_pre(const StepArgs &a, const ChemArgs &ch,
     q[(SOA_UPTK + k) * n] = st.uptk[k];
   }
   q[SOA_G0 * n] = st.g0;
-  double *h = a.hand + slot;
+  double *h = a.hand + c;
   h[H_GAS1 * n] = s.gas[1];
   double pop[NPOP];
   sub_to_pop(s, pop);
@@ -1222,13 +1173,15 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
   clear_suffix<false, true>(a, dt, temp, pmid, zm, pblh, relhum, dgn_pc, unused, unused, cm, s,
                             nullptr, 0.0, a.aux + AUX_COAG * n + c, n);
   // recombination (form_gcm_of_gases_and_aerosols_from_subareas)
-  const double fsoag = C.fcvt_soag;
+  const GuardedDivisor dsoag(C.fcvt_soag);
+  constexpr GuardedDivisor organic = constant_divisor(K::fcvt_aer(0));
+  auto over_fcvt = [&](double v, int x) { return x == 0 || x == 2 ? organic.under(v) : v; };
   double o_h2so4, o_soag, oi[NPOP];
   double po[NPOP];
   sub_to_pop(s, po);
   if (cld < 1.0e-5) {
     const double f = 1.0 - 0.0;
-    o_soag = dmax(0.0, 0.0 + (s.gas[0] / fsoag) * f);
+    o_soag = dmax(0.0, 0.0 + dsoag.under(s.gas[0]) * f);
     o_h2so4 = dmax(0.0, 0.0 + (s.gas[1] / 1.0) * f);
 #pragma unroll
     for (int m = 0; m < NMODE; ++m) {
@@ -1237,12 +1190,12 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
       for (int x = 0; x < NAER; ++x) {
         const int sl = K::aer_slot(x, m);
         if (sl >= 0)
-          oi[sl] = dmax(0.0, 0.0 + (po[sl] / K::fcvt_aer(x)) * f);
+          oi[sl] = dmax(0.0, 0.0 + over_fcvt(po[sl], x) * f);
       }
     }
   } else {
     const double fclea = 1.0 - cld;
-    o_soag = dmax(0.0, (0.0 + (s.gas[0] / fsoag) * fclea) + src.cg(0));
+    o_soag = dmax(0.0, (0.0 + dsoag.under(s.gas[0]) * fclea) + src.cg(0));
     o_h2so4 = dmax(0.0, (0.0 + (s.gas[1] / 1.0) * fclea) + src.cg(1));
 #pragma unroll
     for (int m = 0; m < NMODE; ++m) {
@@ -1252,7 +1205,7 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
       for (int x = 0; x < NAER; ++x) {
         const int sl = K::aer_slot(x, m);
         if (sl >= 0)
-          oi[sl] = dmax(0.0, (0.0 + (po[sl] / K::fcvt_aer(x)) * fclea) + src.ci(sl));
+          oi[sl] = dmax(0.0, (0.0 + over_fcvt(po[sl], x) * fclea) + src.ci(sl));
       }
     }
   }
@@ -1263,8 +1216,8 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
   store_interstitial(a, c, o_h2so4, o_soag, oi, src.h2so4(), src.soag(), ai);
 }
 
-// cell_finish's late inputs read from the hand-off of queue slot `slot`
-// and the cell's inputs (post_kernel)
+// cell_finish's late inputs read from the hand-off and the cell's inputs
+// (post_kernel)
 struct FinishLoads {
   const StepArgs &a;
   long long c;
@@ -1277,18 +1230,19 @@ struct FinishLoads {
   __device__ double soag() const { return __ldg(a.in[MAM4B_IN_SOAG] + c); }
 };
 
-// Second half of a queued cell: the state at the SOA loop (hand-off), the
-// loop's result (solver), then cell_finish.
-__device__ __forceinline__ void cell_post(const StepArgs &a, unsigned slot) {
+// Second half of a cell with a clear subarea: the state at the SOA loop
+// (hand-off), the loop's result (solver), then cell_finish.
+__device__ __forceinline__ void cell_post(const StepArgs &a, const long long c) {
   const size_t n = (size_t)a.ncell;
-  const long long c = a.task[slot];
+  const double cld = __ldg(a.in[MAM4B_IN_CLD] + c);
+  if (cld > kCloudy)
+    return;
   const double temp = __ldg(a.in[MAM4B_IN_T] + c);
   const double pmid = __ldg(a.in[MAM4B_IN_P] + c);
   const double zm = __ldg(a.in[MAM4B_IN_ZM] + c);
-  const double cld = __ldg(a.in[MAM4B_IN_CLD] + c);
   const double pblh = __ldg(a.pblh + c / a.nlev);
-  const double *h = a.hand + slot;
-  const double *q = a.soa + slot;
+  const double *h = a.hand + c;
+  const double *q = a.soa + c;
   Sub s;
   {
     double pop[NPOP];
@@ -1334,7 +1288,7 @@ __device__ __forceinline__ void cell_step_chem(const StepArgs &a, const ChemArgs
   const double fsoag = C.fcvt_soag;
   const bool map_gas = a.do_cond || a.do_newnuc;
   const double qgas1[2] = {cp.g1[0] * fsoag, cp.g1[1] * 1.0};
-  if (f.cld > 0.999) {
+  if (f.cld > kCloudy) {
     cloudy_cell_chem(a, f, cp, o_h2so4, o_soag, oi, oc);
   } else if (f.cld < 1.0e-5) {
     Sub s;
@@ -1401,11 +1355,11 @@ __global__ void __launch_bounds__(128) chem_step_kernel(const __grid_constant__ 
 // chosen per device by mam4b_autotune (include/mam4b.h). The arithmetic is
 // the same in every variant, so their results are bit for bit equal.
 // Register caps compiled:
-//   size_kernel 255, 128, 96; pre_kernel and post_kernel 255, 168, 128;
+//   front_kernel 255, 128, 96; pre_kernel and post_kernel 255, 168, 128;
 //   soa_kernel 64, 96, 128.
 
-// Stage 1 of the pipelined step, one thread per cell: calcsize for the dry
-// diameters (an output), the relative humidity of water uptake and the
+// Stage 1 of the step with chemistry, one thread per cell: calcsize for the
+// dry diameters (an output), the relative humidity of water uptake and the
 // H2SO4 diffusivity and mean free path.
 __device__ __forceinline__ void size_cell(const StepArgs &a, const long long c) {
   const StepConsts &C = c_k;
@@ -1431,18 +1385,475 @@ __device__ __forceinline__ void size_cell(const StepArgs &a, const long long c) 
   a.aux[AUX_FPATH * n + c] = fp;
 }
 
-// LOOP: grid-stride loop over cells (cells_per_thread > 1); without it one
-// cell per thread, which leaves the register allocation of the body as is.
+__global__ void __launch_bounds__(128, 4) size_kernel(const __grid_constant__ StepArgs a) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < a.ncell)
+    size_cell(a, c);
+}
+
+// Stage 1, one thread per (cell, mode): a block holds two modes of
+// blockDim.x / 2 cells, accumulation and aitken (blockIdx.y 0) or coarse and
+// primary carbon, a warp one of them. Everything up to the SOA loop of a
+// cell treats its modes apart but for the aitken <-> accumulation exchange
+// of calcsize and renaming, which pass a few values through shared memory
+// (XF_*); the cell's own scalars go to the accumulation mode, which waits
+// for renaming, and to primary carbon, which has the fewest species. A whole
+// cell in one thread needs more than 255 registers and keeps 7.6 warps per
+// SM resident. The mode is a run-time value, its tables (c_modes) in
+// constant memory: with one copy of the code per mode the warps of an SM
+// fetch four times the instructions, and waiting for them takes two thirds
+// of the time.
+enum {
+  XF_DV_I = 0,    // accumulation, aitken: dry volumes, numbers
+  XF_DV_C = 2,
+  XF_N_I = 4,
+  XF_N_C = 6,
+  XF_NOXF_I = 8,  // accumulation: volumes without an aitken counterpart
+  XF_NOXF_C = 9,
+  XF_COMMON = 10,  // common species [accumulation, aitken][interstitial, cloud-borne][4]
+  XF_RN_I = 26,    // rename: number and 4 species moved
+  XF_RN_C = 31,
+  XF_FIELDS = 36
+};
+struct ModeTables {
+  int nspec[NMODE], spec0[NMODE], numslot[NMODE];
+  double dmin[NMODE], dmax[NMODE], dnom[NMODE];
+  double fcvt[NMODE][7];
+  // position of species s among the four that the aitken and accumulation
+  // modes share (SO4, SOA, NaCl, MOM), -1: none
+  int common[NMODE][7];
+  int soa[NMODE], pom[NMODE];  // position of SOA and POM in the mode, -1: none
+};
+constexpr ModeTables make_mode_tables() {
+  ModeTables t = {};
+  for (int m = 0; m < NMODE; ++m) {
+    constexpr int nspec[NMODE] = {7, 4, 7, 3}, spec0[NMODE] = {0, 8, 13, 21},
+                  num[NMODE] = {7, 12, 20, 24};
+    constexpr int spec[NMODE][7] = {{1, 2, 0, 3, 5, 4, 6},
+                                    {1, 0, 4, 6, -1, -1, -1},
+                                    {5, 4, 1, 3, 2, 0, 6},
+                                    {2, 3, 6, -1, -1, -1, -1}};
+    t.nspec[m] = nspec[m];
+    t.spec0[m] = spec0[m];
+    t.numslot[m] = num[m];
+    t.soa[m] = t.pom[m] = -1;
+    constexpr double dmin[NMODE] = {5.35e-8, 8.7e-9, 1e-6, 1e-8},
+                     dmax[NMODE] = {4.4e-7, 5.2e-8, 4e-6, 1e-7},
+                     dnom[NMODE] = {1.1e-7, 2.6e-8, 2e-6, 5e-8};
+    t.dmin[m] = dmin[m];
+    t.dmax[m] = dmax[m];
+    t.dnom[m] = dnom[m];
+    for (int s = 0; s < 7; ++s) {
+      const int x = spec[m][s];
+      t.fcvt[m][s] = x == 0 || x == 2 ? 8.000000000000000E-002 : 1.0;
+      t.common[m][s] =
+          m > 1 ? -1 : x == 1 ? 0 : x == 0 ? 1 : x == 4 ? 2 : x == 6 ? 3 : -1;
+      if (x == 0)
+        t.soa[m] = s;
+      if (x == 2)
+        t.pom[m] = s;
+    }
+  }
+  return t;
+}
+__constant__ ModeTables c_modes = make_mode_tables();
+struct FrontMode {
+  int m, ns, s0, num;           // mode, its species count, first slot, number slot
+  double ai[7], ac[7], ni, nc;  // the mode's inputs (zero beyond its species)
+  double pn_i, pn_c;            // number tendencies of calcsize
+  double num_i, num_c, dv_i, dv_c;
+  double si[7], sc[7], sni, snc;  // cloudy subarea
+};
+
+__device__ __forceinline__ void front_load(const StepArgs &a, long long c, double adj_inv,
+                                           FrontMode &f, double *x, int stride) {
+  const StepConsts &C = c_k;
+  const int m = f.m;
+#pragma unroll
+  for (int s = 0; s < 7; ++s) {
+    f.ai[s] = f.ac[s] = 0.0;
+    if (s < f.ns) {
+      f.ai[s] = __ldg(a.in[MAM4B_IN_AER_I + f.s0 + s] + c);
+      f.ac[s] = __ldg(a.in[MAM4B_IN_AER_C + f.s0 + s] + c);
+    }
+  }
+  f.ni = __ldg(a.in[MAM4B_IN_AER_I + f.num] + c);
+  f.nc = __ldg(a.in[MAM4B_IN_AER_C + f.num] + c);
+  f.dv_i = f.dv_c = 0.0;
+  double chk = f.ni + f.nc;
+#pragma unroll
+  for (int s = 0; s < 7; ++s)
+    if (s < f.ns) {
+      f.dv_i += dmax(0.0, f.ai[s]) * C.inv_density[m][s];
+      f.dv_c += dmax(0.0, f.ac[s]) * C.inv_density[m][s];
+      chk += f.ai[s] + f.ac[s];
+    }
+  if (!isfinite(chk))
+    atomicOr(a.flags, MAM4B_FLAG_NONFINITE_INPUT);
+  f.num_i = f.ni < 0 ? 0.0 : f.ni;
+  f.num_c = f.nc < 0 ? 0.0 : f.nc;
+  f.pn_i = f.pn_c = 0.0;
+  if (m >= 2) {
+    adjust_num_sizes(f.dv_i, f.dv_c, f.ni, f.nc, a.dt, C.n2v_min[m], C.n2v_max[m], adj_inv,
+                     f.num_i, f.num_c, f.pn_i, f.pn_c);
+    return;
+  }
+  x[(XF_DV_I + m) * stride] = f.dv_i;
+  x[(XF_DV_C + m) * stride] = f.dv_c;
+  x[(XF_N_I + m) * stride] = f.num_i;
+  x[(XF_N_C + m) * stride] = f.num_c;
+  if (m == 0) {
+    AitAccTotals v;
+    accumulation_noxf(C, f.ai[1], f.ai[3], f.ai[4], f.ac[1], f.ac[3], f.ac[4], v);
+    x[XF_NOXF_I * stride] = v.noxf_i;
+    x[XF_NOXF_C * stride] = v.noxf_c;
+  }
+#pragma unroll
+  for (int s = 0; s < 7; ++s) {
+    const int k = c_modes.common[m][s];
+    if (k >= 0) {
+      x[(XF_COMMON + 8 * m + k) * stride] = f.ai[s];
+      x[(XF_COMMON + 8 * m + 4 + k) * stride] = f.ac[s];
+    }
+  }
+}
+
+// Partition factor pair of get_partition_factors (mam4_amicphys.hpp:414-449)
+__device__ __forceinline__ void partition(double q_i, double q_c, double fcldy,
+                                          const GuardedDivisor &dy, const GuardedDivisor &dc,
+                                          double fclea, double &fc, double &fy) {
+  const double cldbrn_cldy = dy.under(q_c);
+  const double intrst_cldy = dmax(0.0, ((q_i + q_c) - cldbrn_cldy));
+  const double intrst_clea = dc.under(q_i - fcldy * intrst_cldy);
+  double r = quot(dmax(1.e-35, intrst_clea * fclea), dmax(1.e-35, q_i));
+  r = dmax(0.0, dmin(1.0, r));
+  fc = dc.under(r);
+  fy = dy.under(1 - r);
+}
+
+// The mode from calcsize to the SOA loop: its dry diameter (an output), the
+// calcsize update in amicphys units, the clear subarea at the SOA loop (into
+// the hand-off; cells that are not cloudy) and the cloudy subarea before
+// renaming. The aitken mode renames and leaves what
+// moves in x; the accumulation mode takes it in front_out.
+__device__ __forceinline__ void front_mode(const StepArgs &a, long long c, double cld,
+                                           double adj_inv, FrontMode &f, double *x, int stride) {
+  const StepConsts &C = c_k;
+  const int m = f.m;
+  const size_t n = (size_t)a.ncell;
+  const double dt = a.dt;
+  double qi[7], qc[7], qni, qnc;
+  {
+    // volume and number of the dry diameter, and their size bounds
+    double drv = f.dv_i, num = f.num_i, lo = C.n2v_lo_wide[m], hi = C.n2v_hi_wide[m];
+    AitAccExchange e;
+    e.ait2acc = e.acc2ait = false;
+    if (m < 2) {
+      AitAccTotals t;
+      t.dv_i_acc = x[XF_DV_I * stride];
+      t.dv_i_ait = x[(XF_DV_I + 1) * stride];
+      t.dv_c_acc = x[XF_DV_C * stride];
+      t.dv_c_ait = x[(XF_DV_C + 1) * stride];
+      t.n_i_acc = x[XF_N_I * stride];
+      t.n_i_ait = x[(XF_N_I + 1) * stride];
+      t.n_c_acc = x[XF_N_C * stride];
+      t.n_c_ait = x[(XF_N_C + 1) * stride];
+      t.noxf_i = x[XF_NOXF_I * stride];
+      t.noxf_c = x[XF_NOXF_C * stride];
+      e = aitken_accumulation_exchange(C, t, adj_inv);
+      if (e.ait2acc || e.acc2ait) {
+        // number and volume that leave the aitken mode
+        const double ndi = (e.xt00 - e.xt10) * dt;
+        const double vdi =
+            (t.dv_i_ait * e.xv_ait2acc - (t.dv_i_acc - e.noxf_i) * e.xv_acc2ait) * dt;
+        drv = dmax(0.0, m == 1 ? t.dv_i_ait - vdi : t.dv_i_acc + vdi);
+        num = dmax(0.0, m == 1 ? t.n_i_ait - ndi : t.n_i_acc + ndi);
+        lo = C.n2v_min[m];
+        hi = C.n2v_max[m];
+      }
+      // calcsize adds the transfers one after the other, each with its sign
+      if (e.ait2acc) {
+        f.pn_i += m == 1 ? -e.xt00 : e.xt00;
+        f.pn_c += m == 1 ? -e.xt01 : e.xt01;
+      }
+      if (e.acc2ait) {
+        f.pn_i += m == 1 ? e.xt10 : -e.xt10;
+        f.pn_c += m == 1 ? e.xt11 : -e.xt11;
+      }
+    }
+    const double dgn = size_after_transfer(drv, num, lo, hi, c_modes.dmax[m], c_modes.dmin[m],
+                                           c_modes.dnom[m], C.diam_fac[m]);
+    a.out[MAM4B_OUT_DGN_A + m][c] = dgn;
+    if (m == 3 && !(cld > kCloudy))
+      a.hand[H_DGN_PC * n + c] = dgn;
+#pragma unroll
+    for (int s = 0; s < 7; ++s) {
+      if (s >= f.ns)
+        continue;
+      double pi = 0.0, pc = 0.0;
+      const int k = c_modes.common[m][s];
+      if (k >= 0 && e.ait2acc) {
+        const double xi = dmax(0.0, x[(XF_COMMON + 8 + k) * stride]) * e.xv_ait2acc;
+        const double xc = dmax(0.0, x[(XF_COMMON + 12 + k) * stride]) * e.xv_ait2acc;
+        pi += m == 1 ? -xi : xi;
+        pc += m == 1 ? -xc : xc;
+      }
+      if (k >= 0 && e.acc2ait) {
+        const double xi = dmax(0.0, x[(XF_COMMON + k) * stride]) * e.xv_acc2ait;
+        const double xc = dmax(0.0, x[(XF_COMMON + 4 + k) * stride]) * e.xv_acc2ait;
+        pi += m == 1 ? xi : -xi;
+        pc += m == 1 ? xc : -xc;
+      }
+      qi[s] = dmax(0.0, dmax(0.0, f.ai[s] + pi * dt) * C.to_vmr[2 + f.s0 + s]);
+      qc[s] = dmax(0.0, dmax(0.0, f.ac[s] + pc * dt) * C.to_vmr[2 + f.s0 + s]);
+    }
+    qni = dmax(0.0, dmax(0.0, f.ni + f.pn_i * dt) * C.to_vmr[2 + f.num]);
+    qnc = dmax(0.0, dmax(0.0, f.nc + f.pn_c * dt) * C.to_vmr[2 + f.num]);
+  }
+  const bool cloudy = cld > kCloudy, clear = cld < 1.0e-5;
+  // subarea factors: clear (number, mass), cloudy interstitial (number,
+  // mass); a clear or cloudy cell is its only subarea
+  double fn_c = 1.0, fm_c = 1.0, fn_y = 1.0, fm_y = 1.0;
+  const double fcldy = cld, fclea = 1.0 - fcldy;
+  const GuardedDivisor dy(cloudy ? 1.0 : fcldy);
+  if (!cloudy && !clear) {
+    const GuardedDivisor dc(fclea);
+    double ti = 0.0, tc = 0.0;
+#pragma unroll
+    for (int s = 0; s < 7; ++s)
+      if (s < f.ns) {
+        ti = ti + qi[s];
+        tc = tc + qc[s];
+      }
+    partition(qni, qnc, fcldy, dy, dc, fclea, fn_c, fn_y);
+    partition(ti, tc, fcldy, dy, dc, fclea, fm_c, fm_y);
+  }
+  if (!cloudy) {
+    // the clear subarea at the SOA loop (times one in a clear cell)
+    double *h = a.hand + c;
+    double soa = 0.0, pom = 0.0;
+#pragma unroll
+    for (int s = 0; s < 7; ++s) {
+      if (s >= f.ns)
+        continue;
+      const double q = (qi[s] * fm_c) * c_modes.fcvt[m][s];
+      h[(H_POP + f.s0 + s) * n] = q;
+      if (s == c_modes.soa[m])
+        soa = q;
+      if (s == c_modes.pom[m])
+        pom = q;
+    }
+    h[(H_POP + f.num) * n] = (qni * fn_c) * 1;
+    if (m == 1) {
+      h[H_SV_SO4 * n] = (qi[0] * fm_c) * 1;
+      h[H_SV_SOA * n] = soa;
+    }
+    a.soa[(SOA_A + m) * n + c] = soa;
+    a.soa[(SOA_OPOA + m) * n + c] = 0.0 + (m == 3 ? 0.0 : 0.1) * dmax(pom, 0.0);
+  }
+  // the cloudy subarea, or the cloud-borne populations of a clear cell
+#pragma unroll
+  for (int s = 0; s < 7; ++s) {
+    if (s >= f.ns)
+      continue;
+    f.si[s] = (qi[s] * fm_y) * c_modes.fcvt[m][s];
+    f.sc[s] = clear ? qc[s] : dy.under(qc[s]) * c_modes.fcvt[m][s];
+  }
+  f.sni = (qni * fn_y) * 1;
+  f.snc = clear ? qnc : dy.under(qnc) * 1;
+  if (m == 1 && !clear) {
+    // renaming (rename_subarea<true>, no growth): aitken volumes in AeroId
+    // order SOA, SO4, NaCl, MOM
+    double xn = 0.0, xv = 0.0;
+    bool renamed = false;
+    if (a.do_rename) {
+      constexpr int order[4] = {1, 0, 2, 3};
+      double ti = 0.0, tc = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        ti += f.si[order[k]] * K::mass_2_vol(K::mode_spec(1, order[k]));
+        tc += f.sc[order[k]] * K::mass_2_vol(K::mode_spec(1, order[k]));
+      }
+      renamed = rename_fractions<true>(C, ti - 0.0, 0.0, tc - 0.0, 0.0, f.sni, f.snc, xn, xv);
+    }
+    double mn_i = 0.0, mn_c = 0.0, mi[4] = {0, 0, 0, 0}, mc[4] = {0, 0, 0, 0};
+    if (renamed) {
+      mn_i = f.sni * xn;
+      mn_c = f.snc * xn;
+      f.sni -= mn_i;
+      f.snc -= mn_c;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        mi[k] = f.si[k] * xv;
+        mc[k] = f.sc[k] * xv;
+        f.si[k] -= mi[k];
+        f.sc[k] -= mc[k];
+      }
+    }
+    x[XF_RN_I * stride] = mn_i;
+    x[XF_RN_C * stride] = mn_c;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      x[(XF_RN_I + 1 + k) * stride] = mi[k];
+      x[(XF_RN_C + 1 + k) * stride] = mc[k];
+    }
+  }
+}
+
+// What leaves the stage after renaming: cloud-borne tendencies; the
+// interstitial tendencies of a cloudy cell, or the cloudy subarea's
+// contributions to the grid means of a partly cloudy one.
+__device__ __forceinline__ void front_out(const StepArgs &a, long long c, double cld,
+                                          FrontMode &f, const double *x, int stride) {
+  const StepConsts &C = c_k;
+  const int m = f.m;
+  const size_t n = (size_t)a.ncell;
+  const bool cloudy = cld > kCloudy, clear = cld < 1.0e-5;
+  double *h = a.hand + c;
+  const GuardedDivisor per_dt(a.dt);
+  constexpr GuardedDivisor organic = constant_divisor(K::fcvt_aer(0));
+  static_assert(K::fcvt_aer(0) == K::fcvt_aer(2), "SOA and POM share their unit factor");
+  const double w = cloudy ? 1.0 : cld;
+  if (m == 0 && !clear) {
+    f.sni += x[XF_RN_I * stride];
+    f.snc += x[XF_RN_C * stride];
+  }
+#pragma unroll
+  for (int s = 0; s <= 7; ++s) {
+    if (s >= f.ns && s < 7)
+      continue;
+    const bool number = s == 7;
+    const int p = number ? f.num : f.s0 + s;
+    double vi = number ? f.sni : f.si[s < 7 ? s : 0], vc = number ? f.snc : f.sc[s < 7 ? s : 0];
+    const double ac = number ? f.nc : f.ac[s < 7 ? s : 0];
+    if (!number && !clear) {
+      const int k = c_modes.common[m][s < 7 ? s : 0];
+      if (m == 0 && k >= 0) {
+        vi += x[(XF_RN_I + 1 + k) * stride];
+        vc += x[(XF_RN_C + 1 + k) * stride];
+      }
+      if (c_modes.fcvt[m][s < 7 ? s : 0] != 1.0) {
+        vi = organic.under(vi);
+        vc = organic.under(vc);
+      }
+    }
+    const double oc = clear ? vc : 0.0 + vc * w;
+    a.out[MAM4B_OUT_TEND + 27 + p][c] = per_dt.under(oc * C.to_mmr[2 + p] - ac);
+    if (cloudy) {
+      const double ai = __ldg(a.in[MAM4B_IN_AER_I + p] + c);
+      a.out[MAM4B_OUT_TEND + 2 + p][c] =
+          per_dt.under(dmax(0.0, 0.0 + vi * w) * C.to_mmr[2 + p] - ai);
+    } else if (!clear) {
+      h[(H_CI + p) * n] = vi * w;
+    }
+  }
+}
+
+// The cell's scalars for the mode stage: humidity of water uptake, H2SO4
+// diffusivity and mean free path.
+__device__ __forceinline__ void front_uptake(const StepArgs &a, long long c, double cld) {
+  const size_t n = (size_t)a.ncell;
+  const double temp = __ldg(a.in[MAM4B_IN_T] + c), pmid = __ldg(a.in[MAM4B_IN_P] + c);
+  a.aux[AUX_RH * n + c] = water_uptake_rh(__ldg(a.in[MAM4B_IN_QV] + c), temp, pmid, cld);
+  double gd, fp;
+  h2so4_diffusivity(temp, pmid, gd, fp);
+  a.aux[AUX_GDIFF * n + c] = gd;
+  a.aux[AUX_FPATH * n + c] = fp;
+}
+// The cell's gases: gases and relative humidity of the clear subarea
+// (clear_prefix) and the equilibrium SOA gas for the SOA loop, or the gas
+// tendencies of a cloudy cell.
+__device__ __forceinline__ void front_gases(const StepArgs &a, long long c, double cld) {
+  const StepConsts &C = c_k;
+  const size_t n = (size_t)a.ncell;
+  const double temp = __ldg(a.in[MAM4B_IN_T] + c), pmid = __ldg(a.in[MAM4B_IN_P] + c);
+  const double qv = __ldg(a.in[MAM4B_IN_QV] + c);
+  const double h2so4 = __ldg(a.in[MAM4B_IN_H2SO4] + c), soag = __ldg(a.in[MAM4B_IN_SOAG] + c);
+  {
+    const double chk = temp + pmid + __ldg(a.in[MAM4B_IN_ZM] + c) + qv + cld + h2so4 + soag +
+                       __ldg(a.pblh + c / a.nlev);
+    if (!isfinite(chk))
+      atomicOr(a.flags, MAM4B_FLAG_NONFINITE_INPUT);
+  }
+  const GuardedDivisor per_dt(a.dt);
+  const double g_h2so4 = dmax(0.0, h2so4 * C.to_vmr[0]), g_soag = dmax(0.0, soag * C.to_vmr[1]);
+  if (cld > kCloudy) {
+    const double w = 1.0;
+    a.out[MAM4B_OUT_TEND + 0][c] =
+        per_dt.under(dmax(0.0, 0.0 + g_h2so4 * w) * C.to_mmr[0] - h2so4);
+    a.out[MAM4B_OUT_TEND + 1][c] = per_dt.under(dmax(0.0, 0.0 + g_soag * w) * C.to_mmr[1] - soag);
+    return;
+  }
+  double rh = relhum_gcm(qv, temp, pmid);
+  double gcl[2] = {g_soag, g_h2so4};
+  double *h = a.hand + c;
+  if (!(cld < 1.0e-5)) {
+    // gases: clear keeps the grid mean, cloudy gets the remainder
+    const double fcldy = cld, fclea = 1.0 - fcldy;
+    const GuardedDivisor dy(fcldy), dc(fclea);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      double gcy = dy.under(gcl[g] - fclea * gcl[g]);
+      if (gcy < 0) {
+        gcy = 0;
+        gcl[g] = dc.under(gcl[g]);
+      }
+      h[(H_CG + g) * n] = gcy * fcldy;
+    }
+    rh = bound(0.0, 1.0, dc.under(rh - fcldy));
+  }
+  const double gas0 = gcl[0] * C.fcvt_soag;
+  double gas1 = gcl[1] * 1.0, netprod = 0.0;
+  const double qgas1 = g_h2so4 * 1.0;
+  if (a.optaa == 2) {
+    netprod = per_dt.under(gas1 - qgas1);
+    gas1 = (netprod >= 0) ? qgas1 : 0;
+  }
+  h[H_GAS1 * n] = gas1;
+  h[H_NETPROD * n] = netprod;
+  h[H_RELHUM * n] = rh;
+  h[H_SOAG0 * n] = gas0;
+  a.soa[SOA_G * n + c] = gas0;
+  a.soa[SOA_G0 * n + c] = soa_equilibrium_gas(temp, pmid);
+}
+
+// LOOP: grid-stride loop over groups of cells (cells_per_thread > 1).
+// Dynamic shared memory: XF_FIELDS doubles per cell.
 template <int R, bool LOOP>
-__global__ void __maxnreg__(R) size_kernel(const __grid_constant__ StepArgs a) {
-  const long long c0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if constexpr (LOOP) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-#pragma unroll 1
-    for (long long c = c0; c < a.ncell; c += stride)
-      size_cell(a, c);
-  } else if (c0 < a.ncell) {
-    size_cell(a, c0);
+__global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) {
+  extern __shared__ double s_x[];
+  const int cells = blockDim.x / 2;
+  const int k = threadIdx.x % cells;
+  double *x = s_x + k;
+  FrontMode f;
+  f.m = 2 * blockIdx.y + threadIdx.x / cells;
+  f.ns = c_modes.nspec[f.m];
+  f.s0 = c_modes.spec0[f.m];
+  f.num = c_modes.numslot[f.m];
+  const double adj_inv = safe_denominator(dmax(86400.0, a.dt));
+  for (long long c = blockIdx.x * (long long)cells + k; c - k < a.ncell;
+       c += gridDim.x * (long long)cells) {
+    const bool valid = c < a.ncell;
+    const double cld = valid ? __ldg(a.in[MAM4B_IN_CLD] + c) : 0.0;
+    if (valid)
+      front_load(a, c, adj_inv, f, x, cells);
+    if (blockIdx.y == 0)
+      __syncthreads();
+    if (valid) {
+      front_mode(a, c, cld, adj_inv, f, x, cells);
+      if (f.m == 3)
+        front_uptake(a, c, cld);
+      if (f.m == 0)
+        front_gases(a, c, cld);
+    }
+    if (blockIdx.y == 0)
+      __syncthreads();
+    if (valid)
+      front_out(a, c, cld, f, x, cells);
+    if constexpr (!LOOP)
+      break;
+    if (blockIdx.y == 0)
+      __syncthreads();  // before the next cells' values overwrite these
   }
 }
 
@@ -1548,7 +1959,7 @@ __global__ void pair_kernel(const __grid_constant__ StepArgs a) {
   const int sm = coag_src(p), dm = coag_dst(p);
   const double temp = __ldg(a.in[MAM4B_IN_T] + c);
   const double pmid = __ldg(a.in[MAM4B_IN_P] + c);
-  const double aircon = pmid / (8314.46759100000 * temp);
+  const double aircon = quot(pmid, 8314.46759100000 * temp);
   const double dens_s = dmax(1000.0, a.out[MAM4B_OUT_WETDENS + sm][c]);
   const double dens_d = dmax(1000.0, a.out[MAM4B_OUT_WETDENS + dm][c]);
   const CoagTables T = {kCoagBm0ij, kCoagBm3i, kCoagBm0};
@@ -1584,13 +1995,76 @@ __global__ void pair_kernel(const __grid_constant__ StepArgs a) {
   cc[(9 + p) * n] = bjj0;
 }
 
-// FUSE: cells with short SOA loops finish here (StepArgs::inline_scale)
+// Stage 4, one thread per cell: the uptake rates of the clear subarea from
+// the per-particle rates of the mode stage, and the solver's order of the
+// loops. With MIXED a mode at the threshold of the SOA loop takes the FP64
+// rate. FUSE: cells with short SOA loops finish here
+// (StepArgs::inline_scale).
+template <bool MIXED, bool FUSE>
+__device__ __forceinline__ void pre_cell(const StepArgs &a, const long long c) {
+  const size_t n = (size_t)a.ncell;
+  if (__ldg(a.in[MAM4B_IN_CLD] + c) > kCloudy) {
+    if constexpr (FUSE)
+      a.done[c] = 1;
+    return;
+  }
+  const double temp = __ldg(a.in[MAM4B_IN_T] + c), pmid = __ldg(a.in[MAM4B_IN_P] + c);
+  const double aircon = quot(pmid, 8314.46759100000 * temp);
+  double *h = a.hand + c, *q = a.soa + c;
+  SoaState st;
+#pragma unroll
+  for (int k = 0; k < NMODE; ++k) {
+    const double num = h[(H_POP + K::numslot(k)) * n];
+    double uptk1 = a.aux[(AUX_RATE + k) * n + c] * (num * aircon);
+    st.uptk[k] = uptk1 * 0.81;
+    if constexpr (MIXED) {
+      if (at_soa_threshold(st.uptk[k])) {
+        uptk1 = rate_fp64(a, c, k) * (num * aircon);
+        st.uptk[k] = uptk1 * 0.81;
+      }
+    }
+    h[(H_UPTK + k) * n] = uptk1;
+    q[(SOA_UPTK + k) * n] = st.uptk[k];
+  }
+  st.g = q[SOA_G * n];
+#pragma unroll
+  for (int k = 0; k < NMODE; ++k) {
+    st.a[k] = q[(SOA_A + k) * n];
+    st.opoa[k] = q[(SOA_OPOA + k) * n];
+  }
+  st.g0 = q[SOA_G0 * n];
+  st.dtfull = (double)(int)(a.dt / 1);
+  const double first_rate = soa_first_rate(st) * st.dtfull;
+  if constexpr (FUSE) {
+    // a short loop (first sub-step at least 1/inline_scale of the step)
+    // runs here, and its cell finishes, with the arithmetic of the solver
+    // and post kernels
+    const bool here = first_rate <= 0.05 * a.inline_scale;
+    a.done[c] = here;
+    if (here) {
+      st.tcur = 0.0;
+      st.niter = 0;
+      const bool fast = soa_begin(st);
+      while (soa_pass<MIXED ? 1 : 0>(st, fast)) {
+      }
+      if (st.niter > 1000)
+        atomicOr(a.flags, MAM4B_FLAG_SOA_NITER_LIMIT);
+      q[SOA_G * n] = st.g;
+#pragma unroll
+      for (int k = 0; k < NMODE; ++k)
+        q[(SOA_A + k) * n] = st.a[k];
+      cell_post(a, c);
+      return;
+    }
+  }
+  append_loop(a, c, first_rate);
+}
+
 template <int R, bool MIXED, bool FUSE>
 __global__ void __maxnreg__(R) pre_kernel(const __grid_constant__ StepArgs a) {
-  const ChemArgs none = {nullptr, nullptr, 0};
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c < a.ncell)
-    cell_pre<false, MIXED, FUSE>(a, none, c);
+    pre_cell<MIXED, FUSE>(a, c);
 }
 
 // The pre stage of the step with chemistry (mam4b_step_chem_slab).
@@ -1598,22 +2072,23 @@ __global__ void __launch_bounds__(128) pre_chem_kernel(const __grid_constant__ S
                                                        const __grid_constant__ ChemArgs ch) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c < a.ncell)
-    cell_pre<true>(a, ch, c);
+    cell_pre_chem(a, ch, c);
 }
 
 // (the 128-register cap, 4 blocks of 128 per SM with a few hundred bytes
 // spilled to L1, was 2 % faster than the unconstrained 231-register build)
 template <int R, bool LOOP>
 __global__ void __maxnreg__(R) post_kernel(const __grid_constant__ StepArgs a) {
-  const long long nq = (long long)a.counters[CNT_QUEUED];
-  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long c0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool fused = a.inline_scale > 0.0;
   if constexpr (LOOP) {
     const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 1
-    for (long long i = i0; i < nq; i += stride)
-      cell_post(a, (unsigned)i);
-  } else if (i0 < nq) {
-    cell_post(a, (unsigned)i0);
+    for (long long c = c0; c < a.ncell; c += stride)
+      if (!fused || !a.done[c])
+        cell_post(a, c);
+  } else if (c0 < a.ncell && (!fused || !a.done[c0])) {
+    cell_post(a, c0);
   }
 }
 
@@ -2028,22 +2503,26 @@ MAM4B_HD double &sb_ref(Sub &b, int j) {
   return b.gas[1];
 }
 
+// whether cell c has a clear subarea and with it an SOA loop
+__device__ __forceinline__ bool has_loop(const StepArgs &a, long long c) {
+  return !(__ldg(a.in[MAM4B_IN_CLD] + c) > kCloudy);
+}
+
 __global__ void __launch_bounds__(128, 4) adj_post_kernel(const __grid_constant__ AdjPipeArgs p) {
   const StepArgs &a = p.s;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)a.counters[CNT_QUEUED])
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= a.ncell || !has_loop(a, c))
     return;
   const StepConsts &C = c_k;
   const CoagTables T = {kCoagBm0ij, kCoagBm3i, kCoagBm0};
   const size_t n = (size_t)a.ncell;
-  const long long c = a.task[i];
   const double temp = __ldg(a.in[MAM4B_IN_T] + c);
   const double pmid = __ldg(a.in[MAM4B_IN_P] + c);
   const double zm = __ldg(a.in[MAM4B_IN_ZM] + c);
   const double cld = __ldg(a.in[MAM4B_IN_CLD] + c);
   const double pblh = __ldg(a.pblh + c / a.nlev);
-  const double *h = a.hand + i;
-  double *q = a.soa + i;
+  const double *h = a.hand + c;
+  double *q = a.soa + c;
   adj::SuffixIn in;
   {
     double pop[NPOP];
@@ -2093,7 +2572,7 @@ __global__ void __launch_bounds__(128, 4) adj_post_kernel(const __grid_constant_
   double tb = sb.tb;
   if (p.cfg.do_coag)
     adj::coef_rev(C, T, temp, pmid, dgn_awet, wetdens, sb.ccb, tb, dgn_awetb, wetdensb);
-  // loop-end cotangents for the solver's reverse (slot-indexed)
+  // loop-end cotangents for the solver's reverse
   q[SOA_G * n] = sb.sb.gas[0];
 #pragma unroll
   for (int k = 0; k < NMODE; ++k)
@@ -2125,7 +2604,7 @@ __global__ void __launch_bounds__(128, 4) adj_post_kernel(const __grid_constant_
 // 32 loops of a warp take the same number of passes and run in step:
 // adj_hist_kernel counts the loops per pass count (npass, written by
 // soa_kernel), adj_scan_kernel turns the counts into start offsets (most
-// passes first) and adj_sort_kernel writes the slots in that order over the
+// passes first) and adj_sort_kernel writes the cells in that order over the
 // forward solver's order list, which is free once soa_kernel has run.
 constexpr int kPassBins = 1001;  // pass counts 0..1000
 
@@ -2134,9 +2613,10 @@ __global__ void __launch_bounds__(256) adj_hist_kernel(const __grid_constant__ A
   for (int i = threadIdx.x; i < kPassBins; i += blockDim.x)
     h[i] = 0;
   __syncthreads();
-  const unsigned ntask = p.s.counters[CNT_QUEUED];
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < ntask; t += gridDim.x * blockDim.x)
-    atomicAdd(&h[1000 - p.s.npass[t]], 1u);
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < p.s.ncell; c += stride)
+    if (has_loop(p.s, c))
+      atomicAdd(&h[1000 - p.s.npass[c]], 1u);
   __syncthreads();
   for (int i = threadIdx.x; i < kPassBins; i += blockDim.x)
     if (h[i])
@@ -2169,9 +2649,10 @@ __global__ void __launch_bounds__(1024) adj_scan_kernel(const __grid_constant__ 
 }
 
 __global__ void __launch_bounds__(256) adj_sort_kernel(const __grid_constant__ AdjPipeArgs p) {
-  const unsigned ntask = p.s.counters[CNT_QUEUED];
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < ntask; t += gridDim.x * blockDim.x)
-    p.s.order[atomicAdd(&p.bins[kPassBins + 1000 - p.s.npass[t]], 1u)] = (int)t;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < p.s.ncell; c += stride)
+    if (has_loop(p.s, c))
+      p.s.order[atomicAdd(&p.bins[kPassBins + 1000 - p.s.npass[c]], 1u)] = (int)c;
 }
 
 // Reverse of the SOA loops. Warps take 32 loops at a time from the sorted
@@ -2293,7 +2774,7 @@ __device__ __forceinline__ void adj_long_loops(const AdjPipeArgs &p, unsigned nl
     const double g0b[1] = {b.g0};
     const double g0_sum = adj::sum_modes(0.0, g0b);
     if (valid) {
-      double *lb = p.lbar + a.task[slot];
+      double *lb = p.lbar + slot;
       if (mode == 0) {
         lb[LB_G * n] = b.g;
         lb[LB_G0 * n] = g0_sum;
@@ -2309,7 +2790,7 @@ __device__ __forceinline__ void adj_long_loops(const AdjPipeArgs &p, unsigned nl
 template <int CK, bool FAST>
 __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_constant__ AdjPipeArgs p) {
   const StepArgs &a = p.s;
-  const unsigned ntask = a.counters[CNT_QUEUED];
+  const unsigned ntask = a.counters[CNT_LONG] + a.counters[CNT_SHORT];
   // loops of at least kAdjLongPasses passes: where adj_sort_kernel left off
   // in their last bin
   const unsigned nlong = a.quads ? p.bins[kPassBins + 1000 - kAdjLongPasses] : 0u;
@@ -2418,8 +2899,7 @@ __global__ void __launch_bounds__(kSoaBlock, 2) adj_soa_kernel(const __grid_cons
         }
       }
     }
-    const long long c = a.task[slot];
-    double *lb = p.lbar + c;
+    double *lb = p.lbar + slot;
     lb[LB_G * n] = b.g;
 #pragma unroll
     for (int j = 0; j < NMODE; ++j) {
@@ -2659,7 +3139,18 @@ __host__ __device__ static StepConsts make_consts() {
     for (int s = 0; s < K::nspec(m); ++s)
       C.inv_density[m][s] = 1.0 / K::aero_dens(K::mode_spec(m, s));
     C.log_sig[m] = log(K::sig(m));
+    C.diam_fac[m] = exp(-1.5 * sq(C.log_sig[m]));
+    C.exp45[m] = exp(4.5 * sq(C.log_sig[m]));
+    C.coag[m].e01 = exp(0.125 * C.log_sig[m] * C.log_sig[m]);
+    C.coag[m].e04 = pow(C.coag[m].e01, 4.0);
+    C.coag[m].e36 = exp(4.5 * C.log_sig[m] * C.log_sig[m]);
+    C.coag[m].dlgsqt2 = 1.0 / log(sqrt(2.0));
+    C.coag[m].row = (int)dmax(1.0, dmin(10.0, round(4.0 * (K::sig(m) - 0.75)))) - 1;
+    C.n2v_lo_wide[m] = C.n2v_min[m];
+    C.n2v_hi_wide[m] = C.n2v_max[m];
   }
+  C.n2v_lo_wide[1] /= 1.0e6;
+  C.n2v_hi_wide[0] *= 1.0e6;
   // unit factors: H2SO4 (tracer 2), SOAG (tracer 5), populations 6..30
   auto is_num = [](int i31) { return i31 == 13 || i31 == 18 || i31 == 26 || i31 == 30; };
   const int tr[2] = {2, 5};
@@ -2717,8 +3208,8 @@ __global__ void init_consts_kernel(StepConsts *out) { *out = make_consts(); }
 constexpr size_t kNoAllocCells = MAM4B_NOALLOC_MAX_CELLS;
 constexpr size_t kNoAllocSoa = 0;
 constexpr size_t kNoAllocHand = kNoAllocSoa + (size_t)SOA_FIELDS * kNoAllocCells;
-constexpr size_t kNoAllocTask = kNoAllocHand + (size_t)H_FIELDS * kNoAllocCells;
-constexpr size_t kNoAllocOrder = kNoAllocTask + kNoAllocCells / 2;
+constexpr size_t kNoAllocDone = kNoAllocHand + (size_t)H_FIELDS * kNoAllocCells;
+constexpr size_t kNoAllocOrder = kNoAllocDone + kNoAllocCells / 2;
 constexpr size_t kNoAllocAux = kNoAllocOrder + kNoAllocCells / 2;
 constexpr size_t kNoAllocTail = kNoAllocAux + (size_t)AUX_FIELDS * kNoAllocCells;
 constexpr size_t kNoAllocDoubles = kNoAllocTail + 32;
@@ -3632,7 +4123,7 @@ struct mam4b_ctx {
   // (grown on demand)
   double *d_soa;
   double *d_hand;
-  int *d_task, *d_order;
+  int *d_done, *d_order;
   double *d_aux;
   unsigned *d_counters;  // CNT_WORDS per chunk of the host path
   size_t cap_cells;
@@ -3727,20 +4218,20 @@ cudaError_t ensure_solver_scratch(mam4b_ctx *ctx, size_t ncell) {
     return e;
   cudaFree(ctx->d_soa);
   cudaFree(ctx->d_hand);
-  cudaFree(ctx->d_task);
+  cudaFree(ctx->d_done);
   cudaFree(ctx->d_order);
   cudaFree(ctx->d_aux);
   ctx->d_aux = nullptr;
   ctx->d_soa = nullptr;
   ctx->d_hand = nullptr;
-  ctx->d_task = nullptr;
+  ctx->d_done = nullptr;
   ctx->d_order = nullptr;
   ctx->cap_cells = 0;
   e = cudaMalloc(&ctx->d_soa, (size_t)SOA_FIELDS * ncell * sizeof(double));
   if (e == cudaSuccess)
     e = cudaMalloc(&ctx->d_hand, (size_t)H_FIELDS * ncell * sizeof(double));
   if (e == cudaSuccess)
-    e = cudaMalloc(&ctx->d_task, ncell * sizeof(int));
+    e = cudaMalloc(&ctx->d_done, ncell * sizeof(int));
   if (e == cudaSuccess)
     e = cudaMalloc(&ctx->d_order, ncell * sizeof(int));
   if (e == cudaSuccess)
@@ -3783,7 +4274,7 @@ void set_step_config(const mam4b_ctx *ctx, StepArgs &a, long long ncell, int nle
 void set_step_scratch(const mam4b_ctx *ctx, StepArgs &a, size_t c0, int chunk) {
   a.soa = ctx->d_soa + (size_t)SOA_FIELDS * c0;
   a.hand = ctx->d_hand + (size_t)H_FIELDS * c0;
-  a.task = ctx->d_task + c0;
+  a.done = ctx->d_done + c0;
   a.order = ctx->d_order + c0;
   a.aux = ctx->d_aux + (size_t)AUX_FIELDS * c0;
   a.counters = ctx->d_counters + (size_t)CNT_WORDS * chunk;
@@ -3819,22 +4310,25 @@ unsigned grid_for(long long n, int block, int cpt) {
   return (unsigned)(g > 0 ? g : 1);
 }
 
-// Stage launchers. Stage order: 0 size, 1 mode, 2 pair, 3 pre, 4 soa, 5 post.
+// Stage launchers. Stage order: 0 front (its shape is the tuning's size_*;
+// with chemistry size_kernel), 1 mode, 2 pair, 3 pre, 4 soa, 5 post.
 template <bool LOOP>
-void launch_size_t(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
-  const unsigned g = grid_for(a.ncell, t.size_block, t.cells_per_thread);
+void launch_front_t(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
+  const int cells = t.size_block / 2;
+  const dim3 g(grid_for(a.ncell, cells, t.cells_per_thread), 2);
+  const size_t smem = (size_t)XF_FIELDS * cells * sizeof(double);
   if (t.size_regs == 96)
-    size_kernel<96, LOOP><<<g, t.size_block, 0, s>>>(a);
+    front_kernel<96, LOOP><<<g, t.size_block, smem, s>>>(a);
   else if (t.size_regs == 128)
-    size_kernel<128, LOOP><<<g, t.size_block, 0, s>>>(a);
+    front_kernel<128, LOOP><<<g, t.size_block, smem, s>>>(a);
   else
-    size_kernel<255, LOOP><<<g, t.size_block, 0, s>>>(a);
+    front_kernel<255, LOOP><<<g, t.size_block, smem, s>>>(a);
 }
-void launch_size(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
+void launch_front(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
   if (t.cells_per_thread > 1)
-    launch_size_t<true>(t, a, s);
+    launch_front_t<true>(t, a, s);
   else
-    launch_size_t<false>(t, a, s);
+    launch_front_t<false>(t, a, s);
 }
 void launch_mode(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s, bool mixed) {
   const dim3 g(grid_for(a.ncell, t.mode_block, 1), NMODE);
@@ -3890,7 +4384,6 @@ void launch_soa(const mam4b_tuning &t, int sms, const StepArgs &a, cudaStream_t 
 }
 template <bool LOOP>
 void launch_post_t(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
-  // one thread per queued slot at most; the kernel reads the queue length
   const unsigned g = grid_for(a.ncell, t.post_block, t.cells_per_thread);
   if (t.post_regs == 255)
     post_kernel<255, LOOP><<<g, t.post_block, 0, s>>>(a);
@@ -3942,7 +4435,10 @@ cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_
       cudaEventRecord(ev[k], s);
   };
   mark(0);
-  launch_size(t, a, s);
+  if (ch)
+    size_kernel<<<grid_for(a.ncell, 128, 1), 128, 0, s>>>(a);
+  else
+    launch_front(t, a, s);
   mark(1);
   launch_mode(t, a, s, mixed);
   mark(2);
@@ -4347,7 +4843,7 @@ mam4b_status mam4b_destroy(mam4b_ctx *ctx) {
   cudaFree(ctx->d_pblh);
   cudaFree(ctx->d_soa);
   cudaFree(ctx->d_hand);
-  cudaFree(ctx->d_task);
+  cudaFree(ctx->d_done);
   cudaFree(ctx->d_order);
   cudaFree(ctx->d_aux);
   cudaFree(ctx->d_counters);
@@ -4948,7 +5444,7 @@ mam4b_status mam4b_step_slab_noalloc(const mam4b_config *cfg, const double *in_s
   a.flags = flags ? reinterpret_cast<unsigned *>(flags) : tail + CNT_WORDS;
   a.soa = nd.scratch + kNoAllocSoa;
   a.hand = nd.scratch + kNoAllocHand;
-  a.task = reinterpret_cast<int *>(nd.scratch + kNoAllocTask);
+  a.done = reinterpret_cast<int *>(nd.scratch + kNoAllocDone);
   a.order = reinterpret_cast<int *>(nd.scratch + kNoAllocOrder);
   a.aux = nd.scratch + kNoAllocAux;
   a.ncell = ncell;
@@ -4975,7 +5471,7 @@ mam4b_status mam4b_step_slab_noalloc(const mam4b_config *cfg, const double *in_s
     // the default launch shape (mam4b_default_tuning)
     mam4b_tuning t;
     mam4b_default_tuning(&t);
-    launch_size(t, a, s);
+    launch_front(t, a, s);
     launch_mode(t, a, s, false);
     launch_pair(t, a, s, false);
     launch_pre(t, a, s);
