@@ -1896,44 +1896,48 @@ __device__ __forceinline__ void mode_work(const StepArgs &a, const long long c) 
       uptake_rate_mode(C, M, a.aux[AUX_GDIFF * n + c], a.aux[AUX_FPATH * n + c], dgn_awet);
 }
 
-// FP64: the block's cells are regrouped so that the cells below the
-// crystallisation humidity, whose water uptake needs no Kohler solve, fill
-// warps of their own (cell order kept within each group; blocks of at most
-// 256 threads, the launch shapes allowed).
+// The block's cells c = blockIdx.x * blockDim.x + threadIdx.x regrouped so
+// that the cells below the crystallisation humidity, whose water uptake
+// needs no Kohler solve, fill warps of their own (cell order kept within
+// each group; blocks of whole warps, at most 256 threads). wanted: the cell
+// takes part; returns the thread's cell, -1 for none.
+__device__ __forceinline__ long long group_by_humidity(bool wanted, bool dry) {
+  __shared__ int s_perm[256];
+  __shared__ unsigned s_cnt[8][2];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
+  dry = wanted && dry;
+  const unsigned bd = __ballot_sync(0xffffffffu, dry);
+  const unsigned bo = __ballot_sync(0xffffffffu, wanted && !dry);
+  if (lane == 0) {
+    s_cnt[w][0] = __popc(bd);
+    s_cnt[w][1] = __popc(bo);
+  }
+  __syncthreads();
+  unsigned before_d = 0, before_o = 0, total_d = 0, total = 0;
+  for (int k = 0; k < nw; ++k) {
+    if (k < w) {
+      before_d += s_cnt[k][0];
+      before_o += s_cnt[k][1];
+    }
+    total_d += s_cnt[k][0];
+    total += s_cnt[k][0] + s_cnt[k][1];
+  }
+  if (wanted) {
+    const unsigned below = (1u << lane) - 1u;
+    s_perm[dry ? before_d + __popc(bd & below) : total_d + before_o + __popc(bo & below)] = t;
+  }
+  __syncthreads();
+  return (unsigned)t < total ? (long long)blockIdx.x * blockDim.x + s_perm[t] : -1;
+}
+
 template <bool MIXED>
 __global__ void mode_kernel(const __grid_constant__ StepArgs a) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if constexpr (!MIXED) {
-    __shared__ int s_perm[256];
-    __shared__ unsigned s_cnt[8][2];
-    const long long c0 = (long long)blockIdx.x * blockDim.x;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
     const bool valid = c < a.ncell;
-    const bool dry = valid && a.aux[AUX_RH * (size_t)a.ncell + c] < K::rh_cryst;
-    const unsigned bd = __ballot_sync(0xffffffffu, dry);
-    const unsigned bo = __ballot_sync(0xffffffffu, valid && !dry);
-    if (lane == 0) {
-      s_cnt[w][0] = __popc(bd);
-      s_cnt[w][1] = __popc(bo);
-    }
-    __syncthreads();
-    unsigned before_d = 0, before_o = 0, total_d = 0, total = 0;
-    for (int k = 0; k < nw; ++k) {
-      if (k < w) {
-        before_d += s_cnt[k][0];
-        before_o += s_cnt[k][1];
-      }
-      total_d += s_cnt[k][0];
-      total += s_cnt[k][0] + s_cnt[k][1];
-    }
-    if (valid) {
-      const unsigned below = (1u << lane) - 1u;
-      s_perm[dry ? before_d + __popc(bd & below) : total_d + before_o + __popc(bo & below)] = t;
-    }
-    __syncthreads();
-    if ((unsigned)t >= total)
+    c = group_by_humidity(valid, valid && a.aux[AUX_RH * (size_t)a.ncell + c] < K::rh_cryst);
+    if (c < 0)
       return;
-    c = c0 + s_perm[t];
   }
   if (c >= a.ncell)
     return;
@@ -3039,38 +3043,13 @@ __device__ __forceinline__ void adj_mode_work(const AdjPipeArgs &p, long long c)
 // crystallisation humidity (no Kohler reverse) fill warps of their own.
 // Launched with 128 threads per block.
 __global__ void __launch_bounds__(128) adj_mode_kernel(const __grid_constant__ AdjPipeArgs p) {
-  __shared__ int s_perm[128];
-  __shared__ unsigned s_cnt[4][2];
   const StepArgs &a = p.s;
-  const long long c0 = (long long)blockIdx.x * blockDim.x;
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
-  long long c = c0 + t;
-  const bool valid = c < a.ncell;
-  const bool dry = valid && a.aux[AUX_RH * (size_t)a.ncell + c] < K::rh_cryst;
-  const unsigned bd = __ballot_sync(0xffffffffu, dry);
-  const unsigned bo = __ballot_sync(0xffffffffu, valid && !dry);
-  if (lane == 0) {
-    s_cnt[w][0] = __popc(bd);
-    s_cnt[w][1] = __popc(bo);
-  }
-  __syncthreads();
-  unsigned before_d = 0, before_o = 0, total_d = 0, total = 0;
-  for (int k = 0; k < nw; ++k) {
-    if (k < w) {
-      before_d += s_cnt[k][0];
-      before_o += s_cnt[k][1];
-    }
-    total_d += s_cnt[k][0];
-    total += s_cnt[k][0] + s_cnt[k][1];
-  }
-  if (valid) {
-    const unsigned below = (1u << lane) - 1u;
-    s_perm[dry ? before_d + __popc(bd & below) : total_d + before_o + __popc(bo & below)] = t;
-  }
-  __syncthreads();
-  if ((unsigned)t >= total)
+  const long long c0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = c0 < a.ncell;
+  const long long c =
+      group_by_humidity(valid, valid && a.aux[AUX_RH * (size_t)a.ncell + c0] < K::rh_cryst);
+  if (c < 0)
     return;
-  c = c0 + s_perm[t];
   switch (blockIdx.y) {
   case 0: adj_mode_work<0>(p, c); break;
   case 1: adj_mode_work<1>(p, c); break;
@@ -3355,27 +3334,64 @@ __global__ void __launch_bounds__(128) activate_kernel(const __grid_constant__ A
     a.out[(size_t)k * a.ld + c] = out[k];
 }
 
-// ---- longwave aerosol optics (modal_aero_lw_k) in three launches, as the
-// step is split: mode sizes per cell (calcsize, RH), water uptake and the
-// Chebyshev polynomials per (cell, mode), then the optical depth per
-// (cell, band) summed over the modes in order (one band per block row,
-// so a warp's table reads share a band). Scratch rows (per cell):
-// dry diameter [4], RH, aerosol water [4], Chebyshev polynomials [4][5].
-enum { OS_DGN = 0, OS_RH = 4, OS_QW = 5, OS_CHEB = 9, OS_FIELDS = 29 };
-struct OpticsLwArgs {
+// ---- aerosol optics (modal_aero_lw_k, modal_aero_sw) in three launches, as
+// the step is split: mode sizes per cell (calcsize, RH), water uptake and
+// what the bands take of a mode per (cell, mode), then the products per
+// (cell, band) summed over the modes in order. Scratch rows (per cell): dry
+// diameter [4], RH, ModeOptics [4][4], extinction of geometric optics [4]
+// (shortwave; 0: use the fit), visible-band optical depth of each mode [4]
+// (shortwave).
+//
+// With trop (aero_rad_props) the volcanic extinction is put over the modal
+// optics at and above the column's tropopause level in the same pass: at the
+// level the two are averaged, above it the volcanic values replace the modal
+// ones (volcanic_cmip_sw, aero_rad_props.hpp:38-119;
+// compute_odap_volcanic_at/above_troplayer_lw :121-208), whose computation
+// is then skipped but for the visible band of the column optical depth.
+enum { OS_DGN = 0, OS_RH = 4, OS_MODE = 5, OS_GEO = 21, OS_AOD = 25, OS_FIELDS = 29,
+       OS_LW_FIELDS = 21 };
+struct OpticsArgs {
   const double *in[MAM4B_NIN];
   const double *pdeldry;
-  const double *tables;
-  double *tau;  // [16][ld]
-  double *scr;  // [OS_FIELDS][ncell]
+  const double *tables;          // packed bands (opt::pack_band)
+  double *out;                   // longwave [16][ld]; shortwave [4][14][ld]: tauxar, wa, ga, fa
+  double *scr;                   // [OS_FIELDS or OS_LW_FIELDS][ncell]
+  double *aodvis;                // shortwave: [ncol] or null
+  const int *trop;               // [ncol] or null: tropopause levels
+  const int *modal;              // with trop: the cells at or below the tropopause level
+  const unsigned *nmodal;        // their number
+  const double *zi;              // [col * (nlev + 1) + k]: interface height (with trop)
+  const double *ext, *ssa, *af;  // [band][ld] (with trop; ssa, af shortwave)
   size_t ld;
   long long ncell;
+  int ncol, nlev;
   double dt;
 };
 
-__global__ void __launch_bounds__(128) optics_size_kernel(const __grid_constant__ OpticsLwArgs a) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= a.ncell)
+// Level of a cell relative to its column's tropopause: -1 above (the
+// volcanic values replace the modal ones), 0 at it, 1 below; 1 without trop.
+__device__ __forceinline__ int rel_to_tropopause(const OpticsArgs &a, long long c) {
+  if (!a.trop)
+    return 1;
+  const unsigned col = (unsigned)c / (unsigned)a.nlev;
+  const int k = (int)((unsigned)c - col * (unsigned)a.nlev), lev = __ldg(a.trop + col);
+  return k < lev ? -1 : k == lev ? 0 : 1;
+}
+__device__ __forceinline__ double layer_thickness(const OpticsArgs &a, long long c) {
+  const size_t i = (size_t)c + (unsigned)c / (unsigned)a.nlev;
+  return __ldg(a.zi + i) - __ldg(a.zi + i + 1);
+}
+// The cell of work item i of the modal stages, -1 for none: every cell, or
+// with trop the listed ones when nothing needs the others.
+__device__ __forceinline__ long long modal_cell(const OpticsArgs &a, long long i) {
+  if (!a.trop || a.aodvis)
+    return i < a.ncell ? i : -1;
+  return i < (long long)*a.nmodal ? a.modal[i] : -1;
+}
+
+__global__ void __launch_bounds__(128) optics_size_kernel(const __grid_constant__ OpticsArgs a) {
+  const long long c = modal_cell(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (c < 0)
     return;
   double ai[NPOP], ac[NPOP], dgn_a[NMODE], pt_i[NPOP], pt_c[NPOP];
 #pragma unroll
@@ -3392,8 +3408,8 @@ __global__ void __launch_bounds__(128) optics_size_kernel(const __grid_constant_
                                          __ldg(a.in[MAM4B_IN_P] + c), __ldg(a.in[MAM4B_IN_CLD] + c));
 }
 
-template <int M>
-__device__ __forceinline__ void optics_mode_work(const OpticsLwArgs &a, long long c) {
+template <int M, bool SW>
+__device__ __forceinline__ void optics_mode_work(const OpticsArgs &a, long long c) {
   const size_t n = (size_t)a.ncell;
   double sp[7];
 #pragma unroll
@@ -3402,189 +3418,243 @@ __device__ __forceinline__ void optics_mode_work(const OpticsLwArgs &a, long lon
   double dgn_w, qw, wd;
   water_uptake_mode<M>(c_k, sp, a.scr[OS_RH * n + c], a.scr[(OS_DGN + M) * n + c], dgn_w, qw,
                        wd);
-  double cheb[opt::kNcoef];
-  opt::mode_cheb(M, dgn_w, cheb);
-  a.scr[(OS_QW + M) * n + c] = qw;
-#pragma unroll
-  for (int k = 0; k < opt::kNcoef; ++k)
-    a.scr[(OS_CHEB + opt::kNcoef * M + k) * n + c] = cheb[k];
+  // modal_size_parameters: the log of the surface-mode radius by method 2
+  // (longwave) or of the radius itself (shortwave, method 1)
+  const double alnsg = log(K::sig(M));
+  double lrad;
+  if constexpr (SW) {
+    const double rad = 0.5 * dgn_w * exp(2.0 * alnsg * alnsg);
+    lrad = log(rad);
+    a.scr[(OS_GEO + M) * n + c] = lrad <= log(25.e-6) ? 0.0 : 1.5 / (rad * 1.0e3);
+  } else {
+    lrad = log(0.5 * dgn_w) + 2.0 * alnsg * alnsg;
+  }
+  const opt::ModeOptics o = opt::mode_optics<M>(sp, lrad, qw, SW);
+  double *s = a.scr + (OS_MODE + 4 * M) * n + c;
+  s[0] = o.xrad;
+  s[n] = o.water;
+  s[2 * n] = o.inv_wet;
+  s[3 * n] = o.wet1000;
 }
 
-__global__ void __launch_bounds__(128) optics_mode_kernel(const __grid_constant__ OpticsLwArgs a) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= a.ncell)
+// Cells regrouped by humidity, as in mode_kernel.
+template <bool SW>
+__global__ void __launch_bounds__(256) optics_mode_kernel(const __grid_constant__ OpticsArgs a) {
+  const long long c0 = modal_cell(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+  const long long i = group_by_humidity(
+      c0 >= 0, c0 >= 0 && a.scr[OS_RH * (size_t)a.ncell + c0] < K::rh_cryst);
+  if (i < 0)
     return;
+  const long long c = modal_cell(a, i);
   switch (blockIdx.y) {
-  case 0: optics_mode_work<0>(a, c); break;
-  case 1: optics_mode_work<1>(a, c); break;
-  case 2: optics_mode_work<2>(a, c); break;
-  default: optics_mode_work<3>(a, c); break;
+  case 0: optics_mode_work<0, SW>(a, c); break;
+  case 1: optics_mode_work<1, SW>(a, c); break;
+  case 2: optics_mode_work<2, SW>(a, c); break;
+  default: optics_mode_work<3, SW>(a, c); break;
   }
 }
+
+// What a band reads of mode M of a cell. The next mode's values are loaded
+// before the current one's fits, whose arithmetic hides the latency.
+struct ModeIn {
+  opt::ModeOptics o;
+  double geo, sp[7];
+};
+template <int M, bool SW>
+__device__ __forceinline__ ModeIn load_mode(const OpticsArgs &a, long long c) {
+  const size_t n = (size_t)a.ncell;
+  const double *q = a.scr + (OS_MODE + 4 * M) * n + c;
+  ModeIn x;
+  x.o = {q[0], q[n], q[2 * n], q[3 * n]};
+  x.geo = 0.0;
+  if constexpr (SW)
+    x.geo = a.scr[(OS_GEO + M) * n + c];
+#pragma unroll
+  for (int s = 0; s < 7; ++s)
+    x.sp[s] = s < K::nspec(M) ? __ldg(a.in[MAM4B_IN_AER_I + K::spec0(M) + (s < K::nspec(M) ? s : 0)] + c) : 0.0;
+  return x;
+}
+// The four modes of a cell in the staged band s: the NQ fits of each mode
+// go to put(mode, fit, its ModeIn).
+template <int NQ, int NODE, class Put>
+__device__ __forceinline__ void band_modes(const OpticsArgs &a, const double *s, long long c,
+                                           const Put &put) {
+  constexpr bool SW = NQ == 3;
+  double fit[NQ];
+  const ModeIn m0 = load_mode<0, SW>(a, c);
+  const ModeIn m1 = load_mode<1, SW>(a, c);
+  opt::mode_fit<0, NQ, NODE>(s, m0.sp, m0.o, fit);
+  put(std::integral_constant<int, 0>(), fit, m0);
+  const ModeIn m2 = load_mode<2, SW>(a, c);
+  opt::mode_fit<1, NQ, NODE>(s, m1.sp, m1.o, fit);
+  put(std::integral_constant<int, 1>(), fit, m1);
+  const ModeIn m3 = load_mode<3, SW>(a, c);
+  opt::mode_fit<2, NQ, NODE>(s, m2.sp, m2.o, fit);
+  put(std::integral_constant<int, 2>(), fit, m2);
+  opt::mode_fit<3, NQ, NODE>(s, m3.sp, m3.o, fit);
+  put(std::integral_constant<int, 3>(), fit, m3);
+}
+// The block's band into shared memory.
+template <int DOUBLES>
+__device__ __forceinline__ void stage_band(const OpticsArgs &a, int b, double *s) {
+  const double2 *g = reinterpret_cast<const double2 *>(a.tables + (size_t)b * DOUBLES);
+  for (int i = threadIdx.x; i < DOUBLES / 2; i += blockDim.x)
+    reinterpret_cast<double2 *>(s)[i] = __ldg(g + i);
+  __syncthreads();
+}
+static_assert(opt::kLwBandDoubles % 2 == 0 && opt::kSwBandDoubles % 2 == 0 &&
+                  opt::kBandNodes % 2 == 0 && opt::kLwNode % 2 == 0 && opt::kSwNode % 2 == 0,
+              "16-byte loads of the staged tables");
 
 // The band is the grid's fastest index: the blocks of one group of cells
 // run back to back for every band, so each cell's inputs come from DRAM
-// once and from L2 for the other bands.
-// The block's band tables (12 KB) are staged in shared memory first and
-// serve every group of cells the block steps (at most 1,024 blocks per
-// band): 11.0 -> 10.2 ms per call on 65,536 x 72 cells. (With one group of
-// cells per block the staging cost more than it saved: 12.2 ms.)
-__global__ void __launch_bounds__(128) optics_band_kernel(const __grid_constant__ OpticsLwArgs a) {
-  const int b = blockIdx.x;
-  const size_t n = (size_t)a.ncell;
-  __shared__ double s_tab[opt::kLwBandDoubles];
-  opt::stage_lw_band(a.tables, b, s_tab);
-  __syncthreads();
-  for (long long cb = blockIdx.y; cb * blockDim.x < a.ncell; cb += gridDim.y) {
-  const long long c = cb * blockDim.x + threadIdx.x;
-  if (c >= a.ncell)
-    break;
-  double ai[NPOP];
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p)
-    ai[p] = (K::numslot(0) == p || K::numslot(1) == p || K::numslot(2) == p || K::numslot(3) == p)
-                ? 0.0
-                : __ldg(a.in[MAM4B_IN_AER_I + p] + c);
-  const double mass = __ldg(a.pdeldry + c) * (1.0 / 9.80616);
-  double tau = 0.0;
-#pragma unroll
-  for (int m = 0; m < NMODE; ++m) {
-    double cheb[opt::kNcoef], specvol[7];
-#pragma unroll
-    for (int k = 0; k < opt::kNcoef; ++k)
-      cheb[k] = a.scr[(OS_CHEB + opt::kNcoef * m + k) * n + c];
-    opt::mode_specvol(m, ai, specvol);
-    tau += opt::mode_band_tau<opt::LwBand>(s_tab, m, b, specvol, a.scr[(OS_QW + m) * n + c],
-                                           cheb, mass);
-  }
-  a.tau[(size_t)b * a.ld + c] = tau;
-  }
-}
-
-// ---- shortwave aerosol optics (modal_aero_sw): optics_size_kernel, then
-// per (cell, mode) water uptake and the method-1 size parameters, per
-// (cell, band) the four mode-summed products, and per column the visible
-// optical depth. Scratch rows beyond the longwave ones: Chebyshev
-// polynomials [4][5], surface radius [4], its log [4], visible-band
-// optical depth of each mode [4].
-enum { SS_CHEB = 9, SS_RAD = 29, SS_LOGRAD = 33, SS_AOD = 37, SS_FIELDS = 41 };
-struct OpticsSwArgs {
-  OpticsLwArgs base;  // inputs, tables, scratch, ld, ncell, dt (base.tau unused)
-  double *out;        // [4][14][ld]: tauxar, wa, ga, fa
-  double *aodvis;     // [ncol] or null
-  int ncol, nlev;
-};
-
-template <int M>
-__device__ __forceinline__ void optics_sw_mode_work(const OpticsSwArgs &w, long long c) {
-  const OpticsLwArgs &a = w.base;
-  const size_t n = (size_t)a.ncell;
-  double sp[7];
-#pragma unroll
-  for (int s = 0; s < 7; ++s)
-    sp[s] = (s < K::nspec(M)) ? __ldg(a.in[MAM4B_IN_AER_I + K::spec0(M) + (s < K::nspec(M) ? s : 0)] + c) : 0.0;
-  double dgn_w, qw, wd;
-  water_uptake_mode<M>(c_k, sp, a.scr[OS_RH * n + c], a.scr[(OS_DGN + M) * n + c], dgn_w, qw,
-                       wd);
-  double cheb[opt::kNcoef], rad, lrad;
-  opt::mode_cheb_sw(M, dgn_w, rad, lrad, cheb);
-  a.scr[(OS_QW + M) * n + c] = qw;
-#pragma unroll
-  for (int k = 0; k < opt::kNcoef; ++k)
-    a.scr[(SS_CHEB + opt::kNcoef * M + k) * n + c] = cheb[k];
-  a.scr[(SS_RAD + M) * n + c] = rad;
-  a.scr[(SS_LOGRAD + M) * n + c] = lrad;
-}
-
-__global__ void __launch_bounds__(128) optics_sw_mode_kernel(const __grid_constant__ OpticsSwArgs w) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= w.base.ncell)
+// once and from L2 for the other bands. Each block stages its band's tables
+// once and steps several groups of cells with them: the cells with modal
+// optics (listed ones with trop, whose warps are then full), then the cells
+// above the tropopause.
+constexpr int kBandBlock = 256;
+constexpr unsigned kBandCellBlocks = 512;  // blocks per band at most
+template <class Modal, class Above>
+__device__ __forceinline__ void band_cells(const OpticsArgs &a, bool all, const Modal &modal,
+                                           const Above &above) {
+  const long long i0 = (long long)blockIdx.y * blockDim.x + threadIdx.x;
+  const long long stride = (long long)gridDim.y * blockDim.x;
+  if (!a.trop || all) {
+    for (long long c = i0; c < a.ncell; c += stride)
+      modal(c);
     return;
-  switch (blockIdx.y) {
-  case 0: optics_sw_mode_work<0>(w, c); break;
-  case 1: optics_sw_mode_work<1>(w, c); break;
-  case 2: optics_sw_mode_work<2>(w, c); break;
-  default: optics_sw_mode_work<3>(w, c); break;
   }
+  const long long nm = (long long)*a.nmodal;
+  for (long long i = i0; i < nm; i += stride)
+    modal((long long)__ldg(a.modal + i));
+  for (long long c = i0; c < a.ncell; c += stride)
+    if (rel_to_tropopause(a, c) < 0)
+      above(c);
 }
 
-// band-fastest grid, as optics_band_kernel. The block's band tables are
-// staged in shared memory first (35 KB: three coefficient tables per mode):
-// the table reads of every (cell, band) thread are gathers that would
-// otherwise wait on L1/L2 (with at most 1,024 blocks of cells per band:
-// 17.1 -> 13.7 ms per call on 65,536 x 72 cells).
-__global__ void __launch_bounds__(128) optics_sw_band_kernel(const __grid_constant__ OpticsSwArgs w) {
-  const OpticsLwArgs &a = w.base;
+__global__ void __launch_bounds__(kBandBlock, 3) optics_band_kernel(const __grid_constant__ OpticsArgs a) {
+  __shared__ __align__(16) double s[opt::kLwBandDoubles];
+  const int b = blockIdx.x;
+  stage_band<opt::kLwBandDoubles>(a, b, s);
+  double *out = a.out + (size_t)b * a.ld;
+  auto volcanic = [&](long long c) {
+    return layer_thickness(a, c) * __ldg(a.ext + (size_t)b * a.ld + c);
+  };
+  band_cells(
+      a, false,
+      [&](long long c) {
+        const double mass = __ldg(a.pdeldry + c) * (1.0 / 9.80616);
+        double tau = 0.0;
+        band_modes<1, opt::kLwNode>(a, s, c, [&](auto, const double (&fit)[1], const ModeIn &x) {
+          tau = fma(dmax(0.0, fit[0] * x.o.wet1000), mass, tau);
+        });
+        if (rel_to_tropopause(a, c) == 0)
+          tau = 0.5 * (tau + volcanic(c));
+        out[c] = tau;
+      },
+      [&](long long c) { out[c] = volcanic(c); });
+}
+
+// Bound by the instructions of the mixing, the bracket search and the fits
+// (about 230 per mode and band) and by shared-memory reads of the brackets'
+// corners (32 of 16 bytes per lane, mode and band: 120 cycles per warp at
+// least). With the tables as the host gives them (one 8-byte read per
+// coefficient and corner, linear search, species volumes and two divisions
+// again in every band) 920 instructions per mode and band: the shortwave
+// entry of 16,384 x 72 cells took 3.84 ms (this kernel 2.9) and takes 1.67,
+// the longwave one 2.78 and 0.95.
+__global__ void __launch_bounds__(kBandBlock, 3) optics_sw_band_kernel(const __grid_constant__ OpticsArgs a) {
+  __shared__ __align__(16) double s[opt::kSwBandDoubles];
   const int b = blockIdx.x;
   const size_t n = (size_t)a.ncell;
-  __shared__ double s_tab[opt::kSwBandDoubles];
-  opt::stage_sw_band(a.tables, b, s_tab);
-  __syncthreads();
-  for (long long cb = blockIdx.y; cb * blockDim.x < a.ncell; cb += gridDim.y) {
-  const long long c = cb * blockDim.x + threadIdx.x;
-  if (c >= a.ncell)
-    break;
-  double ai[NPOP];
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p)
-    ai[p] = (K::numslot(0) == p || K::numslot(1) == p || K::numslot(2) == p || K::numslot(3) == p)
-                ? 0.0
-                : __ldg(a.in[MAM4B_IN_AER_I + p] + c);
-  const double mass = __ldg(a.pdeldry + c) * (1.0 / 9.80616);
-  double sum[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-  for (int m = 0; m < NMODE; ++m) {
-    double cheb[opt::kNcoef], specvol[7], o[4];
-#pragma unroll
-    for (int k = 0; k < opt::kNcoef; ++k)
-      cheb[k] = a.scr[(SS_CHEB + opt::kNcoef * m + k) * n + c];
-    opt::mode_specvol(m, ai, specvol);
-    opt::mode_band_sw<opt::SwBand>(s_tab, m, b, specvol, a.scr[(OS_QW + m) * n + c], cheb,
-                      a.scr[(SS_RAD + m) * n + c], a.scr[(SS_LOGRAD + m) * n + c], mass, o);
+  stage_band<opt::kSwBandDoubles>(a, b, s);
+  const bool diag = a.aodvis && b == opt::kSwDiagBand;
+  auto store = [&](long long c, const double (&v)[4]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      sum[q] += o[q];
-    if (b == opt::kSwDiagBand)
-      a.scr[(SS_AOD + m) * n + c] = o[0];
-  }
+      a.out[((size_t)q * opt::kSwBands + b) * a.ld + c] = v[q];
+  };
+  auto volcanic = [&](long long c, double (&v)[4]) {
+    const double ext = layer_thickness(a, c) * __ldg(a.ext + (size_t)b * a.ld + c);
+    const double asym = __ldg(a.af + (size_t)b * a.ld + c);
+    v[0] = ext;
+    v[1] = ext * __ldg(a.ssa + (size_t)b * a.ld + c);
+    v[2] = v[1] * asym;
+    v[3] = v[2] * asym;
+  };
+  band_cells(
+      a, diag,
+      [&](long long c) {
+        const double mass = __ldg(a.pdeldry + c) * (1.0 / 9.80616);
+        double sum[4] = {0.0, 0.0, 0.0, 0.0};
+        band_modes<3, opt::kSwNode>(a, s, c, [&](auto mode, const double (&fit)[3], const ModeIn &x) {
+          constexpr int M = decltype(mode)::value;
+          const double pext = (x.geo == 0.0 ? exp(fit[0]) : x.geo) * x.o.wet1000;
+          const double pabs = bound(0.0, pext, fit[1] * x.o.wet1000);
+          const double palb = 1.0 - pabs / dmax(pext, 1.e-40);
+          double o = pext * mass;
+          if (diag)
+            a.scr[(OS_AOD + M) * n + c] = o;
+          sum[0] += o;
+          o *= palb;
+          sum[1] += o;
+          o *= fit[2];
+          sum[2] += o;
+          sum[3] = fma(o, fit[2], sum[3]);
+        });
+        const int rel = rel_to_tropopause(a, c);
+        if (rel <= 0) {
+          double v[4];
+          volcanic(c, v);
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-    w.out[((size_t)q * opt::kSwBands + b) * a.ld + c] = sum[q];
-  }
+          for (int q = 0; q < 4; ++q)
+            sum[q] = rel == 0 ? 0.5 * (sum[q] + v[q]) : v[q];
+        }
+        store(c, sum);
+      },
+      [&](long long c) {
+        double v[4];
+        volcanic(c, v);
+        store(c, v);
+      });
 }
 
 // visible optical depth of each column: its levels' mode optical depths
-// summed level by level, mode by mode (the reduction of modal_aero_sw)
-__global__ void __launch_bounds__(128) optics_sw_aod_kernel(const __grid_constant__ OpticsSwArgs w) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= w.ncol)
-    return;
-  const size_t n = (size_t)w.base.ncell;
+// summed, one warp per column
+__global__ void __launch_bounds__(128) optics_sw_aod_kernel(const __grid_constant__ OpticsArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (col >= a.ncol)
+    return;  // the whole warp
+  const size_t n = (size_t)a.ncell;
   double s = 0.0;
-  for (int k = 0; k < w.nlev; ++k) {
-    const size_t c = (size_t)col * w.nlev + k;
+  for (int k = lane; k < a.nlev; k += 32) {
+    const size_t c = (size_t)col * a.nlev + k;
 #pragma unroll
     for (int m = 0; m < NMODE; ++m)
-      s += w.base.scr[(SS_AOD + m) * n + c];
+      s += a.scr[(OS_AOD + m) * n + c];
   }
-  w.aodvis[col] = s;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+    s += __shfl_xor_sync(0xffffffffu, s, d);
+  if (lane == 0)
+    a.aodvis[col] = s;
 }
 
-// ---- aero_rad_props: tropopause per column, then the volcanic (CMIP6)
-// extinction over the modal optics at and above it
+// ---- aero_rad_props: the tropopause of each column
 struct RadArgs {
   const double *temp, *pmid;     // step input fields (cell = col * nlev + k)
-  const double *pint, *zi;       // [col * (nlev + 1) + k]: interface pressure, height
-  const double *ext, *ssa, *af;  // [band][ld]: extinction [1/m], albedo, asymmetry
-  double *out;                   // shortwave [4][14][ld], longwave [16][ld]
+  const double *pint;            // [col * (nlev + 1) + k]: interface pressure
   int *trop;                     // [ncol]
-  size_t ld;
+  int *modal;                    // [ncol * nlev]: the cells at or below the level
+  unsigned *nmodal;              // their number (zero at the launch)
   int ncol, nlev;
 };
 
 // one warp per column: the lanes compute every layer's lapse-rate
 // quantities (the pow-heavy part) into shared memory, then one lane runs
-// the scan on them
+// the scan on them, and the column's cells at or below the level go to the
+// list of cells with modal optics
 __global__ void __launch_bounds__(128) tropopause_kernel(const __grid_constant__ RadArgs r) {
   extern __shared__ double tsm[];  // [warps][4][nlev]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nlev = r.nlev;
@@ -3595,75 +3665,49 @@ __global__ void __launch_bounds__(128) tropopause_kernel(const __grid_constant__
   const size_t c0 = (size_t)col * nlev, i0 = (size_t)col * (nlev + 1);
   auto T = [&](int k) { return __ldg(r.temp + c0 + k); };
   auto P = [&](int k) { return __ldg(r.pmid + c0 + k); };
-  for (int k = 1 + lane; k < nlev; k += 32) {
-    const rad::LapsePair q = rad::lapse_pair(T, P, k);
-    s[k] = q.pmk;
-    s[nlev + k] = q.pm;
-    s[2 * nlev + k] = q.dtdz;
-    s[3 * nlev + k] = q.tm;
-  }
+  // p^kappa of every level first (in the last row, whose layer values
+  // replace it): a layer needs those of both its levels
+  double *pk = s + 3 * nlev;
+  for (int k = lane; k < nlev; k += 32)
+    pk[k] = rad::p_kappa(P(k));
   __syncwarp();
+  for (int k0 = 1; k0 < nlev; k0 += 32) {
+    const int k = k0 + lane;
+    rad::LapsePair q;
+    if (k < nlev)
+      q = rad::lapse_pair(T, P, k, pk[k - 1], pk[k]);
+    __syncwarp();  // the next 32 layers still read pk[k0 + 31] and above
+    if (k < nlev) {
+      s[k] = q.pmk;
+      s[nlev + k] = q.pm;
+      s[2 * nlev + k] = q.dtdz;
+      // layer k + 31's pk[k - 1 + 32] is read by the next round: write one
+      // below, where this round was the last reader
+      pk[k - 1] = q.tm;
+    }
+    __syncwarp();
+  }
+  int lev = 0;
   if (lane == 0) {
     auto pair = [&](int k) {
       rad::LapsePair q;
       q.pmk = s[k];
       q.pm = s[nlev + k];
       q.dtdz = s[2 * nlev + k];
-      q.tm = s[3 * nlev + k];
+      q.tm = pk[k - 1];
       return q;
     };
     auto PI = [&](int k) { return __ldg(r.pint + i0 + k); };
-    r.trop[col] = rad::tropopause_level_at(rad::twmo_from_pairs(pair, nlev), PI, nlev);
+    lev = rad::tropopause_level_at(rad::twmo_from_pairs(pair, nlev), PI, nlev);
+    r.trop[col] = lev;
   }
-}
-
-// volcanic_cmip_sw (aero_rad_props.hpp:38-119): at the tropopause level the
-// four layer products are averaged with the volcanic ones, above it they
-// are replaced (the file's values hold all stratospheric aerosol there)
-__global__ void __launch_bounds__(128) volcanic_sw_kernel(const __grid_constant__ RadArgs r) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= (long long)r.ncol * r.nlev)
-    return;
-  const int col = (int)(c / r.nlev), k = (int)(c % r.nlev);
-  const int lev = __ldg(r.trop + col);
-  if (k > lev)
-    return;
-  const size_t i0 = (size_t)col * (r.nlev + 1);
-  const double thk = __ldg(r.zi + i0 + k) - __ldg(r.zi + i0 + k + 1);
-  const size_t ld = r.ld, nb = opt::kSwBands;
-  for (int b = 0; b < opt::kSwBands; ++b) {
-    const double ext = thk * __ldg(r.ext + b * ld + c);
-    const double asym = __ldg(r.af + b * ld + c);
-    const double ext_ssa = ext * __ldg(r.ssa + b * ld + c);
-    const double ext_ssa_asym = ext_ssa * asym;
-    const double v[4] = {ext, ext_ssa, ext_ssa_asym, ext_ssa_asym * asym};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      double *o = r.out + (q * nb + b) * ld + c;
-      *o = k == lev ? 0.5 * (*o + v[q]) : v[q];
-    }
-  }
-}
-
-// compute_odap_volcanic_at_troplayer_lw / _above_troplayer_lw
-// (aero_rad_props.hpp:121-208): the absorption optical depth, averaged at
-// the tropopause level, replaced above it
-__global__ void __launch_bounds__(128) volcanic_lw_kernel(const __grid_constant__ RadArgs r) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= (long long)r.ncol * r.nlev)
-    return;
-  const int col = (int)(c / r.nlev), k = (int)(c % r.nlev);
-  const int lev = __ldg(r.trop + col);
-  if (k > lev)
-    return;
-  const size_t i0 = (size_t)col * (r.nlev + 1);
-  const double thk = __ldg(r.zi + i0 + k) - __ldg(r.zi + i0 + k + 1);
-  const size_t ld = r.ld;
-  for (int b = 0; b < opt::kLwBands; ++b) {
-    double *o = r.out + b * ld + c;
-    const double v = thk * __ldg(r.ext + b * ld + c);
-    *o = k == lev ? 0.5 * (*o + v) : v;
-  }
+  lev = __shfl_sync(0xffffffffu, lev, 0);
+  unsigned base = 0;
+  if (lane == 0)
+    base = atomicAdd(r.nmodal, (unsigned)(nlev - lev));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  for (int k = lev + lane; k < nlev; k += 32)
+    r.modal[base + (k - lev)] = (int)(c0 + k);
 }
 
 // ---- droplet activation and vertical mixing (ndrop dropmixnuc), one
@@ -4146,12 +4190,14 @@ struct mam4b_ctx {
   int adj_ck;           // SOA checkpoint interval of the pipelined adjoint (0 = 1)
   int ck2_slots;        // SOA states per solver thread d_ck2 holds
   int *d_npass;         // [cap_adj]: passes of each SOA loop
-  double *d_optics_lw;  // longwave optics tables (opt::kTableDoubles), set by the host
-  double *d_optics_sw;  // shortwave optics tables (opt::kSwTableDoubles), set by the host
-  double *d_optics_scr; // optics per-cell sizes (SS_FIELDS per cell), grown
+  double *d_optics_lw;  // longwave optics tables (16 packed bands), set by the host
+  double *d_optics_sw;  // shortwave optics tables (14 packed bands), set by the host
+  double *d_optics_scr; // optics per-cell values (OS_FIELDS per cell), grown
   size_t cap_optics_scr;
   int *d_trop;          // [cap_trop]: tropopause level per column (aero_rad_props)
   size_t cap_trop;
+  int *d_modal;         // [cap_modal + 1]: number and list of cells with modal optics
+  size_t cap_modal;
   double *d_dmx;        // dropmixnuc activation results (DA_FIELDS per cell), grown
   double *d_coag_cc;    // coagulation process: 12 coefficients per cell, grown
   size_t cap_coag_cc;
@@ -4857,6 +4903,7 @@ mam4b_status mam4b_destroy(mam4b_ctx *ctx) {
   cudaFree(ctx->d_optics_scr);
   cudaFree(ctx->d_optics_sw);
   cudaFree(ctx->d_trop);
+  cudaFree(ctx->d_modal);
   cudaFree(ctx->d_dmx);
   cudaFree(ctx->d_coag_cc);
   if (ctx->host_streams) {
@@ -5691,6 +5738,27 @@ mam4b_status mam4b_step_tracers(mam4b_ctx *ctx, const double *q, const double *q
   return mam4b_step(ctx, &iv, &ov, ncol, nlev, dt, precision, stream);
 }
 
+// Copies a set of packed bands into the context (*dev).
+static mam4b_status set_optics_tables(mam4b_ctx *ctx, const char *what, double **dev,
+                                      const double *specref, const double *water,
+                                      const double *refr, const double *refi,
+                                      const double *const *tabs, int ntab, int node, int bands) {
+  const size_t per = (size_t)opt::band_doubles(node), bytes = per * bands * sizeof(double);
+  double *h = (double *)malloc(bytes);
+  if (!h)
+    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
+  for (int b = 0; b < bands; ++b)
+    opt::pack_band(specref, MAM4B_OPTICS_NTYPES, water, refr, refi, tabs, ntab, node, bands, b,
+                   h + per * b);
+  cudaError_t e = cudaSuccess;
+  if (!*dev)
+    e = cudaMalloc(dev, bytes);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(*dev, h, bytes, cudaMemcpyHostToDevice);
+  free(h);
+  return e == cudaSuccess ? MAM4B_OK : set_err(ctx, MAM4B_ERR_CUDA, what, e);
+}
+
 // longwave optics tables: the reference's per-type species refractive
 // indices mapped to modes by species type (set_device_specrefindex,
 // modal_aero_opt.hpp:142-190), water, grids and absorption tables
@@ -5699,37 +5767,9 @@ mam4b_status mam4b_optics_lw_set_tables(mam4b_ctx *ctx, const mam4b_optics_lw_ta
   if (!ctx || !t || !t->specrefindex || !t->water_refindex || !t->refrtab || !t->refitab ||
       !t->absp)
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  double *h = (double *)malloc(sizeof(double) * opt::kTableDoubles);
-  if (!h)
-    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, "mam4b_optics_lw_set_tables: host memory",
-                   cudaSuccess);
-  memset(h, 0, sizeof(double) * opt::kTableDoubles);
-  for (int m = 0; m < NMODE; ++m)
-    for (int s = 0; s < K::nspec(m); ++s)
-      for (int b = 0; b < opt::kLwBands; ++b) {
-        const int type = act::spectype(m, s) - 1;
-        const size_t src = 2 * ((size_t)b * MAM4B_OPTICS_NTYPES + type);
-        h[opt::kSpecRe + (m * 7 + s) * opt::kLwBands + b] = t->specrefindex[src];
-        h[opt::kSpecIm + (m * 7 + s) * opt::kLwBands + b] = t->specrefindex[src + 1];
-      }
-  for (int b = 0; b < opt::kLwBands; ++b) {
-    h[opt::kWaterRe + b] = t->water_refindex[2 * b];
-    h[opt::kWaterIm + b] = t->water_refindex[2 * b + 1];
-  }
-  memcpy(h + opt::kRefr, t->refrtab, sizeof(double) * 4 * opt::kLwBands * opt::kPrefr);
-  memcpy(h + opt::kRefi, t->refitab, sizeof(double) * 4 * opt::kLwBands * opt::kPrefi);
-  memcpy(h + opt::kAbsp, t->absp,
-         sizeof(double) * 4 * opt::kLwBands * opt::kNcoef * opt::kPrefr * opt::kPrefi);
-  cudaError_t e = cudaSuccess;
-  if (!ctx->d_optics_lw)
-    e = cudaMalloc(&ctx->d_optics_lw, sizeof(double) * opt::kTableDoubles);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(ctx->d_optics_lw, h, sizeof(double) * opt::kTableDoubles,
-                   cudaMemcpyHostToDevice);
-  free(h);
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-  return MAM4B_OK;
+  const double *tabs[1] = {t->absp};
+  return set_optics_tables(ctx, what, &ctx->d_optics_lw, t->specrefindex, t->water_refindex,
+                           t->refrtab, t->refitab, tabs, 1, opt::kLwNode, opt::kLwBands);
 }
 
 // shortwave optics tables (layouts of mam4b_optics_sw_tables)
@@ -5738,38 +5778,75 @@ mam4b_status mam4b_optics_sw_set_tables(mam4b_ctx *ctx, const mam4b_optics_sw_ta
   if (!ctx || !t || !t->specrefindex || !t->water_refindex || !t->refrtab || !t->refitab ||
       !t->extp || !t->absp || !t->asmp)
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  double *h = (double *)malloc(sizeof(double) * opt::kSwTableDoubles);
-  if (!h)
-    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, "mam4b_optics_sw_set_tables: host memory",
-                   cudaSuccess);
-  memset(h, 0, sizeof(double) * opt::kSwTableDoubles);
-  for (int m = 0; m < NMODE; ++m)
-    for (int s = 0; s < K::nspec(m); ++s)
-      for (int b = 0; b < opt::kSwBands; ++b) {
-        const int type = act::spectype(m, s) - 1;
-        const size_t src = 2 * ((size_t)b * MAM4B_OPTICS_NTYPES + type);
-        h[opt::kSwSpecRe + (m * 7 + s) * opt::kSwBands + b] = t->specrefindex[src];
-        h[opt::kSwSpecIm + (m * 7 + s) * opt::kSwBands + b] = t->specrefindex[src + 1];
-      }
-  for (int b = 0; b < opt::kSwBands; ++b) {
-    h[opt::kSwWaterRe + b] = t->water_refindex[2 * b];
-    h[opt::kSwWaterIm + b] = t->water_refindex[2 * b + 1];
+  const double *tabs[3] = {t->extp, t->absp, t->asmp};
+  return set_optics_tables(ctx, what, &ctx->d_optics_sw, t->specrefindex, t->water_refindex,
+                           t->refrtab, t->refitab, tabs, 3, opt::kSwNode, opt::kSwBands);
+}
+
+// The arguments that both optics entries share; volc with the volcanic
+// fields for the radiation-facing entries (its trop set), else null.
+static mam4b_status run_optics(mam4b_ctx *ctx, const char *what, bool sw, const double *in_slab,
+                               size_t ld, const double *pdeldry, double *out, double *aodvis,
+                               int ncol, int nlev, double dt, const OpticsArgs *volc,
+                               cudaStream_t s) {
+  OpticsArgs a;
+  memset(&a, 0, sizeof(a));
+  if (volc)
+    a = *volc;
+  const size_t n = (size_t)ncol * nlev;
+  for (int f = 0; f < MAM4B_NIN; ++f)
+    a.in[f] = in_slab + (size_t)f * ld;
+  a.pdeldry = pdeldry;
+  a.tables = sw ? ctx->d_optics_sw : ctx->d_optics_lw;
+  a.out = out;
+  a.aodvis = aodvis;
+  a.ld = ld;
+  a.ncell = (long long)n;
+  a.ncol = ncol;
+  a.nlev = nlev;
+  a.dt = dt;
+  a.scr = ctx->d_optics_scr;
+  const unsigned grid = (unsigned)((n + 127) / 128), grid2 = (unsigned)((n + 255) / 256);
+  const unsigned cells = std::min((unsigned)((n + kBandBlock - 1) / kBandBlock), kBandCellBlocks);
+  optics_size_kernel<<<grid, 128, 0, s>>>(a);
+  int launches = 3;
+  if (sw) {
+    optics_mode_kernel<true><<<dim3(grid2, NMODE), 256, 0, s>>>(a);
+    optics_sw_band_kernel<<<dim3(opt::kSwBands, cells), kBandBlock, 0, s>>>(a);
+    if (aodvis) {
+      optics_sw_aod_kernel<<<(unsigned)((ncol + 3) / 4), 128, 0, s>>>(a);
+      ++launches;
+    }
+  } else {
+    optics_mode_kernel<false><<<dim3(grid2, NMODE), 256, 0, s>>>(a);
+    optics_band_kernel<<<dim3(opt::kLwBands, cells), kBandBlock, 0, s>>>(a);
   }
-  memcpy(h + opt::kSwRefr, t->refrtab, sizeof(double) * 4 * opt::kSwBands * opt::kPrefr);
-  memcpy(h + opt::kSwRefi, t->refitab, sizeof(double) * 4 * opt::kSwBands * opt::kPrefi);
-  memcpy(h + opt::kSwExt, t->extp, sizeof(double) * 4 * opt::kSwBands * opt::kSwTab);
-  memcpy(h + opt::kSwAbs, t->absp, sizeof(double) * 4 * opt::kSwBands * opt::kSwTab);
-  memcpy(h + opt::kSwAsm, t->asmp, sizeof(double) * 4 * opt::kSwBands * opt::kSwTab);
-  cudaError_t e = cudaSuccess;
-  if (!ctx->d_optics_sw)
-    e = cudaMalloc(&ctx->d_optics_sw, sizeof(double) * opt::kSwTableDoubles);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(ctx->d_optics_sw, h, sizeof(double) * opt::kSwTableDoubles,
-                   cudaMemcpyHostToDevice);
-  free(h);
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return set_err(ctx, MAM4B_ERR_CUDA, what, e);
+  ctx->launches += launches;
   return MAM4B_OK;
+}
+
+// Argument checks and scratch of an optics entry; *empty: nothing to do.
+static mam4b_status begin_optics(mam4b_ctx *ctx, const char *what, bool sw, const double *in_slab,
+                                 size_t ld, const double *pdeldry, const double *out, int ncol,
+                                 int nlev, double dt, cudaStream_t s, bool *empty) {
+  const size_t n = (size_t)(ncol > 0 ? ncol : 0) * (size_t)(nlev > 0 ? nlev : 0);
+  if (!ctx || !in_slab || !pdeldry || !out || ncol < 0 || nlev <= 0 || ld < n || !(dt > 0.0) ||
+      !isfinite(dt))
+    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
+  if (!(sw ? ctx->d_optics_sw : ctx->d_optics_lw))
+    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT,
+                   sw ? "mam4b_optics_sw: tables not set" : "mam4b_optics_lw: tables not set",
+                   cudaSuccess);
+  ctx->last_stream = s;
+  *empty = n == 0;
+  if (*empty)
+    return MAM4B_OK;
+  const cudaError_t e = grow(&ctx->d_optics_scr, &ctx->cap_optics_scr,
+                             (size_t)(sw ? OS_FIELDS : OS_LW_FIELDS) * n);
+  return e == cudaSuccess ? MAM4B_OK : set_err(ctx, MAM4B_ERR_CUDA, what, e);
 }
 
 // modal_aero_opt::modal_aero_sw (modal_aero_opt.hpp:536-878), batched
@@ -5777,51 +5854,13 @@ mam4b_status mam4b_optics_sw(mam4b_ctx *ctx, const double *in_slab, size_t ld,
                              const double *pdeldry, double *out, double *aodvis, int ncol,
                              int nlev, double dt, void *stream) {
   const char *what = "mam4b_optics_sw";
-  const size_t n = (size_t)(ncol > 0 ? ncol : 0) * (size_t)(nlev > 0 ? nlev : 0);
-  if (!ctx || !in_slab || !pdeldry || !out || ncol < 0 || nlev <= 0 || ld < n || !(dt > 0.0) ||
-      !isfinite(dt))
-    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  if (!ctx->d_optics_sw)
-    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, "mam4b_optics_sw: tables not set",
-                   cudaSuccess);
-  OpticsSwArgs w;
-  memset(&w, 0, sizeof(w));
-  for (int f = 0; f < MAM4B_NIN; ++f)
-    w.base.in[f] = in_slab + (size_t)f * ld;
-  w.base.pdeldry = pdeldry;
-  w.base.tables = ctx->d_optics_sw;
-  w.base.ld = ld;
-  w.base.ncell = (long long)n;
-  w.base.dt = dt;
-  w.out = out;
-  w.aodvis = aodvis;
-  w.ncol = ncol;
-  w.nlev = nlev;
   cudaStream_t s = (cudaStream_t)stream;
-  ctx->last_stream = s;
-  if (n == 0)
-    return MAM4B_OK;
-  cudaError_t e = grow(&ctx->d_optics_scr, &ctx->cap_optics_scr, (size_t)SS_FIELDS * n);
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, "mam4b_optics_sw scratch", e);
-  w.base.scr = ctx->d_optics_scr;
-  const int block = 128;
-  const unsigned grid = (unsigned)((n + block - 1) / block);
-  optics_size_kernel<<<grid, block, 0, s>>>(w.base);
-  optics_sw_mode_kernel<<<dim3(grid, NMODE), block, 0, s>>>(w);
-  // at most 1,024 blocks of cells per band: each block stages its band's
-  // tables once and then steps several groups of cells
-  optics_sw_band_kernel<<<dim3(opt::kSwBands, grid < 1024u ? grid : 1024u), block, 0, s>>>(w);
-  int launches = 3;
-  if (aodvis) {
-    optics_sw_aod_kernel<<<(unsigned)((ncol + block - 1) / block), block, 0, s>>>(w);
-    ++launches;
-  }
-  e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-  ctx->launches += launches;
-  return MAM4B_OK;
+  bool empty;
+  const mam4b_status st =
+      begin_optics(ctx, what, true, in_slab, ld, pdeldry, out, ncol, nlev, dt, s, &empty);
+  if (st != MAM4B_OK || empty)
+    return st;
+  return run_optics(ctx, what, true, in_slab, ld, pdeldry, out, aodvis, ncol, nlev, dt, nullptr, s);
 }
 
 // modal_aero_opt::modal_aero_lw_k (modal_aero_opt.hpp:879-989), batched
@@ -5829,70 +5868,64 @@ mam4b_status mam4b_optics_lw(mam4b_ctx *ctx, const double *in_slab, size_t ld,
                              const double *pdeldry, double *tauxar, int ncol, int nlev,
                              double dt, void *stream) {
   const char *what = "mam4b_optics_lw";
-  const size_t n = (size_t)(ncol > 0 ? ncol : 0) * (size_t)(nlev > 0 ? nlev : 0);
-  if (!ctx || !in_slab || !pdeldry || !tauxar || ncol < 0 || nlev <= 0 || ld < n ||
-      !(dt > 0.0) || !isfinite(dt))
-    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  if (!ctx->d_optics_lw)
-    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, "mam4b_optics_lw: tables not set",
-                   cudaSuccess);
-  OpticsLwArgs a;
-  for (int f = 0; f < MAM4B_NIN; ++f)
-    a.in[f] = in_slab + (size_t)f * ld;
-  a.pdeldry = pdeldry;
-  a.tables = ctx->d_optics_lw;
-  a.tau = tauxar;
-  a.ld = ld;
-  a.ncell = (long long)n;
-  a.dt = dt;
   cudaStream_t s = (cudaStream_t)stream;
-  ctx->last_stream = s;
-  if (n == 0)
-    return MAM4B_OK;
-  cudaError_t e = grow(&ctx->d_optics_scr, &ctx->cap_optics_scr, (size_t)OS_FIELDS * n);
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, "mam4b_optics_lw scratch", e);
-  a.scr = ctx->d_optics_scr;
-  const int block = 128;
-  const unsigned grid = (unsigned)((n + block - 1) / block);
-  optics_size_kernel<<<grid, block, 0, s>>>(a);
-  optics_mode_kernel<<<dim3(grid, NMODE), block, 0, s>>>(a);
-  // at most 1,024 blocks of cells per band, as the shortwave band kernel
-  optics_band_kernel<<<dim3(opt::kLwBands, grid < 1024u ? grid : 1024u), block, 0, s>>>(a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-  ctx->launches += 3;
-  return MAM4B_OK;
+  bool empty;
+  const mam4b_status st =
+      begin_optics(ctx, what, false, in_slab, ld, pdeldry, tauxar, ncol, nlev, dt, s, &empty);
+  if (st != MAM4B_OK || empty)
+    return st;
+  return run_optics(ctx, what, false, in_slab, ld, pdeldry, tauxar, nullptr, ncol, nlev, dt,
+                    nullptr, s);
 }
 
-// Tropopause levels of the columns into trop (caller's array, or the
-// context's when NULL); r gets the layout fields.
-static mam4b_status rad_props_tropopause(mam4b_ctx *ctx, const char *what, RadArgs &r,
-                                         const double *in_slab, const double *pint,
-                                         const double *zi, int *trop_level, cudaStream_t s) {
-  r.temp = in_slab + (size_t)MAM4B_IN_T * r.ld;
-  r.pmid = in_slab + (size_t)MAM4B_IN_P * r.ld;
+// Tropopause levels of the columns into *trop_level (the caller's array, or
+// the context's, which it is then set to) and the list of cells at or below
+// them into the context's.
+static mam4b_status rad_props_tropopause(mam4b_ctx *ctx, const char *what, const double *in_slab,
+                                         size_t ld, const double *pint, int ncol, int nlev,
+                                         int **trop_level, cudaStream_t s) {
+  RadArgs r;
+  memset(&r, 0, sizeof(r));
+  r.temp = in_slab + (size_t)MAM4B_IN_T * ld;
+  r.pmid = in_slab + (size_t)MAM4B_IN_P * ld;
   r.pint = pint;
-  r.zi = zi;
-  r.trop = trop_level;
-  if (!r.trop) {
-    if (ctx->cap_trop < (size_t)r.ncol) {
+  r.ncol = ncol;
+  r.nlev = nlev;
+  if (!*trop_level) {
+    if (ctx->cap_trop < (size_t)ncol) {
       cudaFree(ctx->d_trop);
       ctx->d_trop = nullptr;
       ctx->cap_trop = 0;
-      const cudaError_t e = cudaMalloc(&ctx->d_trop, (size_t)r.ncol * sizeof(int));
+      const cudaError_t e = cudaMalloc(&ctx->d_trop, (size_t)ncol * sizeof(int));
       if (e != cudaSuccess)
         return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-      ctx->cap_trop = (size_t)r.ncol;
+      ctx->cap_trop = (size_t)ncol;
     }
-    r.trop = ctx->d_trop;
+    *trop_level = ctx->d_trop;
   }
+  r.trop = *trop_level;
+  const size_t n = (size_t)ncol * nlev;
+  if (n > 0x7fffffffu)
+    return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
+  if (ctx->cap_modal < n) {
+    cudaFree(ctx->d_modal);
+    ctx->d_modal = nullptr;
+    ctx->cap_modal = 0;
+    const cudaError_t e = cudaMalloc(&ctx->d_modal, (n + 1) * sizeof(int));
+    if (e != cudaSuccess)
+      return set_err(ctx, MAM4B_ERR_CUDA, what, e);
+    ctx->cap_modal = n;
+  }
+  r.nmodal = reinterpret_cast<unsigned *>(ctx->d_modal);
+  r.modal = ctx->d_modal + 1;
   const int block = 128, per_block = block / 32;
-  const size_t smem = (size_t)per_block * 4 * r.nlev * sizeof(double);
+  const size_t smem = (size_t)per_block * 4 * nlev * sizeof(double);
   if (smem > 48 * 1024)
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  tropopause_kernel<<<(unsigned)((r.ncol + per_block - 1) / per_block), block, smem, s>>>(r);
+  const cudaError_t e0 = cudaMemsetAsync(r.nmodal, 0, sizeof(unsigned), s);
+  if (e0 != cudaSuccess)
+    return set_err(ctx, MAM4B_ERR_CUDA, what, e0);
+  tropopause_kernel<<<(unsigned)((ncol + per_block - 1) / per_block), block, smem, s>>>(r);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return set_err(ctx, MAM4B_ERR_CUDA, what, e);
@@ -5910,30 +5943,25 @@ mam4b_status mam4b_aero_rad_props_sw(mam4b_ctx *ctx, const double *in_slab, size
   const char *what = "mam4b_aero_rad_props_sw";
   if (!ctx || !pint || !zi || !ext_sw || !ssa_sw || !af_sw || nlev < 2)
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  mam4b_status st = mam4b_optics_sw(ctx, in_slab, ld, pdeldry, out, aodvis, ncol, nlev, dt, stream);
-  if (st != MAM4B_OK || ncol == 0)
-    return st;
   cudaStream_t s = (cudaStream_t)stream;
-  RadArgs r;
-  memset(&r, 0, sizeof(r));
-  r.ld = ld;
-  r.ncol = ncol;
-  r.nlev = nlev;
-  r.ext = ext_sw;
-  r.ssa = ssa_sw;
-  r.af = af_sw;
-  r.out = out;
-  st = rad_props_tropopause(ctx, what, r, in_slab, pint, zi, trop_level, s);
+  bool empty;
+  mam4b_status st = begin_optics(ctx, "mam4b_optics_sw", true, in_slab, ld, pdeldry, out, ncol,
+                                 nlev, dt, s, &empty);
+  if (st != MAM4B_OK || empty)
+    return st;
+  st = rad_props_tropopause(ctx, what, in_slab, ld, pint, ncol, nlev, &trop_level, s);
   if (st != MAM4B_OK)
     return st;
-  const int block = 128;
-  const size_t n = (size_t)ncol * nlev;
-  volcanic_sw_kernel<<<(unsigned)((n + block - 1) / block), block, 0, s>>>(r);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-  ctx->launches += 1;
-  return MAM4B_OK;
+  OpticsArgs v;
+  memset(&v, 0, sizeof(v));
+  v.trop = trop_level;
+  v.nmodal = reinterpret_cast<unsigned *>(ctx->d_modal);
+  v.modal = ctx->d_modal + 1;
+  v.zi = zi;
+  v.ext = ext_sw;
+  v.ssa = ssa_sw;
+  v.af = af_sw;
+  return run_optics(ctx, what, true, in_slab, ld, pdeldry, out, aodvis, ncol, nlev, dt, &v, s);
 }
 
 // aero_rad_props_lw (aero_rad_props.hpp:339-410), batched
@@ -5944,28 +5972,23 @@ mam4b_status mam4b_aero_rad_props_lw(mam4b_ctx *ctx, const double *in_slab, size
   const char *what = "mam4b_aero_rad_props_lw";
   if (!ctx || !pint || !zi || !ext_lw || nlev < 2)
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  mam4b_status st = mam4b_optics_lw(ctx, in_slab, ld, pdeldry, odap, ncol, nlev, dt, stream);
-  if (st != MAM4B_OK || ncol == 0)
-    return st;
   cudaStream_t s = (cudaStream_t)stream;
-  RadArgs r;
-  memset(&r, 0, sizeof(r));
-  r.ld = ld;
-  r.ncol = ncol;
-  r.nlev = nlev;
-  r.ext = ext_lw;
-  r.out = odap;
-  st = rad_props_tropopause(ctx, what, r, in_slab, pint, zi, trop_level, s);
+  bool empty;
+  mam4b_status st = begin_optics(ctx, "mam4b_optics_lw", false, in_slab, ld, pdeldry, odap, ncol,
+                                 nlev, dt, s, &empty);
+  if (st != MAM4B_OK || empty)
+    return st;
+  st = rad_props_tropopause(ctx, what, in_slab, ld, pint, ncol, nlev, &trop_level, s);
   if (st != MAM4B_OK)
     return st;
-  const int block = 128;
-  const size_t n = (size_t)ncol * nlev;
-  volcanic_lw_kernel<<<(unsigned)((n + block - 1) / block), block, 0, s>>>(r);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess)
-    return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-  ctx->launches += 1;
-  return MAM4B_OK;
+  OpticsArgs v;
+  memset(&v, 0, sizeof(v));
+  v.trop = trop_level;
+  v.nmodal = reinterpret_cast<unsigned *>(ctx->d_modal);
+  v.modal = ctx->d_modal + 1;
+  v.zi = zi;
+  v.ext = ext_lw;
+  return run_optics(ctx, what, false, in_slab, ld, pdeldry, odap, nullptr, ncol, nlev, dt, &v, s);
 }
 
 // ndrop::dropmixnuc (ndrop.hpp:1393-1714), one block per column
