@@ -601,7 +601,7 @@ mam4b_status mam4b_aero_rad_props_lw(mam4b_ctx *ctx, const double *in_slab, size
  *              reference reads one level above it)
  *   vertical_mix  enable_aero_vertical_mix
  * factnum starts at zero; rpdel is 1 / pdel. One block of 128 threads per
- * column; about 1 KB of shared memory per level (at most ~200 levels).
+ * column; at most 201 levels.
  * Asynchronous on `stream`.
  */
 enum {

@@ -27,23 +27,13 @@ MAM4B_HD constexpr int mode_of(int p) {
   return p <= K::numslot(0) ? 0 : p <= K::numslot(1) ? 1 : p <= K::numslot(2) ? 2 : 3;
 }
 
-// explmix (ndrop.hpp:1090-1110): droplet number and cloud-borne aerosol
-MAM4B_HD double explmix(double qkm1, double qk, double qkp1, double src, double ekp, double ekm,
-                        double ovp, double ovm, double dtmix) {
-  const double q = qk + dtmix * (src + ekp * (ovp * qkp1 - qk) + ekm * (ovm * qkm1 - qk));
-  return dmax(q, 0.0);
-}
-
-// explmix (ndrop.hpp:1111-1162): interstitial aerosol, which gains the
-// cloud-borne aerosol of neighbouring levels where the cloud does not
-// overlap
-MAM4B_HD double explmix_act(double qkm1, double qk, double qkp1, double src, double ekp,
-                            double ekm, double ovp, double ovm, double dtmix, double qact_km1,
-                            double qact_kp1) {
-  const double q = qk + dtmix * (-src + ekp * (qkp1 - qk + qact_kp1 * (1.0 - ovp)) +
-                                 ekm * (qkm1 - qk + qact_km1 * (1.0 - ovm)));
-  return dmax(q, 0.0);
-}
+// explmix (ndrop.hpp:1090-1110) advances droplet number and cloud-borne
+// aerosol q by dt (src + ekp (ovp q[k+1] - q) + ekm (ovm q[k-1] - q)),
+// explmix (:1111-1162) interstitial aerosol by dt (-src + ekp (q[k+1] - q +
+// qact[k+1] (1 - ovp)) + ekm (q[k-1] - q + qact[k-1] (1 - ovm))), with qact
+// the cloud-borne aerosol: it gains that of neighbouring levels where the
+// cloud does not overlap. Both are bounded below by zero. The column kernel
+// takes them as fused multiply-adds of coefficients with dt multiplied in.
 
 // CCN number [#/cm3] at 0.02, 0.05, 0.1, 0.2, 0.5 and 1 % supersaturation
 // from interstitial plus cloud-borne aerosol (ccncalc, with loadaer's
@@ -91,10 +81,10 @@ MAM4B_HD void ccn_cell(const StepConsts &C, const double (&ai)[NPOP],
       const double amcube = (3.0 / 4.0) / (K::pi * exp45) * vol / na;
       ss_crit = ssat_coeff / sqrt(hyg * amcube);
     }
-    const double argf = (2.0 / 3.0) / (sq2 * alogsig);
+    const double argf = (2.0 / 3.0) / (sq2 * alogsig), lss = log(ss_crit);
 #pragma unroll
     for (int l = 0; l < kPsat; ++l) {
-      const double arg = argf * log(ss_crit / super[l]);
+      const double arg = argf * (lss - log(super[l]));
       ccn[l] += na * 0.5 * (1.0 - erf(arg));
     }
   }
