@@ -97,16 +97,49 @@ enum { CNT_TAKEN = 0, CNT_LONG = 1, CNT_SHORT = 2, CNT_TAKEN_ADJ = 3, CNT_TAKEN_
 constexpr double kCloudy = 0.999;
 
 // ----------------------------------------------------- per-cell amicphys
+__device__ __forceinline__ constexpr int pop_to_i31(int p) { return 6 + p; }
+// amicphys tracer index of the number of mode m (mam4_amicphys.hpp:36)
+__device__ __forceinline__ constexpr int num_i31(int m) {
+  return m == 0 ? 13 : m == 1 ? 18 : m == 2 ? 26 : 30;
+}
+
+// Process tendencies of a grid cell, in the 31-tracer order ([process
+// 0..3][tracer], then cloud-borne renaming [tracer]), straight to the
+// caller's arrays, which may be absent. Every one is a single term, but that
+// renaming in a partly cloudy cell is the clear subarea's plus the cloudy
+// one's, which was stored first (`joined`). Increments come in amicphys
+// units over the step: volume mixing ratio times unit (the unit factor of
+// the species), scaled by the subarea's fraction.
 struct Diag {
-  // amicphys process tendencies for the grid cell, in the 31-tracer
-  // order: [process 0..3][tracer], cloud-borne renaming [tracer]
-  double t[NQTEND][31];
-  double cw[31];
+  const StepArgs &a;
+  long long c;
+  GuardedDivisor per_dt, organic, soag;
+  bool joined;
+  __device__ __forceinline__ Diag(const StepArgs &a_, long long c_)
+      : a(a_), c(c_), per_dt(a_.dt), organic(K::fcvt_aer(0) * a_.dt), soag(c_k.fcvt_soag * a_.dt),
+        joined(false) {}
+  // increment v of a population of species x (number: x < 0)
+  __device__ __forceinline__ double rate(int x, double v) const {
+    return (x == 0 || x == 2 ? organic : per_dt).under(0.0 + v);
+  }
+  __device__ __forceinline__ void put(int k, int i, double t) const {
+    double *d = a.diag[k * 31 + i];
+    if (d)
+      d[c] = k == 1 && joined ? (0.0 + t) + d[c] : 0.0 + t;
+  }
 };
 
-__device__ __forceinline__ int pop_to_i31(int p) { return 6 + p; }
-// amicphys tracer index of the number of mode m (mam4_amicphys.hpp:36)
-__device__ __forceinline__ int num_i31(int m) { return m == 0 ? 13 : m == 1 ? 18 : m == 2 ? 26 : 30; }
+// Zeros to the fields that a cell leaves without a term: bit i of fields[k] is
+// tracer i of process k.
+__device__ __forceinline__ void diag_zeros(const StepArgs &a, long long c,
+                                           const unsigned (&fields)[NQTEND + 1]) {
+#pragma unroll 1
+  for (int k = 0; k <= NQTEND; ++k)
+#pragma unroll 1
+    for (int i = 0; i < 31; ++i)
+      if (((fields[k] >> i) & 1u) && a.diag[31 * k + i])
+        a.diag[31 * k + i][c] = 0.0;
+}
 
 // Hand-off of a cell with a clear subarea from the first stage to the later
 // ones: one double per field and cell.
@@ -164,8 +197,8 @@ __device__ __forceinline__ void clear_prefix(const StepArgs &a, double deltat, d
 }
 
 // Part 2, after the SOA loop: H2SO4 update, renaming, nucleation,
-// coagulation, aging. With DIAG the per-process increments are added to dg
-// scaled by afrac/(fcvt*deltat). With PRECOAG, cc_pre (stride cc_stride)
+// coagulation, aging. With DIAG the per-process increments go to dg, scaled
+// by afrac. With PRECOAG, cc_pre (stride cc_stride)
 // holds the 12 coagulation coefficients of the cell (coag_all_coefs) and
 // dgn_awet/wetdens are not read.
 template <bool DIAG, bool PRECOAG>
@@ -221,8 +254,8 @@ __device__ __forceinline__ void clear_suffix(const StepArgs &a, double deltat, d
         for (int m = 0; m < NMODE; ++m)
           dcond[x][m] = s.aer[x][m] - cm.sv_all[x][m];
       // gas increment of condensation (mam4_amicphys.hpp:1434-1438)
-      dg->t[0][5] += ((0.0 + (s.gas[0] - (cm.gas_sv[0] + 0.0 * dtsub))) / (C.fcvt_soag * deltat)) * afrac;
-      dg->t[0][2] += ((0.0 + (s.gas[1] - (cm.gas_sv[1] + cm.netprod1 * dtsub))) / (1.0 * deltat)) * afrac;
+      dg->put(0, 5, dg->soag.under(0.0 + (s.gas[0] - (cm.gas_sv[0] + 0.0 * dtsub))) * afrac);
+      dg->put(0, 2, dg->rate(-1, s.gas[1] - (cm.gas_sv[1] + cm.netprod1 * dtsub)) * afrac);
     }
   }
 
@@ -243,13 +276,12 @@ __device__ __forceinline__ void clear_suffix(const StepArgs &a, double deltat, d
     if (DIAG) {
 #pragma unroll
       for (int m = 0; m < NMODE; ++m) {
-        dg->t[1][num_i31(m)] += ((0.0 + (s.num[m] - nsv[m])) / (1.0 * deltat)) * afrac;
+        dg->put(1, num_i31(m), dg->rate(-1, s.num[m] - nsv[m]) * afrac);
 #pragma unroll
         for (int x = 0; x < NAER; ++x) {
           const int slot = K::aer_slot(x, m);
           if (slot >= 0)
-            dg->t[1][pop_to_i31(slot)] +=
-                ((0.0 + (s.aer[x][m] - asv[x][m])) / (K::fcvt_aer(x) * deltat)) * afrac;
+            dg->put(1, pop_to_i31(slot), dg->rate(x, s.aer[x][m] - asv[x][m]) * afrac);
         }
       }
     }
@@ -260,9 +292,9 @@ __device__ __forceinline__ void clear_suffix(const StepArgs &a, double deltat, d
     const double g1 = s.gas[1], n1 = s.num[1], a1 = s.aer[1][1];
     nucleation(C, dtsub, temp, pmid, zmid, pblh, relhum, uptkrate_h2so4, qgas_avg1, s);
     if (DIAG) {
-      dg->t[2][2] += ((0.0 + (s.gas[1] - g1)) / (1.0 * deltat)) * afrac;
-      dg->t[2][18] += ((0.0 + (s.num[1] - n1)) / (1.0 * deltat)) * afrac;
-      dg->t[2][14] += ((0.0 + (s.aer[1][1] - a1)) / (1.0 * deltat)) * afrac;
+      dg->put(2, 2, dg->rate(-1, s.gas[1] - g1) * afrac);
+      dg->put(2, 18, dg->rate(-1, s.num[1] - n1) * afrac);
+      dg->put(2, 14, dg->rate(1, s.aer[1][1] - a1) * afrac);
     }
   }
 
@@ -300,12 +332,12 @@ __device__ __forceinline__ void clear_suffix(const StepArgs &a, double deltat, d
       }
 #pragma unroll
       for (int m = 0; m < NMODE; ++m) {
-        dg->t[3][num_i31(m)] += ((0.0 + dncoag[m]) / (1.0 * deltat)) * afrac;
+        dg->put(3, num_i31(m), dg->rate(-1, dncoag[m]) * afrac);
 #pragma unroll
         for (int x = 0; x < NAER; ++x) {
           const int slot = K::aer_slot(x, m);
           if (slot >= 0)
-            dg->t[3][pop_to_i31(slot)] += ((0.0 + dcoag[x][m]) / (K::fcvt_aer(x) * deltat)) * afrac;
+            dg->put(3, pop_to_i31(slot), dg->rate(x, dcoag[x][m]) * afrac);
         }
       }
     }
@@ -321,12 +353,12 @@ __device__ __forceinline__ void clear_suffix(const StepArgs &a, double deltat, d
 #pragma unroll
     for (int m = 0; m < NMODE; ++m) {
       if (a.do_cond)
-        dg->t[0][num_i31(m)] += ((0.0 + dncond[m]) / (1.0 * deltat)) * afrac;
+        dg->put(0, num_i31(m), dg->rate(-1, dncond[m]) * afrac);
 #pragma unroll
       for (int x = 0; x < NAER; ++x) {
         const int slot = K::aer_slot(x, m);
         if (slot >= 0 && a.do_cond)
-          dg->t[0][pop_to_i31(slot)] += ((0.0 + dcond[x][m]) / (K::fcvt_aer(x) * deltat)) * afrac;
+          dg->put(0, pop_to_i31(slot), dg->rate(x, dcond[x][m]) * afrac);
       }
     }
   } else {
@@ -521,20 +553,17 @@ __device__ __forceinline__ void cloudy_rename(const StepArgs &a, Sub &si, Sub &s
     rename_subarea<true>(C, si, sc, zero7, zero7);
   }
   if (DIAG && a.do_rename) {
-    const double dt = a.dt;
 #pragma unroll
     for (int m = 0; m < NMODE; ++m) {
       const int ln = num_i31(m);
-      dg->t[1][ln] += ((0.0 + (si.num[m] - nsv_i[m])) / (1.0 * dt)) * f;
-      dg->cw[ln] += ((0.0 + (sc.num[m] - nsv_c[m])) / (1.0 * dt)) * f;
+      dg->put(1, ln, dg->rate(-1, si.num[m] - nsv_i[m]) * f);
+      dg->put(NQTEND, ln, dg->rate(-1, sc.num[m] - nsv_c[m]) * f);
 #pragma unroll
       for (int x = 0; x < NAER; ++x) {
         const int slot = K::aer_slot(x, m);
         if (slot >= 0) {
-          dg->t[1][pop_to_i31(slot)] +=
-              ((0.0 + (si.aer[x][m] - asv_i[x][m])) / (K::fcvt_aer(x) * dt)) * f;
-          dg->cw[pop_to_i31(slot)] +=
-              ((0.0 + (sc.aer[x][m] - asv_c[x][m])) / (K::fcvt_aer(x) * dt)) * f;
+          dg->put(1, pop_to_i31(slot), dg->rate(x, si.aer[x][m] - asv_i[x][m]) * f);
+          dg->put(NQTEND, pop_to_i31(slot), dg->rate(x, sc.aer[x][m] - asv_c[x][m]) * f);
         }
       }
     }
@@ -657,18 +686,10 @@ __device__ __forceinline__ void cell_step(const StepArgs &a, const long long c) 
   Front f;
   cell_front<true>(a, c, f);
   const double dt = a.dt;
-  Diag dgv;
+  Diag dgv(a, c);
   Diag *dg = DIAG ? &dgv : nullptr;
-  if (DIAG) {
-#pragma unroll
-    for (int k = 0; k < NQTEND; ++k)
-#pragma unroll
-      for (int i = 0; i < 31; ++i)
-        dgv.t[k][i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < 31; ++i)
-      dgv.cw[i] = 0.0;
-  }
+  if (DIAG)
+    diag_zeros(a, c, {~0u, ~0u, ~0u, ~0u, ~0u});
   // outgoing grid-cell means (amicphys units): gases, interstitial, cloud
   double o_h2so4, o_soag, oi[NPOP], oc[NPOP];
   const double fsoag = C.fcvt_soag;
@@ -710,27 +731,11 @@ __device__ __forceinline__ void cell_step(const StepArgs &a, const long long c) 
     Sub s;
     double gcl[2], rhc, ci[NPOP], cg[2];
     partly_cloudy_setup<DIAG>(a, f, s, gcl, rhc, ci, cg, oc, dg);
-    Diag dclear;
-    Diag *dcp = DIAG ? &dclear : nullptr;
-    if (DIAG) {
-#pragma unroll
-      for (int k = 0; k < NQTEND; ++k)
-#pragma unroll
-        for (int i = 0; i < 31; ++i)
-          dclear.t[k][i] = 0.0;
-    }
+    dgv.joined = true;
     const int niter = clear_subarea<DIAG>(a, dt, f.temp, f.pmid, f.zm, f.pblh, rhc, f.dgn_a,
-                                                f.dgn_awet, f.wetdens, qgas1, s, dcp, fclea);
+                                                f.dgn_awet, f.wetdens, qgas1, s, dg, fclea);
     if (niter > 1000)
       atomicOr(a.flags, MAM4B_FLAG_SOA_NITER_LIMIT);
-    if (DIAG) {
-      // jsub 1 then jsub 2: t = (0 + clear) + cloudy
-#pragma unroll
-      for (int k = 0; k < NQTEND; ++k)
-#pragma unroll
-        for (int i = 0; i < 31; ++i)
-          dgv.t[k][i] = dclear.t[k][i] + dgv.t[k][i];
-    }
     o_soag = dmax(0.0, (0.0 + (map_gas ? s.gas[0] / fsoag : gcl[0]) * fclea) + cg[0]);
     o_h2so4 = dmax(0.0, (0.0 + (map_gas ? s.gas[1] / 1.0 : gcl[1]) * fclea) + cg[1]);
 #pragma unroll
@@ -746,18 +751,6 @@ __device__ __forceinline__ void cell_step(const StepArgs &a, const long long c) 
   }
 
   store_outputs(a, c, o_h2so4, o_soag, oi, oc, f.h2so4, f.soag, f.ai, f.ac);
-  if (DIAG) {
-#pragma unroll
-    for (int k = 0; k < NQTEND; ++k)
-#pragma unroll
-      for (int i = 0; i < 31; ++i)
-        if (a.diag[k * 31 + i])
-          a.diag[k * 31 + i][c] = dgv.t[k][i];
-#pragma unroll
-    for (int i = 0; i < 31; ++i)
-      if (a.diag[4 * 31 + i])
-        a.diag[4 * 31 + i][c] = dgv.cw[i];
-  }
 }
 
 // ---- the step with the chemistry that precedes amicphys, one thread per
@@ -1049,11 +1042,6 @@ __device__ __forceinline__ void append_loop(const StepArgs &a, long long c, doub
     a.order[a.ncell - 1 - (b_short + __popc(m_short & below))] = (int)c;
 }
 
-template <class Src>
-__device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c, double temp,
-                                            double pmid, double zm, double cld, double pblh,
-                                            double relhum, double dgn_pc, Sub &s, ClearMid &cm,
-                                            const Src &src);
 template <int SOA, class State>
 __device__ __forceinline__ bool soa_pass(State &st, bool fast);
 
@@ -1159,7 +1147,7 @@ __device__ __forceinline__ void cell_pre_chem(const StepArgs &a, const ChemArgs 
 // soag()): from registers in pre's fused path, from the hand-off and the
 // inputs in post_kernel, where reading them only when needed keeps them out
 // of registers during the suffix.
-template <class Src>
+template <bool DIAG, class Src>
 __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c, double temp,
                                             double pmid, double zm, double cld, double pblh,
                                             double relhum, double dgn_pc, Sub &s, ClearMid &cm,
@@ -1170,8 +1158,10 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
   // wet sizes enter the suffix only through the coagulation coefficients,
   // which pair_kernel computed
   const double unused[NMODE] = {0, 0, 0, 0};
-  clear_suffix<false, true>(a, dt, temp, pmid, zm, pblh, relhum, dgn_pc, unused, unused, cm, s,
-                            nullptr, 0.0, a.aux + AUX_COAG * n + c, n);
+  Diag dgv(a, c);
+  dgv.joined = !(cld < 1.0e-5);
+  clear_suffix<DIAG, true>(a, dt, temp, pmid, zm, pblh, relhum, dgn_pc, unused, unused, cm, s,
+                           &dgv, dgv.joined ? 1.0 - cld : 1.0, a.aux + AUX_COAG * n + c, n);
   // recombination (form_gcm_of_gases_and_aerosols_from_subareas)
   const GuardedDivisor dsoag(C.fcvt_soag);
   constexpr GuardedDivisor organic = constant_divisor(K::fcvt_aer(0));
@@ -1232,6 +1222,7 @@ struct FinishLoads {
 
 // Second half of a cell with a clear subarea: the state at the SOA loop
 // (hand-off), the loop's result (solver), then cell_finish.
+template <bool DIAG = false>
 __device__ __forceinline__ void cell_post(const StepArgs &a, const long long c) {
   const size_t n = (size_t)a.ncell;
   const double cld = __ldg(a.in[MAM4B_IN_CLD] + c);
@@ -1263,8 +1254,19 @@ __device__ __forceinline__ void cell_post(const StepArgs &a, const long long c) 
 #pragma unroll
   for (int k = 0; k < NMODE; ++k)
     cm.uptk1[k] = h[(H_UPTK + k) * n];
+  if (DIAG) {
+    cm.gas_sv[0] = h[H_SOAG0 * n];
+    cm.gas_sv[1] = s.gas[1];
+#pragma unroll
+    for (int m = 0; m < NMODE; ++m)
+#pragma unroll
+      for (int x = 0; x < NAER; ++x) {
+        const int slot = K::aer_slot(x, m);
+        cm.sv_all[x][m] = slot >= 0 ? h[(H_POP + slot) * n] : 0.0;
+      }
+  }
   const FinishLoads src{a, c, h, n};
-  cell_finish(a, c, temp, pmid, zm, cld, pblh, h[H_RELHUM * n], h[H_DGN_PC * n], s, cm, src);
+  cell_finish<DIAG>(a, c, temp, pmid, zm, cld, pblh, h[H_RELHUM * n], h[H_DGN_PC * n], s, cm, src);
 }
 
 template <bool DIAG>
@@ -1536,6 +1538,7 @@ __device__ __forceinline__ void partition(double q_i, double q_c, double fcldy,
 // the hand-off; cells that are not cloudy) and the cloudy subarea before
 // renaming. The aitken mode renames and leaves what
 // moves in x; the accumulation mode takes it in front_out.
+template <bool DIAG>
 __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, double cld,
                                            double adj_inv, FrontMode &f, double *x, int stride) {
   const StepConsts &C = c_k;
@@ -1677,6 +1680,22 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
       renamed = rename_fractions<true>(C, ti - 0.0, 0.0, tc - 0.0, 0.0, f.sni, f.snc, xn, xv);
     }
     double mn_i = 0.0, mn_c = 0.0, mi[4] = {0, 0, 0, 0}, mc[4] = {0, 0, 0, 0};
+    if constexpr (DIAG)
+      if (a.do_rename) {
+        const double w = cloudy ? 1.0 : cld;
+        auto lost = [](double v, double by, bool yes) { return yes ? (v - by) - v : v - v; };
+        const Diag dg(a, c);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          const int x = k < 4 ? K::mode_spec(1, k < 4 ? k : 0) : -1;
+          const int i = pop_to_i31(k < 4 ? K::spec0(1) + k : K::numslot(1));
+          const double vi = k < 4 ? f.si[k < 4 ? k : 0] : f.sni;
+          const double vc = k < 4 ? f.sc[k < 4 ? k : 0] : f.snc;
+          const double part = k < 4 ? xv : xn;
+          dg.put(1, i, dg.rate(x, lost(vi, vi * part, renamed)) * w);
+          dg.put(NQTEND, i, dg.rate(x, lost(vc, vc * part, renamed)) * w);
+        }
+      }
     if (renamed) {
       mn_i = f.sni * xn;
       mn_c = f.snc * xn;
@@ -1700,9 +1719,44 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
   }
 }
 
+// The process tendencies of renaming in cloud that front_mode did not store
+// (it stores the aitken mode's); zero for the cloud-borne populations of a
+// clear cell.
+__device__ __forceinline__ void front_rename_diag(const StepArgs &a, long long c, double cld,
+                                                  const FrontMode &f, const double *x,
+                                                  int stride) {
+  const bool clear = cld < 1.0e-5;
+  if (f.m == 1 && !clear && a.do_rename)
+    return;
+  const double w = cld > kCloudy ? 1.0 : cld;
+  const Diag dg(a, c);
+#pragma unroll
+  for (int s = 0; s <= 7; ++s) {
+    if (s >= f.ns && s < 7)
+      continue;
+    const int i = pop_to_i31(s == 7 ? f.num : f.s0 + (s < 7 ? s : 0));
+    double ti = 0.0, tc = 0.0;
+    if (!clear && a.do_rename) {
+      const int k = s == 7 ? -1 : c_modes.common[f.m][s < 7 ? s : 0];
+      const double vi = s == 7 ? f.sni : f.si[s < 7 ? s : 0];
+      const double vc = s == 7 ? f.snc : f.sc[s < 7 ? s : 0];
+      const bool gains = f.m == 0 && (s == 7 || k >= 0);
+      ti = (gains ? vi + x[(XF_RN_I + 1 + k) * stride] : vi) - vi;
+      tc = (gains ? vc + x[(XF_RN_C + 1 + k) * stride] : vc) - vc;
+      const bool org = s < 7 && c_modes.fcvt[f.m][s < 7 ? s : 0] != 1.0;
+      ti = dg.rate(org ? 0 : -1, ti) * w;
+      tc = dg.rate(org ? 0 : -1, tc) * w;
+    }
+    if (!clear)
+      dg.put(1, i, ti);
+    dg.put(NQTEND, i, tc);
+  }
+}
+
 // What leaves the stage after renaming: cloud-borne tendencies; the
 // interstitial tendencies of a cloudy cell, or the cloudy subarea's
 // contributions to the grid means of a partly cloudy one.
+template <bool DIAG>
 __device__ __forceinline__ void front_out(const StepArgs &a, long long c, double cld,
                                           FrontMode &f, const double *x, int stride) {
   const StepConsts &C = c_k;
@@ -1714,6 +1768,8 @@ __device__ __forceinline__ void front_out(const StepArgs &a, long long c, double
   constexpr GuardedDivisor organic = constant_divisor(K::fcvt_aer(0));
   static_assert(K::fcvt_aer(0) == K::fcvt_aer(2), "SOA and POM share their unit factor");
   const double w = cloudy ? 1.0 : cld;
+  if constexpr (DIAG)
+    front_rename_diag(a, c, cld, f, x, stride);
   if (m == 0 && !clear) {
     f.sni += x[XF_RN_I * stride];
     f.snc += x[XF_RN_C * stride];
@@ -1819,7 +1875,7 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
 
 // LOOP: grid-stride loop over groups of cells (cells_per_thread > 1).
 // Dynamic shared memory: XF_FIELDS doubles per cell.
-template <int R, bool LOOP>
+template <int R, bool LOOP, bool DIAG = false>
 __global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ double s_x[];
   const int cells = blockDim.x / 2;
@@ -1840,7 +1896,7 @@ __global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) 
     if (blockIdx.y == 0)
       __syncthreads();
     if (valid) {
-      front_mode(a, c, cld, adj_inv, f, x, cells);
+      front_mode<DIAG>(a, c, cld, adj_inv, f, x, cells);
       if (f.m == 3)
         front_uptake(a, c, cld);
       if (f.m == 0)
@@ -1849,7 +1905,7 @@ __global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) 
     if (blockIdx.y == 0)
       __syncthreads();
     if (valid)
-      front_out(a, c, cld, f, x, cells);
+      front_out<DIAG>(a, c, cld, f, x, cells);
     if constexpr (!LOOP)
       break;
     if (blockIdx.y == 0)
@@ -2094,6 +2150,26 @@ __global__ void __maxnreg__(R) post_kernel(const __grid_constant__ StepArgs a) {
   } else if (c0 < a.ncell && (!fused || !a.done[c0])) {
     cell_post(a, c0);
   }
+}
+
+// The post stage with process tendencies. The front stage has stored those
+// of renaming in cloud (processes 1 and 4 of the populations). Bound by the
+// latency of the suffix and of some hundred stores a cell, as post_kernel;
+// 128 registers keep 16 warps per SM.
+__global__ void __launch_bounds__(128, 4) post_diag_kernel(const __grid_constant__ StepArgs a) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= a.ncell)
+    return;
+  const double cld = __ldg(a.in[MAM4B_IN_CLD] + c);
+  const bool cloudy = cld > kCloudy;
+  constexpr unsigned all = 0x7fffffffu, gases = 0x3fu, mapped = 1u << 2 | 1u << 5;
+  constexpr unsigned nucleated = 1u << 2 | 1u << 14 | 1u << 18;
+  const bool keep_rename = a.do_rename || !(cld < 1.0e-5);
+  diag_zeros(a, c,
+             {cloudy ? all : gases & ~mapped, keep_rename ? gases : all,
+              cloudy || !a.do_newnuc ? all : all & ~nucleated, cloudy || !a.do_coag ? all : gases,
+              gases});
+  cell_post<true>(a, c);
 }
 
 // SOA sub-stepping of the queued cells.
@@ -4412,6 +4488,8 @@ struct mam4b_ctx {
   size_t cap_optics_scr;
   int *d_trop;          // [cap_trop]: tropopause level per column (aero_rad_props)
   size_t cap_trop;
+  double *d_diag;       // scratch of the step with process tendencies
+  size_t cap_diag;      // its cells
   int *d_modal;         // [cap_modal + 1]: number and list of cells with modal optics
   size_t cap_modal;
   double *d_dmx;        // dropmixnuc activation results (DA_FIELDS per cell), grown
@@ -4542,6 +4620,38 @@ void set_step_scratch(const mam4b_ctx *ctx, StepArgs &a, size_t c0, int chunk) {
   a.counters = ctx->d_counters + (size_t)CNT_WORDS * chunk;
 }
 
+// Scratch of the step with process tendencies, an allocation of its own that
+// only such steps grow. False when there is none to be had: under capture
+// (such a step has always been capturable from its first call, and what it
+// captures must not depend on a later call's growth) or out of memory.
+bool set_diag_scratch(mam4b_ctx *ctx, StepArgs &a, cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!a.do_cond || cudaStreamIsCapturing(s, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  const size_t n = (size_t)a.ncell, fields = SOA_FIELDS + H_FIELDS + AUX_FIELDS;
+  if (ctx->cap_diag < n) {
+    cudaFree(ctx->d_diag);
+    ctx->d_diag = nullptr;
+    ctx->cap_diag = 0;
+    if (cudaMalloc(&ctx->d_diag, n * (fields * sizeof(double) + 2 * sizeof(int)) +
+                                     CNT_WORDS * sizeof(unsigned)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    ctx->cap_diag = n;
+  }
+  a.soa = ctx->d_diag;
+  a.hand = a.soa + SOA_FIELDS * n;
+  a.aux = a.hand + H_FIELDS * n;
+  a.done = (int *)(a.aux + AUX_FIELDS * n);
+  a.order = a.done + n;
+  a.counters = (unsigned *)(a.order + n);
+  return true;
+}
+
 // ----------------------------------------------------- launch shapes
 // The forward pipeline's launch shape (mam4b_tuning): block sizes, register
 // caps (compiled variants of the whole-cell kernels) and cells per thread.
@@ -4668,12 +4778,13 @@ void launch_post(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
 // ev[6] after the last: the per-stage times of mam4b_autotune.
 cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_in,
                               cudaStream_t s, int precision, const ChemArgs *ch, cudaEvent_t *ev,
-                              std::atomic<unsigned long long> *launches) {
+                              std::atomic<unsigned long long> *launches, bool diag = false) {
   StepArgs a = a_in;
   a.mixed = precision != MAM4B_FP64;
   // short SOA loops finish in pre unless the adjoint needs every loop's
   // pass count (npass) or the loop runs in FP32 (MIXED_FAST)
-  const bool fuse = t.inline_scale > 0 && !a.npass && precision != MAM4B_MIXED_FAST;
+  const bool fuse =
+      t.inline_scale > 0 && !a.npass && precision != MAM4B_MIXED_FAST && !diag;
   a.inline_scale = fuse ? (double)t.inline_scale : 0.0;
   cudaError_t e = cudaMemsetAsync(a.counters, 0, CNT_WORDS * sizeof(unsigned), s);
   if (e != cudaSuccess)
@@ -4699,6 +4810,9 @@ cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_
   mark(0);
   if (ch)
     size_kernel<<<grid_for(a.ncell, 128, 1), 128, 0, s>>>(a);
+  else if (diag)
+    front_kernel<128, false, true><<<dim3(grid_for(a.ncell, 64, 1), 2), 128,
+                                     (size_t)XF_FIELDS * 64 * sizeof(double), s>>>(a);
   else
     launch_front(t, a, s);
   mark(1);
@@ -4718,7 +4832,9 @@ cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_
   // the adjoint's forward (npass set) has no post stage: adj_post_kernel
   // recomputes the suffix from the hand-off, and the forward's outputs are
   // not returned
-  if (!a.npass)
+  if (diag)
+    post_diag_kernel<<<grid_for(a.ncell, 128, 1), 128, 0, s>>>(a);
+  else if (!a.npass)
     launch_post(t, a, s);
   mark(6);
   e = cudaGetLastError();
@@ -5120,6 +5236,7 @@ mam4b_status mam4b_destroy(mam4b_ctx *ctx) {
   cudaFree(ctx->d_optics_sw);
   cudaFree(ctx->d_trop);
   cudaFree(ctx->d_modal);
+  cudaFree(ctx->d_diag);
   cudaFree(ctx->d_dmx);
   cudaFree(ctx->d_coag_cc);
   if (ctx->host_streams) {
@@ -5176,8 +5293,17 @@ mam4b_status mam4b_step(mam4b_ctx *ctx, const mam4b_state_view *in, const mam4b_
   if (diag && precision != MAM4B_FP64)
     return set_err(ctx, MAM4B_ERR_NOT_SUPPORTED,
                    "mam4b_step: process diagnostics are FP64 only", cudaSuccess);
+  // with process tendencies, in the pipeline's stages where their scratch can
+  // be had (1,024 x 72 cells: 0.27 ms against 0.78 ms start to end in one
+  // thread per cell, which waits for instructions and spilled registers)
+  if (diag && set_diag_scratch(ctx, a, s)) {
+    e = launch_pipeline_t(ctx->tune, ctx->sms, a, s, precision, nullptr, nullptr, &ctx->launches,
+                          true);
+    if (e != cudaSuccess)
+      return set_err(ctx, MAM4B_ERR_CUDA, "mam4b_step launch", e);
+    return MAM4B_OK;
+  }
   if (diag) {
-    // per-process diagnostics: one thread per cell, start to end
     full_kernel<true><<<(unsigned)grid, block, 0, s>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess)
