@@ -114,7 +114,6 @@ MAM4B_HD bool newton(const System &s, const Het &het, double dti,
       if (fabs(f) > kSmallForcing && !(fabs(f) <= kRelErr * fabs(v)))
         all = false;
     };
-#pragma unroll
     for (int k = kImplicit - 1; k >= 4; --k) {
       const double h = het(k + 1);
       double f = y[k + 1] * dti - (inv_term[k] - h * y[k + 1]);
@@ -132,7 +131,6 @@ MAM4B_HD bool newton(const System &s, const Het &het, double dti,
     f[1] -= s.c12 * f[2];
     f[1] *= 1.0 / (s.lin_diag[1] - dti);
     f[0] *= 1.0 / (s.lin_diag[0] - dti);
-#pragma unroll
     for (int k = 3; k >= 0; --k)
       finish(k, f[k]);
     if (it > 0 && all)
@@ -141,35 +139,24 @@ MAM4B_HD bool newton(const System &s, const Het &het, double dti,
   return false;
 }
 
-// gas_phase_chemistry for one cell: qq [tracers, mol/mol] advanced over
-// delt by the implicit Euler scheme with imp_sol's step control (halve the
-// step after a failed Newton solve, the fifth time cut it to a tenth;
-// double it after two converged steps; the interval counts the step as
-// taken either way). extfrc [molecules/cm3/s], het(t) the removal rate of
-// tracer t [1/s].
+// imp_sol's sub-steps of y over delt, each with a Newton solve: halve the
+// step after a failed solve, the fifth time cut it to a tenth; double it
+// after two converged steps; the interval counts the step as taken either
+// way. ind: independent production.
 template <class Het>
-MAM4B_HD void gas_chemistry_cell(double temp, double delt, double photo,
-                                 const double (&extfrc)[kExt], const double (&inv)[kInv],
-                                 const Het &het, double (&qq)[kTracers]) {
-  double r[kRxn];
-  reaction_rates(temp, photo, inv, r);
-  System s;
-  make_system(r, het, s);
-  double ind[kImplicit];
-#pragma unroll
-  for (int k = 0; k < kImplicit; ++k) {
-    const int e = ext_of_species(k);
-    ind[k] = k == 0 ? +r[1] : (e >= 0 ? +(extfrc[e] / inv[0]) : 0.0);
-  }
+#ifdef __CUDACC__
+__noinline__
+#endif
+MAM4B_HD void implicit_steps(const System &s, const Het &het, double delt,
+                             const double (&ind)[kImplicit], double (&y)[kTracers]) {
   double dt = delt, done = 0.0;
   int cuts = 0, good = 0;
   for (int step = 0; step < kStepsMax; ++step) {
     const double dti = 1.0 / dt;
     double inv_term[kImplicit];
-#pragma unroll
     for (int k = 0; k < kImplicit; ++k)
-      inv_term[k] = dti * qq[k + 1] + ind[k];
-    const bool ok = newton(s, het, dti, inv_term, qq);
+      inv_term[k] = dti * y[k + 1] + ind[k];
+    const bool ok = newton(s, het, dti, inv_term, y);
     if (!ok) {
       good = 0;
       if (cuts < kCutLimit) {
@@ -188,6 +175,104 @@ MAM4B_HD void gas_chemistry_cell(double temp, double delt, double photo,
     }
     dt = dmin(dt, delt - done);
   }
+}
+
+// gas_phase_chemistry for one cell over delt from the values start(t)
+// [mol/mol] of the tracers, into qq: the implicit Euler scheme of imp_sol.
+// extfrc [molecules/cm3/s], het(t) the removal rate of tracer t [1/s].
+// The system is linear, so the first step, over all of delt, nearly always
+// converges in two iterations, and then that is all. They run species by
+// species, so that nothing but the result is held of each; what they do not
+// finish starts again with implicit_steps.
+template <class Het, class Start>
+MAM4B_HD void gas_chemistry_from(double temp, double delt, double photo,
+                                 const double (&extfrc)[kExt], const double (&inv)[kInv],
+                                 const Het &het, const Start &start, double (&qq)[kTracers]) {
+  double r[kRxn];
+  reaction_rates(temp, photo, inv, r);
+  System s;
+  make_system(r, het, s);
+  const GuardedDivisor air(inv[0]);
+  auto production = [&](int k) {
+    const int e = ext_of_species(k);
+    return k == 0 ? +r[1] : (e >= 0 ? +air.under(extfrc[e >= 0 ? e : 0]) : 0.0);
+  };
+  const double dti = quot(1.0, delt);
+  bool all = true;
+  auto finish = [&](int it, double f, double &y) {
+    double v = y + f;
+    if (v < 0.0)
+      v = 0.0;
+    y = v;
+    if (it > 0 && fabs(f) > kSmallForcing && !(fabs(f) <= kRelErr * fabs(v)))
+      all = false;
+  };
+  qq[0] = start(0);
+#pragma unroll
+  for (int k = kImplicit - 1; k >= 4; --k) {
+    double y = start(k + 1);
+    const double h = het(k + 1), d = quot(1.0, -(+h) - dti), term = dti * y + production(k);
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      double f = y * dti - (term - h * y);
+      f *= d;
+      finish(it, f, y);
+    }
+    qq[k + 1] = y;
+  }
+  {
+    double y[5], term[4], d[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      y[k + 1] = start(k + 1);
+      term[k] = dti * y[k + 1] + production(k);
+      d[k] = quot(1.0, s.lin_diag[k] - dti);
+    }
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      double f[4];
+      f[0] = y[1] * dti - (term[0] - s.loss[0] * y[1]);
+      f[1] = y[2] * dti - (term[1] + s.c12 * y[3] - s.loss[1] * y[2]);
+      f[2] = y[3] * dti - (term[2] + s.c23 * y[4] - s.loss[2] * y[3]);
+      f[3] = y[4] * dti - (term[3] - s.loss[3] * y[4]);
+      f[3] *= d[3];
+      f[2] -= s.c23 * f[3];
+      f[2] *= d[2];
+      f[1] -= s.c12 * f[2];
+      f[1] *= d[1];
+      f[0] *= d[0];
+#pragma unroll
+      for (int k = 3; k >= 0; --k)
+        finish(it, f[k], y[k + 1]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      qq[k + 1] = y[k + 1];
+  }
+  if (!all) {
+    const System system = s;
+    double y[kTracers], ind[kImplicit];
+#pragma unroll
+    for (int k = 0; k < kImplicit; ++k) {
+      ind[k] = production(k);
+      y[k + 1] = start(k + 1);
+    }
+    implicit_steps(system, het, delt, ind, y);
+#pragma unroll
+    for (int k = 1; k < kTracers; ++k)
+      qq[k] = y[k];
+  }
+}
+
+// the same in place
+template <class Het>
+MAM4B_HD void gas_chemistry_cell(double temp, double delt, double photo,
+                                 const double (&extfrc)[kExt], const double (&inv)[kInv],
+                                 const Het &het, double (&qq)[kTracers]) {
+  double q0[kTracers];
+  for (int t = 0; t < kTracers; ++t)
+    q0[t] = qq[t];
+  gas_chemistry_from(temp, delt, photo, extfrc, inv, het, [&](int t) { return q0[t]; }, qq);
 }
 
 }  // namespace gch

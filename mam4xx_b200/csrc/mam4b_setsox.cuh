@@ -47,11 +47,12 @@ MAM4B_HD double net_positive(double yph, double f1, double f2, double f3, double
                              double eco2, double eh2o, double eso4, double so4_fact,
                              double &xph) {
   xph = pow(10.0, -yph);
-  const double eso2 = f1 / (1.0 + f2 * (1.0 + (f3 / xph) * (1.0 + f4 / xph)));
-  const double hso3 = eso2 / xph;
-  const double so3 = hso3 * 2.0 * f4 / xph;
-  const double hco3 = eco2 / xph;
-  const double oh = eh2o / xph;
+  const GuardedDivisor h(xph);
+  const double eso2 = quot(f1, 1.0 + f2 * (1.0 + h.under(f3) * (1.0 + h.under(f4))));
+  const double hso3 = h.under(eso2);
+  const double so3 = h.under(hso3 * 2.0 * f4);
+  const double hco3 = h.under(eco2);
+  const double oh = h.under(eh2o);
   const double so4 = so4_fact * eso4;
   const double neg = oh + hco3 + hso3 + so3 + so4;
   return xph - neg;

@@ -70,24 +70,29 @@ struct StepArgs {
                         // is at least 1/inline_scale of the step finish in pre
 };
 
-// The step runs as a pipeline of six kernels when condensation is on and
-// no diagnostics are asked for: front_kernel runs calcsize, the humidity of
+// The step runs as a pipeline of six kernels when condensation is on:
+// front_kernel runs calcsize, the humidity of
 // water uptake, the subarea set-up and the cloudy subarea, and leaves the
-// clear subarea at its SOA condensation loop in slot-indexed scratch (cloudy
+// clear subarea at its SOA condensation loop in scratch (cloudy
 // cells finish there); mode_kernel and pair_kernel compute water uptake,
 // uptake rates and coagulation coefficients; pre_kernel adds the uptake
 // rates and orders the loops; soa_kernel runs them with per-lane work
 // stealing; post_kernel finishes the queued cells from the hand-off and the
-// loop result. With chemistry, which runs between calcsize's update and the
-// subareas, size_kernel takes the place of front_kernel and pre_chem_kernel
-// does the rest of its work with pre_kernel's. Otherwise full_kernel runs
-// each cell start to end in one thread.
+// loop result. With process tendencies the front stage stores some of them
+// and post_diag_kernel the others. With chemistry, which runs between
+// calcsize's update and the subareas, front_kernel's work is that of
+// chem_size_kernel, chem_cell_kernel and chem_subarea_kernel. Without
+// condensation full_kernel or chem_step_kernel runs each cell start to end in
+// one thread.
 enum { SOA_G = 0, SOA_A = 1, SOA_OPOA = 5, SOA_UPTK = 9, SOA_G0 = 13, SOA_FIELDS = 14 };
 // per-cell values from the first two stages for the later ones:
 // relative humidity for water uptake, H2SO4 diffusivity and mean free path,
 // per-particle H2SO4 uptake rate of each mode
 // and the 12 coagulation coefficients (coag_all_coefs order)
 enum { AUX_RH = 0, AUX_GDIFF = 1, AUX_FPATH = 2, AUX_RATE = 3, AUX_COAG = 7, AUX_FIELDS = 19 };
+// with chemistry, until pair_kernel fills the coagulation rows: cloud-borne SO4
+// of modes 1-3 after cloud chemistry; SOAG and H2SO4 before it and after it
+enum { AUX_CHEM_SO4 = AUX_COAG, AUX_CHEM_GAS = AUX_COAG + 3 };
 // queue counters: long and short loops in the order list, short and long
 // loops handed to the solver, and to the adjoint's
 enum { CNT_TAKEN = 0, CNT_LONG = 1, CNT_SHORT = 2, CNT_TAKEN_ADJ = 3, CNT_TAKEN_LONG = 4,
@@ -467,9 +472,7 @@ __device__ __forceinline__ double relhum_gcm(double qv, double temp, double pmid
 // size outputs and prepares the amicphys inputs: the part of
 // modal_aero_amicphys_intr (mam4_amicphys.hpp:2120-2260) before the
 // subarea loop, with q_pregaschem = q_precldchem = qq and
-// qqcw_precldchem = qqcw. Without WU the wet sizes are read back from the
-// outputs, written by size_kernel and mode_kernel.
-template <bool WU>
+// qqcw_precldchem = qqcw.
 __device__ __forceinline__ void cell_front(const StepArgs &a, const long long c, Front &f) {
   const StepConsts &C = c_k;
   f.temp = __ldg(a.in[MAM4B_IN_T] + c);
@@ -497,22 +500,14 @@ __device__ __forceinline__ void cell_front(const StepArgs &a, const long long c,
   double pt_i[NPOP], pt_c[NPOP];
   calcsize(C, f.ai, f.ac, dt, f.dgn_a, pt_i, pt_c);
   double wetdens_wu[NMODE];
-  if (WU) {
-    double qaerwat[NMODE];
-    water_uptake(C, f.ai, f.qv, f.temp, f.pmid, f.cld, f.dgn_a, f.dgn_awet, qaerwat, wetdens_wu);
+  double qaerwat[NMODE];
+  water_uptake(C, f.ai, f.qv, f.temp, f.pmid, f.cld, f.dgn_a, f.dgn_awet, qaerwat, wetdens_wu);
 #pragma unroll
-    for (int m = 0; m < NMODE; ++m) {
-      a.out[MAM4B_OUT_DGN_A + m][c] = f.dgn_a[m];
-      a.out[MAM4B_OUT_DGN_AWET + m][c] = f.dgn_awet[m];
-      a.out[MAM4B_OUT_WETDENS + m][c] = wetdens_wu[m];
-      a.out[MAM4B_OUT_QAERWAT + m][c] = qaerwat[m];
-    }
-  } else {
-#pragma unroll
-    for (int m = 0; m < NMODE; ++m) {
-      f.dgn_awet[m] = a.out[MAM4B_OUT_DGN_AWET + m][c];
-      wetdens_wu[m] = a.out[MAM4B_OUT_WETDENS + m][c];
-    }
+  for (int m = 0; m < NMODE; ++m) {
+    a.out[MAM4B_OUT_DGN_A + m][c] = f.dgn_a[m];
+    a.out[MAM4B_OUT_DGN_AWET + m][c] = f.dgn_awet[m];
+    a.out[MAM4B_OUT_WETDENS + m][c] = wetdens_wu[m];
+    a.out[MAM4B_OUT_QAERWAT + m][c] = qaerwat[m];
   }
   // calcsize tendencies applied for one step, then amicphys units
 #pragma unroll
@@ -684,7 +679,7 @@ template <bool DIAG>
 __device__ __forceinline__ void cell_step(const StepArgs &a, const long long c) {
   const StepConsts &C = c_k;
   Front f;
-  cell_front<true>(a, c, f);
+  cell_front(a, c, f);
   const double dt = a.dt;
   Diag dgv(a, c);
   Diag *dg = DIAG ? &dgv : nullptr;
@@ -910,35 +905,30 @@ __device__ __forceinline__ void partly_cloudy_setup_chem(const StepArgs &a, cons
 // amicphys tracer index of the gas-chemistry gases O3, H2O2, SO2, DMS
 __device__ __forceinline__ constexpr int chem_gas_i31(int g) { return g < 2 ? g : g + 1; }
 
-// The chemistry of a cell between its front (calcsize, water uptake, the
-// calcsize update) and amicphys: gas-phase chemistry, then aqueous
-// chemistry, on the cell's 31 tracers in vmr; cp receives the states before
-// each, f the state after both (clipped, as amicphys reads it), and the
-// four chemistry gases' tendencies are written.
-__device__ __forceinline__ void run_chemistry(const StepArgs &a, const ChemArgs &ch,
-                                              const long long c, Front &f, ChemPre &cp) {
+// The chemistry of a cell between calcsize and amicphys: gas-phase
+// chemistry of the gases and of the interstitial populations qi(p), then
+// aqueous chemistry, on the cell's 31 tracers in vmr (qq, qqcw). before() is
+// called between the two; it sets the cloud-borne populations. The four
+// chemistry gases' tendencies are written.
+template <class Qi, class Before>
+__device__ __forceinline__ void chemistry(const StepArgs &a, const ChemArgs &ch,
+                                          const long long c, double temp, double pmid, double cld,
+                                          double h2so4, double soag, const Qi &qi,
+                                          double (&qq)[31], double (&qqcw)[31],
+                                          const Before &before) {
   const StepConsts &C = c_k;
   const double dt = a.dt;
   auto CIN = [&](int k) { return __ldg(ch.in + (size_t)k * ch.ld + c); };
-  double qq[31], qqcw[31];
-  double gas_in[4];
+  auto start = [&](int t) {
+    if (t >= 6)
+      return qi(t - 6);
+    if (t == 2 || t == 5)
+      return t == 2 ? h2so4 * C.to_vmr[0] : soag * C.to_vmr[1];
+    return CIN(MAM4B_CHEM_IN_O3 + (t < 2 ? t : t - 1)) * (K::mw_dry_air / K::adv_mass(t));
+  };
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    const int i = chem_gas_i31(g);
-    gas_in[g] = CIN(MAM4B_CHEM_IN_O3 + g);
-    qq[i] = gas_in[g] * (K::mw_dry_air / K::adv_mass(i));
-    qqcw[i] = 0.0;
-  }
-  qq[2] = f.h2so4 * C.to_vmr[0];
-  qq[5] = f.soag * C.to_vmr[1];
-  qqcw[2] = qqcw[5] = 0.0;
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p) {
-    qq[6 + p] = f.qi[p];
-    qqcw[6 + p] = f.qc[p];
-  }
-  cp.g1[0] = dmax(0.0, qq[5]);
-  cp.g1[1] = dmax(0.0, qq[2]);
+  for (int t = 0; t < 6; ++t)
+    qqcw[t] = 0.0;
   {  // gas-phase chemistry
     double ext[gch::kExt], inv[gch::kInv];
 #pragma unroll
@@ -950,21 +940,43 @@ __device__ __forceinline__ void run_chemistry(const StepArgs &a, const ChemArgs 
     const double *het_c = ch.in + (size_t)MAM4B_CHEM_IN_HET * ch.ld + c;
     const size_t ld = ch.ld;
     auto het = [het_c, ld](int t) { return __ldg(het_c + (size_t)t * ld); };
-    gch::gas_chemistry_cell(f.temp, dt, CIN(MAM4B_CHEM_IN_PHOTO), ext, inv, het, qq);
+    gch::gas_chemistry_from(temp, dt, CIN(MAM4B_CHEM_IN_PHOTO), ext, inv, het, start, qq);
   }
-  cp.g2[0] = dmax(0.0, qq[5]);
-  cp.g2[1] = dmax(0.0, qq[2]);
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p) {
-    cp.qi2[p] = dmax(0.0, qq[6 + p]);
-    cp.qc2[p] = dmax(0.0, qqcw[6 + p]);
-  }
+  before();
   {  // cloud chemistry; the total air density is the invariant density of air
     double dso4[3], dh2so4[3];
-    sox::setsox_cell(dt, f.pmid, f.temp, CIN(MAM4B_CHEM_IN_LWC), f.cld,
+    sox::setsox_cell(dt, pmid, temp, CIN(MAM4B_CHEM_IN_LWC), cld,
                      CIN(MAM4B_CHEM_IN_CLDNUM), CIN(MAM4B_CHEM_IN_INV + 0), qq, qqcw, dso4,
                      dh2so4);
   }
+  // the gases amicphys does not map keep the chemistry's result
+  const GuardedDivisor per_dt(dt);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const int i = chem_gas_i31(g);
+    ch.out[(size_t)(MAM4B_CHEM_OUT_TEND + g) * ch.ld + c] = per_dt.under(
+        qq[i] * (K::adv_mass(i) / K::mw_dry_air) - CIN(MAM4B_CHEM_IN_O3 + g));
+  }
+}
+
+// chemistry() of a cell in one thread: cp receives the states before each
+// part, f the state after both (clipped, as amicphys reads it).
+__device__ __forceinline__ void run_chemistry(const StepArgs &a, const ChemArgs &ch,
+                                              const long long c, Front &f, ChemPre &cp) {
+  double qq[31], qqcw[31];
+  cp.g1[0] = f.g_soag;
+  cp.g1[1] = f.g_h2so4;
+  auto qi = [&](int p) { return f.qi[p]; };
+  chemistry(a, ch, c, f.temp, f.pmid, f.cld, f.h2so4, f.soag, qi, qq, qqcw, [&] {
+    cp.g2[0] = dmax(0.0, qq[5]);
+    cp.g2[1] = dmax(0.0, qq[2]);
+#pragma unroll
+    for (int p = 0; p < NPOP; ++p) {
+      qqcw[6 + p] = f.qc[p];
+      cp.qi2[p] = dmax(0.0, qq[6 + p]);
+      cp.qc2[p] = dmax(0.0, qqcw[6 + p]);
+    }
+  });
   f.g_soag = dmax(0.0, qq[5]);
   f.g_h2so4 = dmax(0.0, qq[2]);
 #pragma unroll
@@ -972,13 +984,34 @@ __device__ __forceinline__ void run_chemistry(const StepArgs &a, const ChemArgs 
     f.qi[p] = dmax(0.0, qq[6 + p]);
     f.qc[p] = dmax(0.0, qqcw[6 + p]);
   }
-  // the gases amicphys does not map keep the chemistry's result
+}
+
+// chemistry() of a cell between chem_size_kernel and chem_subarea_kernel, on
+// the populations in the hand-off. Aqueous chemistry changes of them but the
+// cloud-borne SO4; the states before it and after it differ in no other.
+__device__ __forceinline__ void chem_cell(const StepArgs &a, const ChemArgs &ch,
+                                          const long long c) {
+  const size_t n = (size_t)a.ncell;
+  double *hi = a.hand + H_POP * n + c, *hc = a.hand + H_CI * n + c;
+  double *aux = a.aux + c;
+  double qq[31], qqcw[31];
+  auto qi = [&](int p) { return hi[p * n]; };
+  chemistry(a, ch, c, __ldg(a.in[MAM4B_IN_T] + c), __ldg(a.in[MAM4B_IN_P] + c),
+            __ldg(a.in[MAM4B_IN_CLD] + c), __ldg(a.in[MAM4B_IN_H2SO4] + c),
+            __ldg(a.in[MAM4B_IN_SOAG] + c), qi, qq, qqcw, [&] {
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    const int i = chem_gas_i31(g);
-    ch.out[(size_t)(MAM4B_CHEM_OUT_TEND + g) * ch.ld + c] =
-        (qq[i] * (K::adv_mass(i) / K::mw_dry_air) - gas_in[g]) / dt;
-  }
+              for (int p = 0; p < NPOP; ++p) {
+                hi[p * n] = dmax(0.0, qq[6 + p]);
+                qqcw[6 + p] = hc[p * n];
+              }
+              aux[AUX_CHEM_GAS * n] = dmax(0.0, qq[5]);
+              aux[(AUX_CHEM_GAS + 1) * n] = dmax(0.0, qq[2]);
+            });
+  aux[(AUX_CHEM_GAS + 2) * n] = dmax(0.0, qq[5]);
+  aux[(AUX_CHEM_GAS + 3) * n] = dmax(0.0, qq[2]);
+#pragma unroll
+  for (int m = 0; m < 3; ++m)
+    aux[(AUX_CHEM_SO4 + m) * n] = dmax(0.0, qqcw[sox::so4_cw(m)]);
 }
 
 // The per-particle H2SO4 uptake rate of mode M of cell c as the FP64 step
@@ -1045,96 +1078,8 @@ __device__ __forceinline__ void append_loop(const StepArgs &a, long long c, doub
 template <int SOA, class State>
 __device__ __forceinline__ bool soa_pass(State &st, bool fast);
 
-// The pre stage of the step with chemistry: the cell's front (wet sizes
-// from the mode stage), its chemistry (run_chemistry), then cloudy cells
-// finish here; every other cell sets up its clear subarea with the
-// pre-chemistry states (and, when partly cloudy, runs the cloudy one), runs
-// the clear subarea up to the SOA loop and hands the state at that point to
-// the solver and the post kernel. The clear-subarea part runs converged for
-// clear and partly cloudy cells alike. Nothing later needs more, as
-// everything the post kernel reads of the cell's state comes through the
-// hand-off.
-__device__ __forceinline__ void cell_pre_chem(const StepArgs &a, const ChemArgs &ch,
-                                              const long long c) {
-  const StepConsts &C = c_k;
-  Front f;
-  cell_front<false>(a, c, f);
-  ChemPre cp;
-  run_chemistry(a, ch, c, f, cp);
-  const double dt = a.dt;
-  const double fsoag = C.fcvt_soag;
-  if (f.cld > kCloudy) {
-    double o_h2so4, o_soag, oi[NPOP], oc[NPOP];
-    cloudy_cell_chem(a, f, cp, o_h2so4, o_soag, oi, oc);
-    store_outputs(a, c, o_h2so4, o_soag, oi, oc, f.h2so4, f.soag, f.ai, f.ac);
-    return;
-  }
-  const bool partly = !(f.cld < 1.0e-5);
-  Sub s;
-  double rh, oc[NPOP], ci[NPOP], cg[2] = {0.0, 0.0};
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p)
-    ci[p] = 0.0;
-  if (!partly) {
-    load_sub_plain(s, f.qi);
-    s.gas[0] = f.g_soag * fsoag;
-    s.gas[1] = f.g_h2so4 * 1.0;
-    rh = f.relhumgcm;
-#pragma unroll
-    for (int p = 0; p < NPOP; ++p)
-      oc[p] = f.qc[p];
-  } else {
-    double gcl[2];
-    partly_cloudy_setup_chem(a, f, cp, s, gcl, rh, ci, cg, oc);
-  }
-  const double qgas1[2] = {cp.g1[0] * fsoag, cp.g1[1] * 1.0};
-  ClearMid cm;
-  double uptk0[NMODE], rate[NMODE];
-#pragma unroll
-  for (int k = 0; k < NMODE; ++k)
-    rate[k] = a.aux[(AUX_RATE + k) * (size_t)a.ncell + c];
-  clear_prefix<false>(a, dt, f.temp, f.pmid, rate, qgas1, s, cm, uptk0);
-
-  // queue the cell: solver state and hand-off at the start of the SOA loop
-  SoaState st;
-  soa_init(st, (double)(int)(dt / 1), f.temp, f.pmid, s, uptk0);
-  const double first_rate = soa_first_rate(st) * st.dtfull;
-  append_loop(a, c, first_rate);
-  const size_t n = (size_t)a.ncell;
-  double *q = a.soa + c;
-  q[SOA_G * n] = st.g;
-#pragma unroll
-  for (int k = 0; k < NMODE; ++k) {
-    q[(SOA_A + k) * n] = st.a[k];
-    q[(SOA_OPOA + k) * n] = st.opoa[k];
-    q[(SOA_UPTK + k) * n] = st.uptk[k];
-  }
-  q[SOA_G0 * n] = st.g0;
-  double *h = a.hand + c;
-  h[H_GAS1 * n] = s.gas[1];
-  double pop[NPOP];
-  sub_to_pop(s, pop);
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p)
-    h[(H_POP + p) * n] = pop[p];
-#pragma unroll
-  for (int k = 0; k < NMODE; ++k)
-    h[(H_UPTK + k) * n] = cm.uptk1[k];
-  h[H_NETPROD * n] = cm.netprod1;
-  h[H_SV_SO4 * n] = cm.sv_so4_ait;
-  h[H_SV_SOA * n] = cm.sv_soa_ait;
-  h[H_DGN_PC * n] = f.dgn_a[3];
-  h[H_RELHUM * n] = rh;
-  h[H_SOAG0 * n] = s.gas[0];
-  store_cloudborne(a, c, oc, f.ac);
-  if (partly) {
-#pragma unroll
-    for (int p = 0; p < NPOP; ++p)
-      h[(H_CI + p) * n] = ci[p];
-    h[H_CG * n] = cg[0];
-    h[(H_CG + 1) * n] = cg[1];
-  }
-}
+template <int SOA, class State>
+__device__ __forceinline__ bool soa_pass(State &st, bool fast);
 
 // Second half of a cell after its SOA loop: the rest of the clear subarea
 // (H2SO4 update, renaming, nucleation, coagulation with the coefficients of
@@ -1282,7 +1227,7 @@ __device__ __forceinline__ void cell_step_chem(const StepArgs &a, const ChemArgs
                                                const long long c) {
   const StepConsts &C = c_k;
   Front f;
-  cell_front<true>(a, c, f);
+  cell_front(a, c, f);
   const double dt = a.dt;
   ChemPre cp;
   run_chemistry(a, ch, c, f, cp);
@@ -1360,39 +1305,6 @@ __global__ void __launch_bounds__(128) chem_step_kernel(const __grid_constant__ 
 //   front_kernel 255, 128, 96; pre_kernel and post_kernel 255, 168, 128;
 //   soa_kernel 64, 96, 128.
 
-// Stage 1 of the step with chemistry, one thread per cell: calcsize for the
-// dry diameters (an output), the relative humidity of water uptake and the
-// H2SO4 diffusivity and mean free path.
-__device__ __forceinline__ void size_cell(const StepArgs &a, const long long c) {
-  const StepConsts &C = c_k;
-  double ai[NPOP], ac[NPOP];
-#pragma unroll
-  for (int p = 0; p < NPOP; ++p) {
-    ai[p] = __ldg(a.in[MAM4B_IN_AER_I + p] + c);
-    ac[p] = __ldg(a.in[MAM4B_IN_AER_C + p] + c);
-  }
-  double dgn_a[NMODE], pt_i[NPOP], pt_c[NPOP];
-  calcsize(C, ai, ac, a.dt, dgn_a, pt_i, pt_c);
-#pragma unroll
-  for (int m = 0; m < NMODE; ++m)
-    a.out[MAM4B_OUT_DGN_A + m][c] = dgn_a[m];
-  const double temp = __ldg(a.in[MAM4B_IN_T] + c);
-  const double pmid = __ldg(a.in[MAM4B_IN_P] + c);
-  const size_t n = (size_t)a.ncell;
-  a.aux[AUX_RH * n + c] =
-      water_uptake_rh(__ldg(a.in[MAM4B_IN_QV] + c), temp, pmid, __ldg(a.in[MAM4B_IN_CLD] + c));
-  double gd, fp;
-  h2so4_diffusivity(temp, pmid, gd, fp);
-  a.aux[AUX_GDIFF * n + c] = gd;
-  a.aux[AUX_FPATH * n + c] = fp;
-}
-
-__global__ void __launch_bounds__(128, 4) size_kernel(const __grid_constant__ StepArgs a) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < a.ncell)
-    size_cell(a, c);
-}
-
 // Stage 1, one thread per (cell, mode): a block holds two modes of
 // blockDim.x / 2 cells, accumulation and aitken (blockIdx.y 0) or coarse and
 // primary carbon, a warp one of them. Everything up to the SOA loop of a
@@ -1467,6 +1379,15 @@ struct FrontMode {
   double si[7], sc[7], sni, snc;  // cloudy subarea
 };
 
+__device__ __forceinline__ FrontMode front_mode_of(int m) {
+  FrontMode f;
+  f.m = m;
+  f.ns = c_modes.nspec[m];
+  f.s0 = c_modes.spec0[m];
+  f.num = c_modes.numslot[m];
+  return f;
+}
+
 __device__ __forceinline__ void front_load(const StepArgs &a, long long c, double adj_inv,
                                            FrontMode &f, double *x, int stride) {
   const StepConsts &C = c_k;
@@ -1533,19 +1454,16 @@ __device__ __forceinline__ void partition(double q_i, double q_c, double fcldy,
   fy = dy.under(1 - r);
 }
 
-// The mode from calcsize to the SOA loop: its dry diameter (an output), the
-// calcsize update in amicphys units, the clear subarea at the SOA loop (into
-// the hand-off; cells that are not cloudy) and the cloudy subarea before
-// renaming. The aitken mode renames and leaves what
-// moves in x; the accumulation mode takes it in front_out.
-template <bool DIAG>
-__device__ __forceinline__ void front_mode(const StepArgs &a, long long c, double cld,
-                                           double adj_inv, FrontMode &f, double *x, int stride) {
+// The mode's calcsize: its dry diameter (an output) and its populations after
+// the calcsize update, in amicphys units.
+__device__ __forceinline__ void front_sizes(const StepArgs &a, long long c, double cld,
+                                            double adj_inv, FrontMode &f, const double *x,
+                                            int stride, double (&qi)[7], double (&qc)[7],
+                                            double &qni, double &qnc) {
   const StepConsts &C = c_k;
   const int m = f.m;
   const size_t n = (size_t)a.ncell;
   const double dt = a.dt;
-  double qi[7], qc[7], qni, qnc;
   {
     // volume and number of the dry diameter, and their size bounds
     double drv = f.dv_i, num = f.num_i, lo = C.n2v_lo_wide[m], hi = C.n2v_hi_wide[m];
@@ -1613,6 +1531,24 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
     qni = dmax(0.0, dmax(0.0, f.ni + f.pn_i * dt) * C.to_vmr[2 + f.num]);
     qnc = dmax(0.0, dmax(0.0, f.nc + f.pn_c * dt) * C.to_vmr[2 + f.num]);
   }
+}
+
+// The mode's populations split between the subareas: the clear subarea at
+// the SOA loop (into the hand-off; cells that are not cloudy) and the cloudy
+// subarea before renaming. The aitken mode renames and leaves what moves in
+// x; the accumulation mode takes it in front_out. With CHEM the populations
+// are those before cloud chemistry, which changes but the cloud-borne SO4, to
+// so4: the split is that of the values before, renaming counts the change of
+// the aitken mode as growth.
+template <bool DIAG, bool CHEM>
+__device__ __forceinline__ void front_subareas(const StepArgs &a, long long c, double cld,
+                                               FrontMode &f, double *x, int stride,
+                                               const double (&qi)[7], double (&qc)[7],
+                                               const double qni, const double qnc,
+                                               const double so4) {
+  const StepConsts &C = c_k;
+  const int m = f.m;
+  const size_t n = (size_t)a.ncell;
   const bool cloudy = cld > kCloudy, clear = cld < 1.0e-5;
   // subarea factors: clear (number, mass), cloudy interstitial (number,
   // mass); a clear or cloudy cell is its only subarea
@@ -1654,6 +1590,15 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
     a.soa[(SOA_A + m) * n + c] = soa;
     a.soa[(SOA_OPOA + m) * n + c] = 0.0 + (m == 3 ? 0.0 : 0.1) * dmax(pom, 0.0);
   }
+  double grow = 0.0;
+  if (CHEM) {
+    if (m < 2) {
+      grow = dy.under(so4) * 1.0 - dy.under(qc[0]) * 1.0;
+      qc[0] = so4;
+    } else if (m == 2) {
+      qc[2] = so4;
+    }
+  }
   // the cloudy subarea, or the cloud-borne populations of a clear cell
 #pragma unroll
   for (int s = 0; s < 7; ++s) {
@@ -1665,8 +1610,8 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
   f.sni = (qni * fn_y) * 1;
   f.snc = clear ? qnc : dy.under(qnc) * 1;
   if (m == 1 && !clear) {
-    // renaming (rename_subarea<true>, no growth): aitken volumes in AeroId
-    // order SOA, SO4, NaCl, MOM
+    // renaming (rename_subarea<true>): aitken volumes in AeroId order SOA,
+    // SO4, NaCl, MOM
     double xn = 0.0, xv = 0.0;
     bool renamed = false;
     if (a.do_rename) {
@@ -1677,7 +1622,8 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
         ti += f.si[order[k]] * K::mass_2_vol(K::mode_spec(1, order[k]));
         tc += f.sc[order[k]] * K::mass_2_vol(K::mode_spec(1, order[k]));
       }
-      renamed = rename_fractions<true>(C, ti - 0.0, 0.0, tc - 0.0, 0.0, f.sni, f.snc, xn, xv);
+      const double td = CHEM ? grow * K::mass_2_vol(1) : 0.0;
+      renamed = rename_fractions<true>(C, ti - 0.0, 0.0, tc - td, td, f.sni, f.snc, xn, xv);
     }
     double mn_i = 0.0, mn_c = 0.0, mi[4] = {0, 0, 0, 0}, mc[4] = {0, 0, 0, 0};
     if constexpr (DIAG)
@@ -1719,7 +1665,7 @@ __device__ __forceinline__ void front_mode(const StepArgs &a, long long c, doubl
   }
 }
 
-// The process tendencies of renaming in cloud that front_mode did not store
+// The process tendencies of renaming in cloud that front_subareas did not store
 // (it stores the aitken mode's); zero for the cloud-borne populations of a
 // clear cell.
 __device__ __forceinline__ void front_rename_diag(const StepArgs &a, long long c, double cld,
@@ -1819,6 +1765,7 @@ __device__ __forceinline__ void front_uptake(const StepArgs &a, long long c, dou
 // The cell's gases: gases and relative humidity of the clear subarea
 // (clear_prefix) and the equilibrium SOA gas for the SOA loop, or the gas
 // tendencies of a cloudy cell.
+template <bool CHEM>
 __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, double cld) {
   const StepConsts &C = c_k;
   const size_t n = (size_t)a.ncell;
@@ -1832,7 +1779,17 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
       atomicOr(a.flags, MAM4B_FLAG_NONFINITE_INPUT);
   }
   const GuardedDivisor per_dt(a.dt);
-  const double g_h2so4 = dmax(0.0, h2so4 * C.to_vmr[0]), g_soag = dmax(0.0, soag * C.to_vmr[1]);
+  double g_h2so4 = dmax(0.0, h2so4 * C.to_vmr[0]), g_soag = dmax(0.0, soag * C.to_vmr[1]);
+  const double qgas1 = g_h2so4 * 1.0;  // before chemistry
+  // the clear subarea's gases: the grid mean before cloud chemistry
+  double gcl[2] = {g_soag, g_h2so4};
+  if (CHEM) {
+    const double *g = a.aux + AUX_CHEM_GAS * n + c;
+    gcl[0] = g[0];
+    gcl[1] = g[n];
+    g_soag = g[2 * n];
+    g_h2so4 = g[3 * n];
+  }
   if (cld > kCloudy) {
     const double w = 1.0;
     a.out[MAM4B_OUT_TEND + 0][c] =
@@ -1841,18 +1798,22 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
     return;
   }
   double rh = relhum_gcm(qv, temp, pmid);
-  double gcl[2] = {g_soag, g_h2so4};
   double *h = a.hand + c;
+  if (CHEM && cld < 1.0e-5) {
+    gcl[0] = g_soag;
+    gcl[1] = g_h2so4;
+  }
   if (!(cld < 1.0e-5)) {
     // gases: clear keeps the grid mean, cloudy gets the remainder
     const double fcldy = cld, fclea = 1.0 - fcldy;
     const GuardedDivisor dy(fcldy), dc(fclea);
+    const double mean[2] = {g_soag, g_h2so4};
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
-      double gcy = dy.under(gcl[g] - fclea * gcl[g]);
+      double gcy = dy.under(mean[g] - fclea * gcl[g]);
       if (gcy < 0) {
         gcy = 0;
-        gcl[g] = dc.under(gcl[g]);
+        gcl[g] = dc.under(mean[g]);
       }
       h[(H_CG + g) * n] = gcy * fcldy;
     }
@@ -1860,7 +1821,6 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
   }
   const double gas0 = gcl[0] * C.fcvt_soag;
   double gas1 = gcl[1] * 1.0, netprod = 0.0;
-  const double qgas1 = g_h2so4 * 1.0;
   if (a.optaa == 2) {
     netprod = per_dt.under(gas1 - qgas1);
     gas1 = (netprod >= 0) ? qgas1 : 0;
@@ -1881,11 +1841,7 @@ __global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) 
   const int cells = blockDim.x / 2;
   const int k = threadIdx.x % cells;
   double *x = s_x + k;
-  FrontMode f;
-  f.m = 2 * blockIdx.y + threadIdx.x / cells;
-  f.ns = c_modes.nspec[f.m];
-  f.s0 = c_modes.spec0[f.m];
-  f.num = c_modes.numslot[f.m];
+  FrontMode f = front_mode_of(2 * blockIdx.y + threadIdx.x / cells);
   const double adj_inv = safe_denominator(dmax(86400.0, a.dt));
   for (long long c = blockIdx.x * (long long)cells + k; c - k < a.ncell;
        c += gridDim.x * (long long)cells) {
@@ -1896,11 +1852,13 @@ __global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) 
     if (blockIdx.y == 0)
       __syncthreads();
     if (valid) {
-      front_mode<DIAG>(a, c, cld, adj_inv, f, x, cells);
+      double qi[7], qc[7], qni, qnc;
+      front_sizes(a, c, cld, adj_inv, f, x, cells, qi, qc, qni, qnc);
+      front_subareas<DIAG, false>(a, c, cld, f, x, cells, qi, qc, qni, qnc, 0.0);
       if (f.m == 3)
         front_uptake(a, c, cld);
       if (f.m == 0)
-        front_gases(a, c, cld);
+        front_gases<false>(a, c, cld);
     }
     if (blockIdx.y == 0)
       __syncthreads();
@@ -1911,6 +1869,128 @@ __global__ void __maxnreg__(R) front_kernel(const __grid_constant__ StepArgs a) 
     if (blockIdx.y == 0)
       __syncthreads();  // before the next cells' values overwrite these
   }
+}
+
+// The block's cells c = blockIdx.x * blockDim.x + threadIdx.x regrouped so
+// that those with `first` fill warps of their own (cell order kept within
+// each group; blocks of whole warps, at most 256 threads): cells below the
+// crystallisation humidity, whose water uptake needs no Kohler solve, cells
+// with cloud water. wanted: the cell takes part; returns the thread's cell,
+// -1 for none.
+__device__ __forceinline__ long long group_cells(bool wanted, bool first) {
+  __shared__ int s_perm[256];
+  __shared__ unsigned s_cnt[8][2];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
+  first = wanted && first;
+  const unsigned bd = __ballot_sync(0xffffffffu, first);
+  const unsigned bo = __ballot_sync(0xffffffffu, wanted && !first);
+  if (lane == 0) {
+    s_cnt[w][0] = __popc(bd);
+    s_cnt[w][1] = __popc(bo);
+  }
+  __syncthreads();
+  unsigned before_d = 0, before_o = 0, total_d = 0, total = 0;
+  for (int k = 0; k < nw; ++k) {
+    if (k < w) {
+      before_d += s_cnt[k][0];
+      before_o += s_cnt[k][1];
+    }
+    total_d += s_cnt[k][0];
+    total += s_cnt[k][0] + s_cnt[k][1];
+  }
+  if (wanted) {
+    const unsigned below = (1u << lane) - 1u;
+    s_perm[first ? before_d + __popc(bd & below) : total_d + before_o + __popc(bo & below)] = t;
+  }
+  __syncthreads();
+  return (unsigned)t < total ? (long long)blockIdx.x * blockDim.x + s_perm[t] : -1;
+}
+
+// ---- the front of the step with chemistry in three launches: calcsize per
+// (cell, mode), as front_kernel's first part; the chemistry per cell; the
+// subareas per (cell, mode), as its second. The populations pass between
+// them in the hand-off rows that the second fills (interstitial H_POP,
+// cloud-borne H_CI), SO4 after cloud chemistry and the gases in the rows that
+// pair_kernel fills later. In one thread per cell this took 254 registers
+// (7.7 warps per SM) and 1.40 ms for 8,192 x 72 cells, against 0.20, 0.40 and
+// 0.29 ms; the second is bound by the latency of its 100 loads a cell and of
+// the pH's bisection, the others by FP64 latency.
+__global__ void __launch_bounds__(128, 5) chem_size_kernel(const __grid_constant__ StepArgs a) {
+  extern __shared__ double s_x[];
+  const int cells = blockDim.x / 2;
+  const int k = threadIdx.x % cells;
+  double *x = s_x + k;
+  FrontMode f = front_mode_of(2 * blockIdx.y + threadIdx.x / cells);
+  const double adj_inv = safe_denominator(dmax(86400.0, a.dt));
+  const long long c = blockIdx.x * (long long)cells + k;
+  const bool valid = c < a.ncell;
+  if (valid)
+    front_load(a, c, adj_inv, f, x, cells);
+  if (blockIdx.y == 0)
+    __syncthreads();
+  if (!valid)
+    return;
+  const double cld = __ldg(a.in[MAM4B_IN_CLD] + c);
+  double qi[7], qc[7], qni, qnc;
+  front_sizes(a, c, cld, adj_inv, f, x, cells, qi, qc, qni, qnc);
+  const size_t n = (size_t)a.ncell;
+  double *hi = a.hand + H_POP * n + c, *hc = a.hand + H_CI * n + c;
+#pragma unroll
+  for (int s = 0; s < 7; ++s)
+    if (s < f.ns) {
+      hi[(f.s0 + s) * n] = qi[s];
+      hc[(f.s0 + s) * n] = qc[s];
+    }
+  hi[f.num * n] = qni;
+  hc[f.num * n] = qnc;
+  if (f.m == 3)
+    front_uptake(a, c, cld);
+}
+
+// The cells with cloud water, whose pH is found by bisection, fill warps of
+// their own.
+__global__ void __launch_bounds__(256, 2) chem_cell_kernel(const __grid_constant__ StepArgs a,
+                                                           const __grid_constant__ ChemArgs ch) {
+  long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = c < a.ncell;
+  c = group_cells(valid, valid && __ldg(a.in[MAM4B_IN_CLD] + c) > 0.0 &&
+                                   __ldg(ch.in + (size_t)MAM4B_CHEM_IN_LWC * ch.ld + c) > 0.0);
+  if (c >= 0)
+    chem_cell(a, ch, c);
+}
+
+__global__ void __launch_bounds__(128, 5) chem_subarea_kernel(const __grid_constant__ StepArgs a) {
+  extern __shared__ double s_x[];
+  const int cells = blockDim.x / 2;
+  const int k = threadIdx.x % cells;
+  double *x = s_x + k;
+  FrontMode f = front_mode_of(2 * blockIdx.y + threadIdx.x / cells);
+  const long long c = blockIdx.x * (long long)cells + k;
+  const bool valid = c < a.ncell;
+  const double cld = valid ? __ldg(a.in[MAM4B_IN_CLD] + c) : 0.0;
+  if (valid) {
+    const size_t n = (size_t)a.ncell;
+    const double *hi = a.hand + H_POP * n + c, *hc = a.hand + H_CI * n + c;
+    double qi[7], qc[7];
+#pragma unroll
+    for (int s = 0; s < 7; ++s) {
+      f.ac[s] = qi[s] = qc[s] = 0.0;
+      if (s < f.ns) {
+        qi[s] = hi[(f.s0 + s) * n];
+        qc[s] = hc[(f.s0 + s) * n];
+        f.ac[s] = __ldg(a.in[MAM4B_IN_AER_C + f.s0 + s] + c);
+      }
+    }
+    f.nc = __ldg(a.in[MAM4B_IN_AER_C + f.num] + c);
+    const double so4 = f.m < 3 ? a.aux[(AUX_CHEM_SO4 + f.m) * n + c] : 0.0;
+    front_subareas<false, true>(a, c, cld, f, x, cells, qi, qc, hi[f.num * n], hc[f.num * n], so4);
+    if (f.m == 3)
+      front_gases<true>(a, c, cld);
+  }
+  if (blockIdx.y == 0)
+    __syncthreads();
+  if (valid)
+    front_out<false>(a, c, cld, f, x, cells);
 }
 
 // Stage 2, one thread per (cell, mode): water uptake of the mode (Kohler
@@ -1952,46 +2032,12 @@ __device__ __forceinline__ void mode_work(const StepArgs &a, const long long c) 
       uptake_rate_mode(C, M, a.aux[AUX_GDIFF * n + c], a.aux[AUX_FPATH * n + c], dgn_awet);
 }
 
-// The block's cells c = blockIdx.x * blockDim.x + threadIdx.x regrouped so
-// that the cells below the crystallisation humidity, whose water uptake
-// needs no Kohler solve, fill warps of their own (cell order kept within
-// each group; blocks of whole warps, at most 256 threads). wanted: the cell
-// takes part; returns the thread's cell, -1 for none.
-__device__ __forceinline__ long long group_by_humidity(bool wanted, bool dry) {
-  __shared__ int s_perm[256];
-  __shared__ unsigned s_cnt[8][2];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
-  dry = wanted && dry;
-  const unsigned bd = __ballot_sync(0xffffffffu, dry);
-  const unsigned bo = __ballot_sync(0xffffffffu, wanted && !dry);
-  if (lane == 0) {
-    s_cnt[w][0] = __popc(bd);
-    s_cnt[w][1] = __popc(bo);
-  }
-  __syncthreads();
-  unsigned before_d = 0, before_o = 0, total_d = 0, total = 0;
-  for (int k = 0; k < nw; ++k) {
-    if (k < w) {
-      before_d += s_cnt[k][0];
-      before_o += s_cnt[k][1];
-    }
-    total_d += s_cnt[k][0];
-    total += s_cnt[k][0] + s_cnt[k][1];
-  }
-  if (wanted) {
-    const unsigned below = (1u << lane) - 1u;
-    s_perm[dry ? before_d + __popc(bd & below) : total_d + before_o + __popc(bo & below)] = t;
-  }
-  __syncthreads();
-  return (unsigned)t < total ? (long long)blockIdx.x * blockDim.x + s_perm[t] : -1;
-}
-
 template <bool MIXED>
 __global__ void mode_kernel(const __grid_constant__ StepArgs a) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if constexpr (!MIXED) {
     const bool valid = c < a.ncell;
-    c = group_by_humidity(valid, valid && a.aux[AUX_RH * (size_t)a.ncell + c] < K::rh_cryst);
+    c = group_cells(valid, valid && a.aux[AUX_RH * (size_t)a.ncell + c] < K::rh_cryst);
     if (c < 0)
       return;
   }
@@ -2125,14 +2171,6 @@ __global__ void __maxnreg__(R) pre_kernel(const __grid_constant__ StepArgs a) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c < a.ncell)
     pre_cell<MIXED, FUSE>(a, c);
-}
-
-// The pre stage of the step with chemistry (mam4b_step_chem_slab).
-__global__ void __launch_bounds__(128) pre_chem_kernel(const __grid_constant__ StepArgs a,
-                                                       const __grid_constant__ ChemArgs ch) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < a.ncell)
-    cell_pre_chem(a, ch, c);
 }
 
 // (the 128-register cap, 4 blocks of 128 per SM with a few hundred bytes
@@ -3123,7 +3161,7 @@ __global__ void __launch_bounds__(128) adj_mode_kernel(const __grid_constant__ A
   const long long c0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = c0 < a.ncell;
   const long long c =
-      group_by_humidity(valid, valid && a.aux[AUX_RH * (size_t)a.ncell + c0] < K::rh_cryst);
+      group_cells(valid, valid && a.aux[AUX_RH * (size_t)a.ncell + c0] < K::rh_cryst);
   if (c < 0)
     return;
   switch (blockIdx.y) {
@@ -3366,22 +3404,20 @@ __global__ void __launch_bounds__(128, 4) gaschem_kernel(const __grid_constant__
   if (c >= a.ncell)
     return;
   double ext[gch::kExt], inv[gch::kInv], qq[gch::kTracers];
+  // O3 is neither read nor changed
+  auto start = [&](int t) { return t == 0 ? 0.0 : a.qq[(size_t)t * a.ld + c]; };
 #pragma unroll
   for (int e = 0; e < gch::kExt; ++e)
     ext[e] = __ldg(a.extfrc + (size_t)e * a.ld + c);
 #pragma unroll
   for (int i = 0; i < gch::kInv; ++i)
     inv[i] = __ldg(a.inv + (size_t)i * a.ld + c);
-#pragma unroll
-  for (int k = 1; k < gch::kTracers; ++k)
-    qq[k] = a.qq[(size_t)k * a.ld + c];
-  qq[0] = 0.0;  // O3 is neither read nor changed
   // removal rates are read where used (each Newton iteration): after the
   // first read they come from L1, and the solver's registers stay free
   const double *het_c = a.het + c;
   const size_t ld = a.ld;
   auto het = [het_c, ld](int t) { return __ldg(het_c + (size_t)t * ld); };
-  gch::gas_chemistry_cell(__ldg(a.temp + c), a.dt, __ldg(a.photo + c), ext, inv, het, qq);
+  gch::gas_chemistry_from(__ldg(a.temp + c), a.dt, __ldg(a.photo + c), ext, inv, het, start, qq);
 #pragma unroll
   for (int k = 1; k < gch::kTracers; ++k)
     a.qq[(size_t)k * a.ld + c] = qq[k];
@@ -3517,7 +3553,7 @@ __device__ __forceinline__ void optics_mode_work(const OpticsArgs &a, long long 
 template <bool SW>
 __global__ void __launch_bounds__(256) optics_mode_kernel(const __grid_constant__ OpticsArgs a) {
   const long long c0 = modal_cell(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
-  const long long i = group_by_humidity(
+  const long long i = group_cells(
       c0 >= 0, c0 >= 0 && a.scr[OS_RH * (size_t)a.ncell + c0] < K::rh_cryst);
   if (i < 0)
     return;
@@ -4683,7 +4719,8 @@ unsigned grid_for(long long n, int block, int cpt) {
 }
 
 // Stage launchers. Stage order: 0 front (its shape is the tuning's size_*;
-// with chemistry size_kernel), 1 mode, 2 pair, 3 pre, 4 soa, 5 post.
+// with chemistry chem_size_kernel), 1 mode (with chemistry then
+// chem_cell_kernel and chem_subarea_kernel), 2 pair, 3 pre, 4 soa, 5 post.
 template <bool LOOP>
 void launch_front_t(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
   const int cells = t.size_block / 2;
@@ -4773,8 +4810,8 @@ void launch_post(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
 
 // Clears the counters and queues the pipeline kernels on s in the
 // arithmetic of `precision` (mam4b_precision) with launch shape t on a
-// device of `sms` SMs. With ch (FP64 only) the cells' chemistry runs in
-// the pre stage. With ev (7 events), ev[k] is recorded before stage k and
+// device of `sms` SMs. With ch (FP64 only) the cells' chemistry runs after
+// the mode stage. With ev (7 events), ev[k] is recorded before stage k and
 // ev[6] after the last: the per-stage times of mam4b_autotune.
 cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_in,
                               cudaStream_t s, int precision, const ChemArgs *ch, cudaEvent_t *ev,
@@ -4808,24 +4845,24 @@ cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_
       cudaEventRecord(ev[k], s);
   };
   mark(0);
+  const dim3 pairs(grid_for(a.ncell, 64, 1), 2);  // blocks of 64 cells, two modes
+  const size_t xf = (size_t)XF_FIELDS * 64 * sizeof(double);
   if (ch)
-    size_kernel<<<grid_for(a.ncell, 128, 1), 128, 0, s>>>(a);
+    chem_size_kernel<<<pairs, 128, xf, s>>>(a);
   else if (diag)
-    front_kernel<128, false, true><<<dim3(grid_for(a.ncell, 64, 1), 2), 128,
-                                     (size_t)XF_FIELDS * 64 * sizeof(double), s>>>(a);
+    front_kernel<128, false, true><<<pairs, 128, xf, s>>>(a);
   else
     launch_front(t, a, s);
   mark(1);
   launch_mode(t, a, s, mixed);
+  if (ch) {
+    chem_cell_kernel<<<grid_for(a.ncell, 256, 1), 256, 0, s>>>(a, *ch);
+    chem_subarea_kernel<<<pairs, 128, xf, s>>>(a);
+  }
   mark(2);
   launch_pair(t, a, s, mixed);
   mark(3);
-  if (ch) {
-    const int block = 128;
-    pre_chem_kernel<<<(unsigned)((a.ncell + block - 1) / block), block, 0, s>>>(a, *ch);
-  } else {
-    launch_pre(t, a, s, mixed, fuse);
-  }
+  launch_pre(t, a, s, mixed, fuse);
   mark(4);
   launch_soa(t, sms, a, s, precision);
   mark(5);
@@ -4839,7 +4876,7 @@ cudaError_t launch_pipeline_t(const mam4b_tuning &t, int sms, const StepArgs &a_
   mark(6);
   e = cudaGetLastError();
   if (e == cudaSuccess && launches)
-    *launches += a.npass ? 5 : 6;
+    *launches += ch ? 8 : a.npass ? 5 : 6;
   return e;
 }
 
