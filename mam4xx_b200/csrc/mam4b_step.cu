@@ -1912,9 +1912,10 @@ __device__ __forceinline__ long long group_cells(bool wanted, bool first) {
 // them in the hand-off rows that the second fills (interstitial H_POP,
 // cloud-borne H_CI), SO4 after cloud chemistry and the gases in the rows that
 // pair_kernel fills later. In one thread per cell this took 254 registers
-// (7.7 warps per SM) and 1.40 ms for 8,192 x 72 cells, against 0.20, 0.40 and
+// (7.7 warps per SM) and 1.40 ms for 8,192 x 72 cells, against 0.20, 0.35 and
 // 0.29 ms; the second is bound by the latency of its 100 loads a cell and of
-// the pH's bisection, the others by FP64 latency.
+// the pH's bisection (three blocks per SM hide more of it than two, 0.40 ms,
+// or four), the others by FP64 latency.
 __global__ void __launch_bounds__(128, 5) chem_size_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ double s_x[];
   const int cells = blockDim.x / 2;
@@ -1949,7 +1950,7 @@ __global__ void __launch_bounds__(128, 5) chem_size_kernel(const __grid_constant
 
 // The cells with cloud water, whose pH is found by bisection, fill warps of
 // their own.
-__global__ void __launch_bounds__(256, 2) chem_cell_kernel(const __grid_constant__ StepArgs a,
+__global__ void __launch_bounds__(256, 3) chem_cell_kernel(const __grid_constant__ StepArgs a,
                                                            const __grid_constant__ ChemArgs ch) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = c < a.ncell;
