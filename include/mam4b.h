@@ -205,16 +205,17 @@ mam4b_status mam4b_step_slab(mam4b_ctx *ctx, const double *in_slab,
 /*
  * Launch shape of the forward step's kernels (no counterpart in the
  * reference, whose only knob is the Kokkos team size of its column loop,
- * src/validation/validation.hpp:25-30). The step runs as six kernels: size
- * (calcsize, one thread per cell), mode (water uptake, one thread per cell
- * and mode), pair (coagulation coefficients, one thread per cell and mode
- * pair), pre (each cell up to the SOA condensation loop), soa (the
- * persistent loop solver) and post (the rest of each cell). Blocks are 64,
+ * src/validation/validation.hpp:25-30). The step runs as six kernels: the
+ * front (size_*: calcsize and the subareas up to the SOA condensation loop,
+ * one thread per cell and mode), mode (water uptake, one thread per cell and
+ * mode), pair (coagulation coefficients, one thread per cell and mode pair),
+ * pre (uptake rates and the order of the loops), soa (the persistent loop
+ * solver) and post (the rest of each cell). Blocks are 64,
  * 128 or 256 threads (128 or 256 for soa); *_regs selects the compiled
  * register cap of a kernel (size 255, 128 or 96; pre and post 255, 168 or 128;
  * soa 64, 96 or 128; block x regs <= 65536); soa_blocks_per_sm sizes the
  * solver's persistent grid (1..16 blocks per SM); cells_per_thread (1, 2,
- * 4) is how many cells each thread of size and post steps, i.e.
+ * 4) is how many cells each thread of the front and post steps, i.e.
  * 32 x cells_per_thread cells per warp; inline_scale (0 = off, 1, 4, 16,
  * 64): cells whose first SOA sub-step is at least 1/inline_scale of the time
  * step (short loops, predicted from the first sub-step) run their loop and
@@ -233,7 +234,7 @@ typedef struct mam4b_tuning {
 } mam4b_tuning;
 
 /* The built-in shape (size 128/128, mode 128, pair 128, pre 128/255, post
- * 128/128, soa 256/64 x 4 per SM, one cell per thread, no inline loops). */
+ * 128/128, soa 128/128 x 4 per SM, one cell per thread, no inline loops). */
 void mam4b_default_tuning(mam4b_tuning *t);
 
 /* A context starts with the shape in the file named by the environment
