@@ -113,9 +113,16 @@ MAM4B_HD ModeOptics mode_optics(const double (&sp)[7], double logradsurf, double
   o.inv_wet = shortwave ? 1.0 / dmax(wet, 1.e-40) : wet > 1.e-40 ? 1.0 / wet : 1.0;
   o.wet1000 = wet * 1.0e3;
   if (shortwave && dry < 0.0 && dry > -1.e-16)
-    o.wet1000 = 0.0;  // no optical depth, as the reference's early return
+    o.inv_wet = o.wet1000 = 0.0;  // no_optics()
   return o;
 }
+// A shortwave mode that contributes nothing: its dry volume is slightly below
+// zero (what advection leaves of an empty mode), where the reference returns
+// before any arithmetic. The divisor of its refractive index would be the
+// bound 1e-40, the index as large as the volume times 1e40, the fit extrapolated
+// to that beyond exp's range, and infinity times the zero volume not a number.
+// The reciprocal of a volume is zero for no other finite one.
+MAM4B_HD bool no_optics(const ModeOptics &o) { return o.inv_wet == 0.0 && o.wet1000 == 0.0; }
 
 #ifdef __CUDACC__
 // Bracket of ref in an ascending grid of N entries padded with infinity for

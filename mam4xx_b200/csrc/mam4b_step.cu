@@ -3704,6 +3704,11 @@ __global__ void __launch_bounds__(kBandBlock, 3) optics_sw_band_kernel(const __g
         double sum[4] = {0.0, 0.0, 0.0, 0.0};
         band_modes<3, opt::kSwNode>(a, s, c, [&](auto mode, const double (&fit)[3], const ModeIn &x) {
           constexpr int M = decltype(mode)::value;
+          if (opt::no_optics(x.o)) {
+            if (diag)
+              a.scr[(OS_AOD + M) * n + c] = 0.0;
+            return;
+          }
           const double pext = (x.geo == 0.0 ? exp(fit[0]) : x.geo) * x.o.wet1000;
           const double pabs = bound(0.0, pext, fit[1] * x.o.wet1000);
           const double palb = 1.0 - pabs / dmax(pext, 1.e-40);
