@@ -114,6 +114,7 @@ MAM4B_HD bool newton(const System &s, const Het &het, double dti,
       if (fabs(f) > kSmallForcing && !(fabs(f) <= kRelErr * fabs(v)))
         all = false;
     };
+#pragma unroll 1
     for (int k = kImplicit - 1; k >= 4; --k) {
       const double h = het(k + 1);
       double f = y[k + 1] * dti - (inv_term[k] - h * y[k + 1]);
@@ -131,6 +132,7 @@ MAM4B_HD bool newton(const System &s, const Het &het, double dti,
     f[1] -= s.c12 * f[2];
     f[1] *= 1.0 / (s.lin_diag[1] - dti);
     f[0] *= 1.0 / (s.lin_diag[0] - dti);
+#pragma unroll 1
     for (int k = 3; k >= 0; --k)
       finish(k, f[k]);
     if (it > 0 && all)
@@ -144,16 +146,15 @@ MAM4B_HD bool newton(const System &s, const Het &het, double dti,
 // after two converged steps; the interval counts the step as taken either
 // way. ind: independent production.
 template <class Het>
-#ifdef __CUDACC__
-__noinline__
-#endif
 MAM4B_HD void implicit_steps(const System &s, const Het &het, double delt,
                              const double (&ind)[kImplicit], double (&y)[kTracers]) {
   double dt = delt, done = 0.0;
   int cuts = 0, good = 0;
+#pragma unroll 1
   for (int step = 0; step < kStepsMax; ++step) {
     const double dti = 1.0 / dt;
     double inv_term[kImplicit];
+#pragma unroll 1
     for (int k = 0; k < kImplicit; ++k)
       inv_term[k] = dti * y[k + 1] + ind[k];
     const bool ok = newton(s, het, dti, inv_term, y);
@@ -192,12 +193,19 @@ MAM4B_HD void gas_chemistry_from(double temp, double delt, double photo,
   reaction_rates(temp, photo, inv, r);
   System s;
   make_system(r, het, s);
-  const GuardedDivisor air(inv[0]);
+  // the first step's quotients; where they may not be taken that way,
+  // implicit_steps takes the step with the division
+#ifdef __CUDA_ARCH__
+  FastQuotients q;
+#else
+  PlainQuotients q;
+#endif
+  const Divisor air = q.divisor(inv[0]);
   auto production = [&](int k) {
     const int e = ext_of_species(k);
-    return k == 0 ? +r[1] : (e >= 0 ? +air.under(extfrc[e >= 0 ? e : 0]) : 0.0);
+    return k == 0 ? +r[1] : (e >= 0 ? +q.under(air, extfrc[e >= 0 ? e : 0]) : 0.0);
   };
-  const double dti = quot(1.0, delt);
+  const double dti = q.quot(1.0, delt);
   bool all = true;
   auto finish = [&](int it, double f, double &y) {
     double v = y + f;
@@ -211,7 +219,7 @@ MAM4B_HD void gas_chemistry_from(double temp, double delt, double photo,
 #pragma unroll
   for (int k = kImplicit - 1; k >= 4; --k) {
     double y = start(k + 1);
-    const double h = het(k + 1), d = quot(1.0, -(+h) - dti), term = dti * y + production(k);
+    const double h = het(k + 1), d = q.quot(1.0, -(+h) - dti), term = dti * y + production(k);
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
       double f = y * dti - (term - h * y);
@@ -226,7 +234,7 @@ MAM4B_HD void gas_chemistry_from(double temp, double delt, double photo,
     for (int k = 0; k < 4; ++k) {
       y[k + 1] = start(k + 1);
       term[k] = dti * y[k + 1] + production(k);
-      d[k] = quot(1.0, s.lin_diag[k] - dti);
+      d[k] = q.quot(1.0, s.lin_diag[k] - dti);
     }
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
@@ -249,12 +257,13 @@ MAM4B_HD void gas_chemistry_from(double temp, double delt, double photo,
     for (int k = 0; k < 4; ++k)
       qq[k + 1] = y[k + 1];
   }
-  if (!all) {
+  if (!(all && q.ok)) {
     const System system = s;
     double y[kTracers], ind[kImplicit];
 #pragma unroll
     for (int k = 0; k < kImplicit; ++k) {
-      ind[k] = production(k);
+      const int e = ext_of_species(k);
+      ind[k] = k == 0 ? +r[1] : (e >= 0 ? +(extfrc[e >= 0 ? e : 0] / inv[0]) : 0.0);
       y[k + 1] = start(k + 1);
     }
     implicit_steps(system, het, delt, ind, y);

@@ -47,14 +47,17 @@ MAM4B_HD double net_positive(double yph, double f1, double f2, double f3, double
                              double eco2, double eh2o, double eso4, double so4_fact,
                              double &xph) {
   xph = pow(10.0, -yph);
-  const GuardedDivisor h(xph);
-  const double eso2 = quot(f1, 1.0 + f2 * (1.0 + h.under(f3) * (1.0 + h.under(f4))));
-  const double hso3 = h.under(eso2);
-  const double so3 = h.under(hso3 * 2.0 * f4);
-  const double hco3 = h.under(eco2);
-  const double oh = h.under(eh2o);
   const double so4 = so4_fact * eso4;
-  const double neg = oh + hco3 + hso3 + so3 + so4;
+  double neg;
+  with_quotients([&](auto &q) {
+    const Divisor h = q.divisor(xph);
+    const double eso2 = q.quot(f1, 1.0 + f2 * (1.0 + q.under(h, f3) * (1.0 + q.under(h, f4))));
+    const double hso3 = q.under(h, eso2);
+    const double so3 = q.under(h, hso3 * 2.0 * f4);
+    const double hco3 = q.under(h, eco2);
+    const double oh = q.under(h, eh2o);
+    neg = oh + hco3 + hso3 + so3 + so4;
+  });
   return xph - neg;
 }
 

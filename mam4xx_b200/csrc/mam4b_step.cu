@@ -118,14 +118,11 @@ __device__ __forceinline__ constexpr int num_i31(int m) {
 struct Diag {
   const StepArgs &a;
   long long c;
-  GuardedDivisor per_dt, organic, soag;
   bool joined;
-  __device__ __forceinline__ Diag(const StepArgs &a_, long long c_)
-      : a(a_), c(c_), per_dt(a_.dt), organic(K::fcvt_aer(0) * a_.dt), soag(c_k.fcvt_soag * a_.dt),
-        joined(false) {}
+  __device__ __forceinline__ Diag(const StepArgs &a_, long long c_) : a(a_), c(c_), joined(false) {}
   // increment v of a population of species x (number: x < 0)
   __device__ __forceinline__ double rate(int x, double v) const {
-    return (x == 0 || x == 2 ? organic : per_dt).under(0.0 + v);
+    return (0.0 + v) / ((x == 0 || x == 2 ? K::fcvt_aer(0) : 1.0) * a.dt);
   }
   __device__ __forceinline__ void put(int k, int i, double t) const {
     double *d = a.diag[k * 31 + i];
@@ -259,7 +256,7 @@ __device__ __forceinline__ void clear_suffix(const StepArgs &a, double deltat, d
         for (int m = 0; m < NMODE; ++m)
           dcond[x][m] = s.aer[x][m] - cm.sv_all[x][m];
       // gas increment of condensation (mam4_amicphys.hpp:1434-1438)
-      dg->put(0, 5, dg->soag.under(0.0 + (s.gas[0] - (cm.gas_sv[0] + 0.0 * dtsub))) * afrac);
+      dg->put(0, 5, ((0.0 + (s.gas[0] - (cm.gas_sv[0] + 0.0 * dtsub))) / (C.fcvt_soag * a.dt)) * afrac);
       dg->put(0, 2, dg->rate(-1, s.gas[1] - (cm.gas_sv[1] + cm.netprod1 * dtsub)) * afrac);
     }
   }
@@ -416,11 +413,11 @@ __device__ __forceinline__ void store_cloudborne(const StepArgs &a, long long c,
                                                  const double (&oc)[NPOP],
                                                  const double (&ac)[NPOP]) {
   const StepConsts &C = c_k;
-  const GuardedDivisor per_dt(a.dt);
+  const double dt = a.dt;
   double *const *out = a.out;
 #pragma unroll
   for (int p = 0; p < NPOP; ++p)
-    out[MAM4B_OUT_TEND + 27 + p][c] = per_dt.under(oc[p] * C.to_mmr[2 + p] - ac[p]);
+    out[MAM4B_OUT_TEND + 27 + p][c] = (oc[p] * C.to_mmr[2 + p] - ac[p]) / dt;
 }
 
 // Tendencies of the gases and the 25 interstitial populations.
@@ -429,13 +426,13 @@ __device__ __forceinline__ void store_interstitial(const StepArgs &a, long long 
                                                    double h2so4, double soag,
                                                    const double (&ai)[NPOP]) {
   const StepConsts &C = c_k;
-  const GuardedDivisor per_dt(a.dt);
+  const double dt = a.dt;
   double *const *out = a.out;
-  out[MAM4B_OUT_TEND + 0][c] = per_dt.under(o_h2so4 * C.to_mmr[0] - h2so4);
-  out[MAM4B_OUT_TEND + 1][c] = per_dt.under(o_soag * C.to_mmr[1] - soag);
+  out[MAM4B_OUT_TEND + 0][c] = (o_h2so4 * C.to_mmr[0] - h2so4) / dt;
+  out[MAM4B_OUT_TEND + 1][c] = (o_soag * C.to_mmr[1] - soag) / dt;
 #pragma unroll
   for (int p = 0; p < NPOP; ++p)
-    out[MAM4B_OUT_TEND + 2 + p][c] = per_dt.under(oi[p] * C.to_mmr[2 + p] - ai[p]);
+    out[MAM4B_OUT_TEND + 2 + p][c] = (oi[p] * C.to_mmr[2 + p] - ai[p]) / dt;
 }
 
 __device__ __forceinline__ void store_outputs(const StepArgs &a, long long c, double o_h2so4,
@@ -462,10 +459,10 @@ struct Front {
 __device__ __forceinline__ double relhum_gcm(double qv, double temp, double pmid) {
   const double epsqs = 0.018016 / 0.028966;
   const double tc = temp - 273.15;
-  const double ew = 610.94 * exp(quot(17.625 * tc, 234.04 + tc));
+  const double ew = 610.94 * exp(17.625 * tc / (234.04 + tc));
   const double ev_sat = 1.00071 * exp(4.5e-8 * pmid) * ew;
-  const double qv_sat = quot(epsqs * ev_sat, pmid - (1 - epsqs) * ev_sat);
-  return dmax(0.0, dmin(1.0, quot(qv, qv_sat)));
+  const double qv_sat = epsqs * ev_sat / (pmid - (1 - epsqs) * ev_sat);
+  return dmax(0.0, dmin(1.0, qv / qv_sat));
 }
 
 // Loads the cell, checks it, runs calcsize and water uptake, writes the
@@ -950,12 +947,11 @@ __device__ __forceinline__ void chemistry(const StepArgs &a, const ChemArgs &ch,
                      dh2so4);
   }
   // the gases amicphys does not map keep the chemistry's result
-  const GuardedDivisor per_dt(dt);
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const int i = chem_gas_i31(g);
-    ch.out[(size_t)(MAM4B_CHEM_OUT_TEND + g) * ch.ld + c] = per_dt.under(
-        qq[i] * (K::adv_mass(i) / K::mw_dry_air) - CIN(MAM4B_CHEM_IN_O3 + g));
+    ch.out[(size_t)(MAM4B_CHEM_OUT_TEND + g) * ch.ld + c] =
+        (qq[i] * (K::adv_mass(i) / K::mw_dry_air) - CIN(MAM4B_CHEM_IN_O3 + g)) / dt;
   }
 }
 
@@ -1033,7 +1029,7 @@ __device__ double rate_fp64_mode(const StepArgs &a, const long long c) {
                        qaerwat, wetdens);
   return uptake_rate_mode(C, M, a.aux[AUX_GDIFF * n + c], a.aux[AUX_FPATH * n + c], dgn_awet);
 }
-__device__ __noinline__ double rate_fp64(const StepArgs &a, const long long c, int m) {
+__device__ __forceinline__ double rate_fp64(const StepArgs &a, const long long c, int m) {
   switch (m) {
   case 0: return rate_fp64_mode<0>(a, c);
   case 1: return rate_fp64_mode<1>(a, c);
@@ -1107,16 +1103,14 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
   dgv.joined = !(cld < 1.0e-5);
   clear_suffix<DIAG, true>(a, dt, temp, pmid, zm, pblh, relhum, dgn_pc, unused, unused, cm, s,
                            &dgv, dgv.joined ? 1.0 - cld : 1.0, a.aux + AUX_COAG * n + c, n);
-  // recombination (form_gcm_of_gases_and_aerosols_from_subareas)
-  const GuardedDivisor dsoag(C.fcvt_soag);
-  constexpr GuardedDivisor organic = constant_divisor(K::fcvt_aer(0));
-  auto over_fcvt = [&](double v, int x) { return x == 0 || x == 2 ? organic.under(v) : v; };
+  // recombination (form_gcm_of_gases_and_aerosols_from_subareas); the division
+  // itself (with_quotients)
   double o_h2so4, o_soag, oi[NPOP];
   double po[NPOP];
   sub_to_pop(s, po);
   if (cld < 1.0e-5) {
     const double f = 1.0 - 0.0;
-    o_soag = dmax(0.0, 0.0 + dsoag.under(s.gas[0]) * f);
+    o_soag = dmax(0.0, 0.0 + (s.gas[0] / C.fcvt_soag) * f);
     o_h2so4 = dmax(0.0, 0.0 + (s.gas[1] / 1.0) * f);
 #pragma unroll
     for (int m = 0; m < NMODE; ++m) {
@@ -1125,12 +1119,12 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
       for (int x = 0; x < NAER; ++x) {
         const int sl = K::aer_slot(x, m);
         if (sl >= 0)
-          oi[sl] = dmax(0.0, 0.0 + over_fcvt(po[sl], x) * f);
+          oi[sl] = dmax(0.0, 0.0 + (po[sl] / K::fcvt_aer(x)) * f);
       }
     }
   } else {
     const double fclea = 1.0 - cld;
-    o_soag = dmax(0.0, (0.0 + dsoag.under(s.gas[0]) * fclea) + src.cg(0));
+    o_soag = dmax(0.0, (0.0 + (s.gas[0] / C.fcvt_soag) * fclea) + src.cg(0));
     o_h2so4 = dmax(0.0, (0.0 + (s.gas[1] / 1.0) * fclea) + src.cg(1));
 #pragma unroll
     for (int m = 0; m < NMODE; ++m) {
@@ -1140,7 +1134,7 @@ __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c
       for (int x = 0; x < NAER; ++x) {
         const int sl = K::aer_slot(x, m);
         if (sl >= 0)
-          oi[sl] = dmax(0.0, (0.0 + over_fcvt(po[sl], x) * fclea) + src.ci(sl));
+          oi[sl] = dmax(0.0, (0.0 + (po[sl] / K::fcvt_aer(x)) * fclea) + src.ci(sl));
       }
     }
   }
@@ -1442,16 +1436,17 @@ __device__ __forceinline__ void front_load(const StepArgs &a, long long c, doubl
 }
 
 // Partition factor pair of get_partition_factors (mam4_amicphys.hpp:414-449)
-__device__ __forceinline__ void partition(double q_i, double q_c, double fcldy,
-                                          const GuardedDivisor &dy, const GuardedDivisor &dc,
-                                          double fclea, double &fc, double &fy) {
-  const double cldbrn_cldy = dy.under(q_c);
+template <class Quotients>
+__device__ __forceinline__ void partition(Quotients &q, double q_i, double q_c, double fcldy,
+                                          const Divisor &dy, const Divisor &dc, double fclea,
+                                          double &fc, double &fy) {
+  const double cldbrn_cldy = q.under(dy, q_c);
   const double intrst_cldy = dmax(0.0, ((q_i + q_c) - cldbrn_cldy));
-  const double intrst_clea = dc.under(q_i - fcldy * intrst_cldy);
-  double r = quot(dmax(1.e-35, intrst_clea * fclea), dmax(1.e-35, q_i));
+  const double intrst_clea = q.under(dc, q_i - fcldy * intrst_cldy);
+  double r = q.quot(dmax(1.e-35, intrst_clea * fclea), dmax(1.e-35, q_i));
   r = dmax(0.0, dmin(1.0, r));
-  fc = dc.under(r);
-  fy = dy.under(1 - r);
+  fc = q.under(dc, r);
+  fy = q.under(dy, 1 - r);
 }
 
 // The mode's calcsize: its dry diameter (an output) and its populations after
@@ -1553,19 +1548,44 @@ __device__ __forceinline__ void front_subareas(const StepArgs &a, long long c, d
   // subarea factors: clear (number, mass), cloudy interstitial (number,
   // mass); a clear or cloudy cell is its only subarea
   double fn_c = 1.0, fm_c = 1.0, fn_y = 1.0, fm_y = 1.0;
+  // cloud-borne amounts of the cloudy subarea (of the cell when clear): with
+  // CHEM the SO4 after cloud chemistry, whose change counts as growth
   const double fcldy = cld, fclea = 1.0 - fcldy;
-  const GuardedDivisor dy(cloudy ? 1.0 : fcldy);
-  if (!cloudy && !clear) {
-    const GuardedDivisor dc(fclea);
-    double ti = 0.0, tc = 0.0;
+  double ti = 0.0, tc = 0.0, grow = 0.0;
+#pragma unroll
+  for (int s = 0; s < 7; ++s)
+    if (s < f.ns) {
+      ti = ti + qi[s];
+      tc = tc + qc[s];
+    }
+  const double so4_0 = qc[0];
+  if (CHEM) {
+    if (m < 2)
+      qc[0] = so4;
+    else if (m == 2)
+      qc[2] = so4;
+  }
+  if (clear) {
 #pragma unroll
     for (int s = 0; s < 7; ++s)
-      if (s < f.ns) {
-        ti = ti + qi[s];
-        tc = tc + qc[s];
+      f.sc[s] = qc[s];
+    f.snc = qnc;
+  } else {
+    with_quotients([&](auto &q) {
+      const Divisor dy = q.divisor(cloudy ? 1.0 : fcldy);
+      if (!cloudy) {
+        const Divisor dc = q.divisor(fclea);
+        partition(q, qni, qnc, fcldy, dy, dc, fclea, fn_c, fn_y);
+        partition(q, ti, tc, fcldy, dy, dc, fclea, fm_c, fm_y);
       }
-    partition(qni, qnc, fcldy, dy, dc, fclea, fn_c, fn_y);
-    partition(ti, tc, fcldy, dy, dc, fclea, fm_c, fm_y);
+      if (CHEM && m < 2)
+        grow = q.under(dy, so4) * 1.0 - q.under(dy, so4_0) * 1.0;
+#pragma unroll
+      for (int s = 0; s < 7; ++s)
+        if (s < f.ns)
+          f.sc[s] = q.under(dy, qc[s]) * c_modes.fcvt[m][s];
+      f.snc = q.under(dy, qnc) * 1;
+    });
   }
   if (!cloudy) {
     // the clear subarea at the SOA loop (times one in a clear cell)
@@ -1590,25 +1610,12 @@ __device__ __forceinline__ void front_subareas(const StepArgs &a, long long c, d
     a.soa[(SOA_A + m) * n + c] = soa;
     a.soa[(SOA_OPOA + m) * n + c] = 0.0 + (m == 3 ? 0.0 : 0.1) * dmax(pom, 0.0);
   }
-  double grow = 0.0;
-  if (CHEM) {
-    if (m < 2) {
-      grow = dy.under(so4) * 1.0 - dy.under(qc[0]) * 1.0;
-      qc[0] = so4;
-    } else if (m == 2) {
-      qc[2] = so4;
-    }
-  }
-  // the cloudy subarea, or the cloud-borne populations of a clear cell
+  // interstitial amounts of the cloudy subarea
 #pragma unroll
-  for (int s = 0; s < 7; ++s) {
-    if (s >= f.ns)
-      continue;
-    f.si[s] = (qi[s] * fm_y) * c_modes.fcvt[m][s];
-    f.sc[s] = clear ? qc[s] : dy.under(qc[s]) * c_modes.fcvt[m][s];
-  }
+  for (int s = 0; s < 7; ++s)
+    if (s < f.ns)
+      f.si[s] = (qi[s] * fm_y) * c_modes.fcvt[m][s];
   f.sni = (qni * fn_y) * 1;
-  f.snc = clear ? qnc : dy.under(qnc) * 1;
   if (m == 1 && !clear) {
     // renaming (rename_subarea<true>): aitken volumes in AeroId order SOA,
     // SO4, NaCl, MOM
@@ -1710,8 +1717,7 @@ __device__ __forceinline__ void front_out(const StepArgs &a, long long c, double
   const size_t n = (size_t)a.ncell;
   const bool cloudy = cld > kCloudy, clear = cld < 1.0e-5;
   double *h = a.hand + c;
-  const GuardedDivisor per_dt(a.dt);
-  constexpr GuardedDivisor organic = constant_divisor(K::fcvt_aer(0));
+  constexpr Divisor organic = constant_divisor(K::fcvt_aer(0));
   static_assert(K::fcvt_aer(0) == K::fcvt_aer(2), "SOA and POM share their unit factor");
   const double w = cloudy ? 1.0 : cld;
   if constexpr (DIAG)
@@ -1720,35 +1726,38 @@ __device__ __forceinline__ void front_out(const StepArgs &a, long long c, double
     f.sni += x[XF_RN_I * stride];
     f.snc += x[XF_RN_C * stride];
   }
+  with_quotients([&](auto &q) {
+    const Divisor dt = q.divisor(a.dt);
 #pragma unroll
-  for (int s = 0; s <= 7; ++s) {
-    if (s >= f.ns && s < 7)
-      continue;
-    const bool number = s == 7;
-    const int p = number ? f.num : f.s0 + s;
-    double vi = number ? f.sni : f.si[s < 7 ? s : 0], vc = number ? f.snc : f.sc[s < 7 ? s : 0];
-    const double ac = number ? f.nc : f.ac[s < 7 ? s : 0];
-    if (!number && !clear) {
-      const int k = c_modes.common[m][s < 7 ? s : 0];
-      if (m == 0 && k >= 0) {
-        vi += x[(XF_RN_I + 1 + k) * stride];
-        vc += x[(XF_RN_C + 1 + k) * stride];
+    for (int s = 0; s <= 7; ++s) {
+      if (s >= f.ns && s < 7)
+        continue;
+      const bool number = s == 7;
+      const int p = number ? f.num : f.s0 + s;
+      double vi = number ? f.sni : f.si[s < 7 ? s : 0], vc = number ? f.snc : f.sc[s < 7 ? s : 0];
+      const double ac = number ? f.nc : f.ac[s < 7 ? s : 0];
+      if (!number && !clear) {
+        const int k = c_modes.common[m][s < 7 ? s : 0];
+        if (m == 0 && k >= 0) {
+          vi += x[(XF_RN_I + 1 + k) * stride];
+          vc += x[(XF_RN_C + 1 + k) * stride];
+        }
+        if (c_modes.fcvt[m][s < 7 ? s : 0] != 1.0) {
+          vi = q.under(organic, vi);
+          vc = q.under(organic, vc);
+        }
       }
-      if (c_modes.fcvt[m][s < 7 ? s : 0] != 1.0) {
-        vi = organic.under(vi);
-        vc = organic.under(vc);
+      const double oc = clear ? vc : 0.0 + vc * w;
+      a.out[MAM4B_OUT_TEND + 27 + p][c] = q.under(dt, oc * C.to_mmr[2 + p] - ac);
+      if (cloudy) {
+        const double ai = __ldg(a.in[MAM4B_IN_AER_I + p] + c);
+        a.out[MAM4B_OUT_TEND + 2 + p][c] =
+            q.under(dt, dmax(0.0, 0.0 + vi * w) * C.to_mmr[2 + p] - ai);
+      } else if (!clear) {
+        h[(H_CI + p) * n] = vi * w;
       }
     }
-    const double oc = clear ? vc : 0.0 + vc * w;
-    a.out[MAM4B_OUT_TEND + 27 + p][c] = per_dt.under(oc * C.to_mmr[2 + p] - ac);
-    if (cloudy) {
-      const double ai = __ldg(a.in[MAM4B_IN_AER_I + p] + c);
-      a.out[MAM4B_OUT_TEND + 2 + p][c] =
-          per_dt.under(dmax(0.0, 0.0 + vi * w) * C.to_mmr[2 + p] - ai);
-    } else if (!clear) {
-      h[(H_CI + p) * n] = vi * w;
-    }
-  }
+  });
 }
 
 // The cell's scalars for the mode stage: humidity of water uptake, H2SO4
@@ -1778,7 +1787,7 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
     if (!isfinite(chk))
       atomicOr(a.flags, MAM4B_FLAG_NONFINITE_INPUT);
   }
-  const GuardedDivisor per_dt(a.dt);
+  const double dt = a.dt;
   double g_h2so4 = dmax(0.0, h2so4 * C.to_vmr[0]), g_soag = dmax(0.0, soag * C.to_vmr[1]);
   const double qgas1 = g_h2so4 * 1.0;  // before chemistry
   // the clear subarea's gases: the grid mean before cloud chemistry
@@ -1793,8 +1802,8 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
   if (cld > kCloudy) {
     const double w = 1.0;
     a.out[MAM4B_OUT_TEND + 0][c] =
-        per_dt.under(dmax(0.0, 0.0 + g_h2so4 * w) * C.to_mmr[0] - h2so4);
-    a.out[MAM4B_OUT_TEND + 1][c] = per_dt.under(dmax(0.0, 0.0 + g_soag * w) * C.to_mmr[1] - soag);
+        (dmax(0.0, 0.0 + g_h2so4 * w) * C.to_mmr[0] - h2so4) / dt;
+    a.out[MAM4B_OUT_TEND + 1][c] = (dmax(0.0, 0.0 + g_soag * w) * C.to_mmr[1] - soag) / dt;
     return;
   }
   double rh = relhum_gcm(qv, temp, pmid);
@@ -1806,23 +1815,22 @@ __device__ __forceinline__ void front_gases(const StepArgs &a, long long c, doub
   if (!(cld < 1.0e-5)) {
     // gases: clear keeps the grid mean, cloudy gets the remainder
     const double fcldy = cld, fclea = 1.0 - fcldy;
-    const GuardedDivisor dy(fcldy), dc(fclea);
     const double mean[2] = {g_soag, g_h2so4};
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
-      double gcy = dy.under(mean[g] - fclea * gcl[g]);
+      double gcy = (mean[g] - fclea * gcl[g]) / fcldy;
       if (gcy < 0) {
         gcy = 0;
-        gcl[g] = dc.under(mean[g]);
+        gcl[g] = mean[g] / fclea;
       }
       h[(H_CG + g) * n] = gcy * fcldy;
     }
-    rh = bound(0.0, 1.0, dc.under(rh - fcldy));
+    rh = bound(0.0, 1.0, (rh - fcldy) / fclea);
   }
   const double gas0 = gcl[0] * C.fcvt_soag;
   double gas1 = gcl[1] * 1.0, netprod = 0.0;
   if (a.optaa == 2) {
-    netprod = per_dt.under(gas1 - qgas1);
+    netprod = (gas1 - qgas1) / dt;
     gas1 = (netprod >= 0) ? qgas1 : 0;
   }
   h[H_GAS1 * n] = gas1;
@@ -2066,7 +2074,7 @@ __global__ void pair_kernel(const __grid_constant__ StepArgs a) {
   const int sm = coag_src(p), dm = coag_dst(p);
   const double temp = __ldg(a.in[MAM4B_IN_T] + c);
   const double pmid = __ldg(a.in[MAM4B_IN_P] + c);
-  const double aircon = quot(pmid, 8314.46759100000 * temp);
+  const double aircon = pmid / (8314.46759100000 * temp);
   const double dens_s = dmax(1000.0, a.out[MAM4B_OUT_WETDENS + sm][c]);
   const double dens_d = dmax(1000.0, a.out[MAM4B_OUT_WETDENS + dm][c]);
   const CoagTables T = {kCoagBm0ij, kCoagBm3i, kCoagBm0};
@@ -2116,7 +2124,7 @@ __device__ __forceinline__ void pre_cell(const StepArgs &a, const long long c) {
     return;
   }
   const double temp = __ldg(a.in[MAM4B_IN_T] + c), pmid = __ldg(a.in[MAM4B_IN_P] + c);
-  const double aircon = quot(pmid, 8314.46759100000 * temp);
+  const double aircon = pmid / (8314.46759100000 * temp);
   double *h = a.hand + c, *q = a.soa + c;
   SoaState st;
 #pragma unroll
@@ -2288,20 +2296,14 @@ __device__ __forceinline__ void soa_quad_fp64(SoaQuad<double> &st, int base) {
   st.g = dmax(0.0, quot(tot - ta, 1.0 + tb));
   st.a = over_den(a + beta * st.g);
 }
-__device__ __noinline__ void soa_quad_exact(SoaQuad<double> &st, int base) {
-  soa_quad_fp64<false>(st, base);
-}
 // fast: the lane's own parameters allow quot_in_range (soa_params_moderate);
 // one form for the whole warp, whose lanes exchange values
 __device__ __forceinline__ void soa_quad_pass(SoaQuad<double> &st, bool fast, int base,
                                               std::integral_constant<int, 0>) {
-  if (__all_sync(0xffffffffu, fast && zero_or_moderate(st.g) && zero_or_moderate(st.a))) {
+  if (__all_sync(0xffffffffu, fast && zero_or_moderate(st.g) && zero_or_moderate(st.a)))
     soa_quad_fp64<true>(st, base);
-  } else {
-    SoaQuad<double> t = st;
-    soa_quad_exact(t, base);
-    st = t;
-  }
+  else
+    soa_quad_fp64<false>(st, base);
 }
 __device__ __forceinline__ void soa_quad_pass(SoaQuad<double> &st, bool, int base,
                                               std::integral_constant<int, 1>) {
