@@ -1502,8 +1502,7 @@ MAM4B_HD void soa_step_rev(const SoaState &st, SoaBar &b) {
 #ifdef __CUDACC__
 // The reverse of a pass for the solver kernel: W modes per lane, W = 4 the
 // whole loop on one lane, W = 1 one mode on each of four consecutive lanes
-// (values without a mode index are then the same on the four, but for
-// LoopBar::g0, of which each lane holds its mode's part). It linearises the
+// (values without a mode index are then the same on the four). It linearises the
 // pass at the stored state with the division-free arithmetic of
 // f32::soa_step_mx, one reciprocal per denominator; the state is the
 // forward's exactly, so its derivative is computed to rounding (a branch
@@ -1600,7 +1599,7 @@ __device__ __forceinline__ void soa_pass_rev(const LoopState<W> &st, LoopBar<W> 
   }
   const double qr = maxc_rev(0.0, q, sum_modes(b.g, part)) * r1;
   const double tbb = -qr * q;  // cotangent of 1 + tbs; of tot qr, of ta -qr
-  double ab[W], gsb[W], satb[W], delb[W];
+  double ab[W], gsb[W], satb[W], delb[W], g0b[W];
 #pragma unroll
   for (int n = 0; n < W; ++n) {
     const double an = fma(beta[n], gn, a[n]) * rden[n];
@@ -1615,11 +1614,12 @@ __device__ __forceinline__ void soa_pass_rev(const LoopState<W> &st, LoopBar<W> 
     delb[n] = aoa2b * beta[n];
     gsb[n] = -delb[n];
     satb[n] = up ? 0.0 : sat2b;
-    b.g0 += up ? sat2b * rM2[n] : 0.0;
+    g0b[n] = up ? sat2b * rM2[n] : 0.0;
     b.opoa[n] += aoa2b;
     b.uptk[n] += betab * dtcur;
     part[n] = betab * st.uptk[n];
   }
+  b.g0 = sum_modes(b.g0, g0b);
   // sub-step: dtfull - tcur in the last pass, 0.05 / tmpa otherwise
   const double dtcurb = sum_modes(last ? 0.0 : b.tcur, part);
   const double tmpbb = last ? 0.0 : maxc_rev(0.0, tmpb, -(dtcurb * dtcur) * rt);
@@ -1637,7 +1637,7 @@ __device__ __forceinline__ void soa_pass_rev(const LoopState<W> &st, LoopBar<W> 
     gsb[n] += of_g ? 0.0 : maxxc_rev(gs[n], 1.0e-20, M1b);
     // gs = sat a, sat = g0 / dmax(aoa, 1e-20)
     satb[n] += gsb[n] * a[n];
-    b.g0 += satb[n] * rM[n];
+    g0b[n] = satb[n] * rM[n];
     const double aoab = maxxc_rev(aoa[n], 1.0e-20, -satb[n] * sat[n] * rM[n]);
     b.opoa[n] += aoab;
     const bool live = st.uptk[n] > 1.0e-15;
@@ -1645,6 +1645,7 @@ __device__ __forceinline__ void soa_pass_rev(const LoopState<W> &st, LoopBar<W> 
     b.a[n] = live ? maxxc_rev(st.a[n], 0.0, ab[n] + qr) : 0.0;
     b.uptk[n] = live ? b.uptk[n] : 0.0;
   }
+  b.g0 = sum_modes(b.g0, g0b);
   double all_p[NMODE], all_m[NMODE];
   all_modes(phir, all_p);
   all_modes(M1g, all_m);

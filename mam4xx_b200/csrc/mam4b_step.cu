@@ -2892,13 +2892,11 @@ __device__ __forceinline__ void adj_long_loops(const AdjPipeArgs &p, unsigned nl
       if (i < k)
         b = nb;
     }
-    const double g0b[1] = {b.g0};
-    const double g0_sum = adj::sum_modes(0.0, g0b);
     if (valid) {
       double *lb = p.lbar + slot;
       if (mode == 0) {
         lb[LB_G * n] = b.g;
-        lb[LB_G0 * n] = g0_sum;
+        lb[LB_G0 * n] = b.g0;
       }
       lb[(LB_A + mode) * n] = b.a[0];
       lb[(LB_OPOA + mode) * n] = b.opoa[0];
