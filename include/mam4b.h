@@ -466,7 +466,9 @@ mam4b_status mam4b_step_tracers(mam4b_ctx *ctx, const double *q, const double *q
  *                   44-114), mapped to the modes by species type
  *   water_refindex  [16] complex, (real, imaginary) pairs
  *   refrtab, refitab  [4 modes][16][7] and [4][16][10]: the real and
- *                   imaginary refractive-index grids of each table
+ *                   imaginary refractive-index grids of each table (in any
+ *                   order: an index is bracketed from the point before the
+ *                   first one above it)
  *   absp            [4][16][5 coefficients][7][10]: Chebyshev coefficients
  *                   of specific absorption
  * mam4b_optics_lw reads the step's input layout (MAM4B_NIN fields of ld

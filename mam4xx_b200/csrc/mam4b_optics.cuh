@@ -24,9 +24,12 @@ constexpr int kSwDiagBand = 9;  // visible band of the optical-depth diagnostic
 //  * species and water refractive indices as (real, imaginary) pairs, the
 //    species' divided by their densities (a pair then multiplies a mass),
 //    21 species in mode order, then water;
-//  * per mode the two refractive-index grids, padded with infinity to the
-//    lengths of a binary search, and the reciprocals of their spacings (zero
-//    where the reference does not interpolate: the last point, equal points);
+//  * per mode and refractive-index grid its running maximum, padded with
+//    infinity to the length of a binary search (the reference takes the first
+//    point above the index, which is the first running maximum above it in a
+//    grid of any order), and the points with the reciprocals of their spacings
+//    (zero where the reference does not interpolate: the last point, equal
+//    points);
 //  * per mode the coefficient tables, one run of kNode doubles per grid point
 //    with the Chebyshev coefficients of that point next to each other (the
 //    first one halved, as the sum takes it), so that a thread reads a corner
@@ -34,8 +37,8 @@ constexpr int kSwDiagBand = 9;  // visible band of the optical-depth diagnostic
 constexpr int kSpecies = 21, kRePad = 8, kImPad = 16;
 constexpr int kBandWater = 2 * kSpecies;
 constexpr int kBandGrids = kBandWater + 2;
-constexpr int kGridRe = 0, kGridReR = kRePad, kGridIm = 2 * kRePad, kGridImR = 2 * kRePad + kImPad,
-              kGridDoubles = 2 * (kRePad + kImPad);
+constexpr int kSearchRe = 0, kSearchIm = kRePad, kPointsRe = kRePad + kImPad,
+              kPointsIm = kPointsRe + 2 * kPrefr, kGridDoubles = kPointsIm + 2 * kPrefi;
 constexpr int kBandNodes = kBandGrids + NMODE * kGridDoubles;
 // doubles per grid point: longwave absorption; shortwave extinction,
 // absorption, asymmetry. The stride (48 and 144 bytes) spreads points over
@@ -65,14 +68,21 @@ inline void pack_band(const double *specref, int ntypes, const double *water, co
     out[kBandWater + k] = water[2 * b + k];
   for (int m = 0; m < NMODE; ++m) {
     double *g = out + kBandGrids + m * kGridDoubles;
-    auto grid = [&](const double *v, int n, int pad, double *to, double *rcp) {
-      for (int i = 0; i < pad; ++i)
-        to[i] = i < n ? v[i] : HUGE_VAL;
-      for (int i = 0; i + 1 < n; ++i)
-        rcp[i] = fabs(v[i + 1] - v[i]) > 1.e-20 ? 1.0 / (v[i + 1] - v[i]) : 0.0;
+    auto grid = [&](const double *v, int n, int pad, double *search, double *points) {
+      double top = -HUGE_VAL;
+      for (int i = 0; i < pad; ++i) {
+        if (i < n)
+          top = v[i] > top ? v[i] : top;
+        search[i] = i < n ? top : HUGE_VAL;
+      }
+      for (int i = 0; i < n; ++i) {
+        const double dx = i + 1 < n ? v[i + 1] - v[i] : 0.0;
+        points[2 * i] = v[i];
+        points[2 * i + 1] = fabs(dx) > 1.e-20 ? 1.0 / dx : 0.0;
+      }
     };
-    grid(refr + ((size_t)m * bands + b) * kPrefr, kPrefr, kRePad, g + kGridRe, g + kGridReR);
-    grid(refi + ((size_t)m * bands + b) * kPrefi, kPrefi, kImPad, g + kGridIm, g + kGridImR);
+    grid(refr + ((size_t)m * bands + b) * kPrefr, kPrefr, kRePad, g + kSearchRe, g + kPointsRe);
+    grid(refi + ((size_t)m * bands + b) * kPrefi, kPrefi, kImPad, g + kSearchIm, g + kPointsIm);
     double *nd = out + kBandNodes + (size_t)m * kPrefr * kPrefi * node;
     for (int q = 0; q < ntab; ++q)
       for (int c = 0; c < kNcoef; ++c)
@@ -125,21 +135,21 @@ MAM4B_HD ModeOptics mode_optics(const double (&sp)[7], double logradsurf, double
 MAM4B_HD bool no_optics(const ModeOptics &o) { return o.inv_wet == 0.0 && o.wet1000 == 0.0; }
 
 #ifdef __CUDACC__
-// Bracket of ref in an ascending grid of N entries padded with infinity for
-// a binary search: index of the lower point (0 below the grid) and the
-// fraction (compute_factors).
+// Bracket of ref in a grid of N points (pack_band): the point before the
+// first one above ref (0 if that is the first, the last if there is none) and
+// the fraction (compute_factors).
 template <int N>
-__device__ __forceinline__ int bracket(const double *grid, const double *rcp, double ref,
+__device__ __forceinline__ int bracket(const double *search, const double *points, double ref,
                                        double &t) {
   int i = 0;
   if constexpr (N > 8)
-    i = !(ref < grid[7]) ? 8 : 0;
-  i += !(ref < grid[i + 3]) ? 4 : 0;
-  i += !(ref < grid[i + 1]) ? 2 : 0;
-  i += !(ref < grid[i]) ? 1 : 0;  // points not above ref
+    i = !(ref < search[7]) ? 8 : 0;
+  i += !(ref < search[i + 3]) ? 4 : 0;
+  i += !(ref < search[i + 1]) ? 2 : 0;
+  i += !(ref < search[i]) ? 1 : 0;  // running maxima not above ref
   i = max(min(i, N) - 1, 0);
-  const double r = rcp[i];
-  t = r != 0.0 ? (ref - grid[i]) * r : 0.0;
+  const double2 p = reinterpret_cast<const double2 *>(points)[i];
+  t = p.y != 0.0 ? (ref - p.x) * p.y : 0.0;
   return i;
 }
 
@@ -163,8 +173,8 @@ __device__ __forceinline__ void mode_fit(const double *s, const double (&sp)[7],
   im = fabs(im * o.inv_wet);
   const double *g = s + kBandGrids + M * kGridDoubles;
   double t, u;
-  const int i = bracket<kPrefr>(g + kGridRe, g + kGridReR, re, t);
-  const int j = bracket<kPrefi>(g + kGridIm, g + kGridImR, im, u);
+  const int i = bracket<kPrefr>(g + kSearchRe, g + kPointsRe, re, t);
+  const int j = bracket<kPrefi>(g + kSearchIm, g + kPointsIm, im, u);
   const double tu = t * u, tuc = t - tu, tcu = u - tu, tcuc = 1.0 - tuc - u;
   double cheb[kNcoef];
   cheb[0] = 1.0;

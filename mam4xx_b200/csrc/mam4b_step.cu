@@ -3618,7 +3618,8 @@ __device__ __forceinline__ void stage_band(const OpticsArgs &a, int b, double *s
   __syncthreads();
 }
 static_assert(opt::kLwBandDoubles % 2 == 0 && opt::kSwBandDoubles % 2 == 0 &&
-                  opt::kBandNodes % 2 == 0 && opt::kLwNode % 2 == 0 && opt::kSwNode % 2 == 0,
+                  opt::kBandNodes % 2 == 0 && opt::kBandGrids % 2 == 0 &&
+                  opt::kGridDoubles % 2 == 0 && opt::kPointsRe % 2 == 0 && opt::kLwNode % 2 == 0 && opt::kSwNode % 2 == 0,
               "16-byte loads of the staged tables");
 
 // The band is the grid's fastest index: the blocks of one group of cells
