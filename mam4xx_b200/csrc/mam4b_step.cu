@@ -4529,14 +4529,12 @@ struct mam4b_ctx {
   int *d_npass;         // [cap_adj]: passes of each SOA loop
   double *d_optics_lw;  // longwave optics tables (16 packed bands), set by the host
   double *d_optics_sw;  // shortwave optics tables (14 packed bands), set by the host
-  double *d_optics_scr; // optics per-cell values (OS_FIELDS per cell), grown
+  double *d_optics_scr; // optics scratch (optics_scratch), grown
   size_t cap_optics_scr;
   int *d_trop;          // [cap_trop]: tropopause level per column (aero_rad_props)
   size_t cap_trop;
   double *d_diag;       // scratch of the step with process tendencies
   size_t cap_diag;      // its cells
-  int *d_modal;         // [cap_modal + 1]: number and list of cells with modal optics
-  size_t cap_modal;
   double *d_dmx;        // dropmixnuc activation results (DA_FIELDS per cell), grown
   double *d_coag_cc;    // coagulation process: 12 coefficients per cell, grown
   size_t cap_coag_cc;
@@ -5290,7 +5288,6 @@ mam4b_status mam4b_destroy(mam4b_ctx *ctx) {
   cudaFree(ctx->d_optics_scr);
   cudaFree(ctx->d_optics_sw);
   cudaFree(ctx->d_trop);
-  cudaFree(ctx->d_modal);
   cudaFree(ctx->d_diag);
   cudaFree(ctx->d_dmx);
   cudaFree(ctx->d_coag_cc);
@@ -6225,6 +6222,16 @@ static mam4b_status run_optics(mam4b_ctx *ctx, const char *what, bool sw, const 
   return MAM4B_OK;
 }
 
+// Doubles of an optics entry's per-cell values. The number and the list of the
+// cells with modal optics (n + 1 ints) follow them in the same allocation, so
+// that the radiation-facing entries can be captured after any entry of the size.
+static size_t optics_scratch(bool sw, size_t n) {
+  return (size_t)(sw ? OS_FIELDS : OS_LW_FIELDS) * n;
+}
+static unsigned *modal_list(const mam4b_ctx *ctx, bool sw, size_t n) {
+  return reinterpret_cast<unsigned *>(ctx->d_optics_scr + optics_scratch(sw, n));
+}
+
 // Argument checks and scratch of an optics entry; *empty: nothing to do.
 static mam4b_status begin_optics(mam4b_ctx *ctx, const char *what, bool sw, const double *in_slab,
                                  size_t ld, const double *pdeldry, const double *out, int ncol,
@@ -6241,8 +6248,8 @@ static mam4b_status begin_optics(mam4b_ctx *ctx, const char *what, bool sw, cons
   *empty = n == 0;
   if (*empty)
     return MAM4B_OK;
-  const cudaError_t e = grow(&ctx->d_optics_scr, &ctx->cap_optics_scr,
-                             (size_t)(sw ? OS_FIELDS : OS_LW_FIELDS) * n);
+  const cudaError_t e =
+      grow(&ctx->d_optics_scr, &ctx->cap_optics_scr, optics_scratch(sw, n) + (n + 2) / 2);
   return e == cudaSuccess ? MAM4B_OK : set_err(ctx, MAM4B_ERR_CUDA, what, e);
 }
 
@@ -6277,10 +6284,10 @@ mam4b_status mam4b_optics_lw(mam4b_ctx *ctx, const double *in_slab, size_t ld,
 
 // Tropopause levels of the columns into *trop_level (the caller's array, or
 // the context's, which it is then set to) and the list of cells at or below
-// them into the context's.
-static mam4b_status rad_props_tropopause(mam4b_ctx *ctx, const char *what, const double *in_slab,
-                                         size_t ld, const double *pint, int ncol, int nlev,
-                                         int **trop_level, cudaStream_t s) {
+// them (modal_list).
+static mam4b_status rad_props_tropopause(mam4b_ctx *ctx, const char *what, bool sw,
+                                         const double *in_slab, size_t ld, const double *pint,
+                                         int ncol, int nlev, int **trop_level, cudaStream_t s) {
   RadArgs r;
   memset(&r, 0, sizeof(r));
   r.temp = in_slab + (size_t)MAM4B_IN_T * ld;
@@ -6304,17 +6311,8 @@ static mam4b_status rad_props_tropopause(mam4b_ctx *ctx, const char *what, const
   const size_t n = (size_t)ncol * nlev;
   if (n > 0x7fffffffu)
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, what, cudaSuccess);
-  if (ctx->cap_modal < n) {
-    cudaFree(ctx->d_modal);
-    ctx->d_modal = nullptr;
-    ctx->cap_modal = 0;
-    const cudaError_t e = cudaMalloc(&ctx->d_modal, (n + 1) * sizeof(int));
-    if (e != cudaSuccess)
-      return set_err(ctx, MAM4B_ERR_CUDA, what, e);
-    ctx->cap_modal = n;
-  }
-  r.nmodal = reinterpret_cast<unsigned *>(ctx->d_modal);
-  r.modal = ctx->d_modal + 1;
+  r.nmodal = modal_list(ctx, sw, n);
+  r.modal = reinterpret_cast<int *>(r.nmodal + 1);
   const int block = 128, per_block = block / 32;
   const size_t smem = (size_t)per_block * 4 * nlev * sizeof(double);
   if (smem > 48 * 1024)
@@ -6346,14 +6344,14 @@ mam4b_status mam4b_aero_rad_props_sw(mam4b_ctx *ctx, const double *in_slab, size
                                  nlev, dt, s, &empty);
   if (st != MAM4B_OK || empty)
     return st;
-  st = rad_props_tropopause(ctx, what, in_slab, ld, pint, ncol, nlev, &trop_level, s);
+  st = rad_props_tropopause(ctx, what, true, in_slab, ld, pint, ncol, nlev, &trop_level, s);
   if (st != MAM4B_OK)
     return st;
   OpticsArgs v;
   memset(&v, 0, sizeof(v));
   v.trop = trop_level;
-  v.nmodal = reinterpret_cast<unsigned *>(ctx->d_modal);
-  v.modal = ctx->d_modal + 1;
+  v.nmodal = modal_list(ctx, true, (size_t)ncol * nlev);
+  v.modal = reinterpret_cast<const int *>(v.nmodal + 1);
   v.zi = zi;
   v.ext = ext_sw;
   v.ssa = ssa_sw;
@@ -6375,14 +6373,14 @@ mam4b_status mam4b_aero_rad_props_lw(mam4b_ctx *ctx, const double *in_slab, size
                                  nlev, dt, s, &empty);
   if (st != MAM4B_OK || empty)
     return st;
-  st = rad_props_tropopause(ctx, what, in_slab, ld, pint, ncol, nlev, &trop_level, s);
+  st = rad_props_tropopause(ctx, what, false, in_slab, ld, pint, ncol, nlev, &trop_level, s);
   if (st != MAM4B_OK)
     return st;
   OpticsArgs v;
   memset(&v, 0, sizeof(v));
   v.trop = trop_level;
-  v.nmodal = reinterpret_cast<unsigned *>(ctx->d_modal);
-  v.modal = ctx->d_modal + 1;
+  v.nmodal = modal_list(ctx, false, (size_t)ncol * nlev);
+  v.modal = reinterpret_cast<const int *>(v.nmodal + 1);
   v.zi = zi;
   v.ext = ext_lw;
   return run_optics(ctx, what, false, in_slab, ld, pdeldry, odap, nullptr, ncol, nlev, dt, &v, s);
