@@ -222,6 +222,10 @@ mam4b_status mam4b_step_slab(mam4b_ctx *ctx, const double *in_slab,
  * finish inside pre, without the hand-off to the solver and post kernels
  * (FP64 and MAM4B_MIXED; not in the adjoint's forward). Every shape computes
  * the same results bit for bit; only the speed differs.
+ * A context whose shape the caller has not chosen (mam4b_set_tuning,
+ * mam4b_autotune, the file named by MAM4B_TUNING_FILE) runs the solver of
+ * MAM4B_MIXED_FAST with 64 registers and twice the blocks per SM in large
+ * batches, where its shape says 128.
  */
 typedef struct mam4b_tuning {
   int size_block, size_regs;

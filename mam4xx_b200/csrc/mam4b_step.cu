@@ -4510,6 +4510,7 @@ struct mam4b_ctx {
   size_t cap_cells;
   int sms;              // SMs of the device (persistent solver grid = sms x blocks per SM)
   mam4b_tuning tune;    // launch shape of the forward pipeline
+  bool tune_given;      // the caller's: set, autotuned or in MAM4B_TUNING_FILE
   // graph mode (mam4b_set_graph_mode): the pipeline of the last call,
   // captured once and replayed while the call's arguments stay the same
   bool use_graph;
@@ -4781,15 +4782,6 @@ void launch_pre(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s, bool m
 template <int SOA>
 void launch_soa_t(const mam4b_tuning &t, int sms, const StepArgs &a, cudaStream_t s) {
   const unsigned g = (unsigned)(sms * t.soa_blocks_per_sm);
-  // The FP32 loop fits 64 registers, so where a thread runs a loop the SM
-  // holds twice the 128-register shape's blocks (16,384 x 72 uniform cells:
-  // 4.10 ms against 4.65); with four lanes to a loop, in small batches, the
-  // loops are fewer than the lanes and the wider shape is the faster (1,024
-  // columns: 0.70 against 0.88).
-  if (SOA == 2 && t.soa_regs == 128 && !a.quads) {
-    soa_kernel<SOA, 64><<<2 * g, t.soa_block, 0, s>>>(a);
-    return;
-  }
   if (t.soa_regs == 128)
     soa_kernel<SOA, 128><<<g, t.soa_block, 0, s>>>(a);
   else if (t.soa_regs == 96)
@@ -4905,6 +4897,21 @@ void drop_graph(mam4b_ctx *ctx) {
   ctx->graph = nullptr;
 }
 
+// The context's launch shape for a step. One that the caller did not choose was
+// chosen on the FP64 step; the FP32 loop fits 64 registers, so where a thread
+// runs a loop the SM holds twice the 128-register shape's blocks (16,384 x 72
+// uniform cells: 4.10 ms against 4.65). With four lanes to a loop, in small
+// batches, the loops are fewer than the lanes and the wider shape is the
+// faster (1,024 columns: 0.70 against 0.88).
+mam4b_tuning step_shape(const mam4b_ctx *ctx, const StepArgs &a, int precision) {
+  mam4b_tuning t = ctx->tune;
+  if (!ctx->tune_given && precision == MAM4B_MIXED_FAST && !a.quads && t.soa_regs == 128) {
+    t.soa_regs = 64;
+    t.soa_blocks_per_sm *= 2;
+  }
+  return t;
+}
+
 // The forward pipeline with the context's launch shape. With graph mode on
 // and `graph` set (mam4b_step's device entry), the pipeline is captured on
 // a private stream into a CUDA graph, instantiated once and replayed on s;
@@ -4913,11 +4920,12 @@ void drop_graph(mam4b_ctx *ctx) {
 // re-instantiates it when the update is refused.
 cudaError_t launch_pipeline(mam4b_ctx *ctx, const StepArgs &a, cudaStream_t s, int precision,
                             const ChemArgs *ch = nullptr, bool graph = false) {
+  const mam4b_tuning tune = step_shape(ctx, a, precision);
   if (!graph || !ctx->use_graph || ch || !a.do_cond)
-    return launch_pipeline_t(ctx->tune, ctx->sms, a, s, precision, ch, nullptr, &ctx->launches);
+    return launch_pipeline_t(tune, ctx->sms, a, s, precision, ch, nullptr, &ctx->launches);
   const bool same = ctx->graph_exec && memcmp(&ctx->graph_args, &a, sizeof(StepArgs)) == 0 &&
                     ctx->graph_precision == precision &&
-                    memcmp(&ctx->graph_tune, &ctx->tune, sizeof(mam4b_tuning)) == 0;
+                    memcmp(&ctx->graph_tune, &tune, sizeof(mam4b_tuning)) == 0;
   cudaError_t e = cudaSuccess;
   if (!same) {
     if (!ctx->cap_stream)
@@ -4926,7 +4934,7 @@ cudaError_t launch_pipeline(mam4b_ctx *ctx, const StepArgs &a, cudaStream_t s, i
     if (e == cudaSuccess)
       e = cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeRelaxed);
     if (e == cudaSuccess) {
-      const cudaError_t el = launch_pipeline_t(ctx->tune, ctx->sms, a, ctx->cap_stream, precision,
+      const cudaError_t el = launch_pipeline_t(tune, ctx->sms, a, ctx->cap_stream, precision,
                                                nullptr, nullptr, nullptr);
       e = cudaStreamEndCapture(ctx->cap_stream, &g);
       if (e == cudaSuccess)
@@ -4951,7 +4959,7 @@ cudaError_t launch_pipeline(mam4b_ctx *ctx, const StepArgs &a, cudaStream_t s, i
     }
     ctx->graph_args = a;
     ctx->graph_precision = precision;
-    ctx->graph_tune = ctx->tune;
+    ctx->graph_tune = tune;
   }
   e = cudaGraphLaunch(ctx->graph_exec, s);
   if (e == cudaSuccess)
@@ -5126,30 +5134,33 @@ mam4b_status read_tuning_file(const char *path, mam4b_tuning *t, char *device, s
 // The tuning a new context starts with: the file named by MAM4B_TUNING_FILE,
 // else mam4b_tuning.json next to this library, when it exists, parses and
 // was chosen on a device of the current device's name; else the defaults.
-void initial_tuning(int dev, mam4b_tuning *t) {
+// Whether it is the named file's.
+bool initial_tuning(int dev, mam4b_tuning *t) {
   mam4b_default_tuning(t);
   char path[1024] = {0};
   const char *env = getenv("MAM4B_TUNING_FILE");
-  if (env && *env) {
+  const bool named = env && *env;
+  if (named) {
     snprintf(path, sizeof(path), "%s", env);
   } else {
     Dl_info info;
     if (!dladdr((void *)&initial_tuning, &info) || !info.dli_fname)
-      return;
+      return false;
     snprintf(path, sizeof(path), "%s", info.dli_fname);
     char *slash = strrchr(path, '/');
     if (!slash)
-      return;
+      return false;
     snprintf(slash + 1, sizeof(path) - (size_t)(slash + 1 - path), "mam4b_tuning.json");
   }
   mam4b_tuning r;
   char name[256];
   if (read_tuning_file(path, &r, name, sizeof(name)) != MAM4B_OK)
-    return;
+    return false;
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess || strcmp(prop.name, name) != 0)
-    return;
+    return false;
   *t = r;
+  return named;
 }
 }  // namespace
 
@@ -5193,6 +5204,7 @@ mam4b_status mam4b_set_tuning(mam4b_ctx *ctx, const mam4b_tuning *t) {
   if (!ctx || !t || !valid_tuning(*t))
     return set_err(ctx, MAM4B_ERR_INVALID_ARGUMENT, "mam4b_set_tuning", cudaSuccess);
   ctx->tune = *t;
+  ctx->tune_given = true;
   return MAM4B_OK;
 }
 
@@ -5256,7 +5268,7 @@ mam4b_status mam4b_create(mam4b_ctx **out, const mam4b_config *cfg) {
     delete ctx;
     return MAM4B_ERR_CUDA;
   }
-  initial_tuning(ctx->device, &ctx->tune);
+  ctx->tune_given = initial_tuning(ctx->device, &ctx->tune);
   *out = ctx;
   return MAM4B_OK;
 }
@@ -5595,6 +5607,7 @@ mam4b_status mam4b_autotune(mam4b_ctx *ctx, const double *in_slab, const double 
     t_best = t_def;
   }
   ctx->tune = b;
+  ctx->tune_given = true;
   if (best)
     *best = b;
   if (default_ms)
