@@ -188,6 +188,13 @@ mam4b_status mam4b_destroy(mam4b_ctx *ctx);
  * (a cudaStream_t; NULL = legacy default stream). All pointers are device
  * pointers. Replaces AeroProcess<MicrophysicsProcess>::compute_tendencies
  * dispatched over all columns (src/validation/aero_process.hpp:114).
+ *
+ * With process tendencies (out->diag, condensation on) the step keeps scratch
+ * of its own in the context, 776 bytes per cell, beside as much of a step
+ * without them: the first such call allocates it, and one with more cells
+ * frees it, waiting for the device, and allocates it again. Where it cannot be
+ * had (no memory, or `stream` is being captured) the step runs one thread per
+ * cell without scratch, with the same results.
  */
 mam4b_status mam4b_step(mam4b_ctx *ctx, const mam4b_state_view *in,
                         const mam4b_tend_view *out, int ncol, int nlev,
@@ -212,7 +219,8 @@ mam4b_status mam4b_step_slab(mam4b_ctx *ctx, const double *in_slab,
  * pre (uptake rates and the order of the loops), soa (the persistent loop
  * solver) and post (the rest of each cell). Blocks are 64,
  * 128 or 256 threads (128 or 256 for soa); *_regs selects the compiled
- * register cap of a kernel (size 255, 128 or 96; pre and post 255, 168 or 128;
+ * register cap of a kernel (size 255, 128 or 96; pre, whose cap matters with
+ * inline_scale only, and post 255, 168 or 128;
  * soa 64, 96 or 128; block x regs <= 65536); soa_blocks_per_sm sizes the
  * solver's persistent grid (1..16 blocks per SM); cells_per_thread (1, 2,
  * 4) is how many cells each thread of the front and post steps, i.e.

@@ -1,11 +1,13 @@
 // mam4b_step.cu -- sm_100a kernels and the C ABI (include/mam4b.h) of the
 // B200-native MAM4 microphysics step.
 //
-// One thread owns one grid cell for the whole step (calcsize -> water
-// uptake -> amicphys); inputs and outputs are structure-of-arrays fields,
-// so each load/store instruction of a warp touches 32 consecutive doubles.
-// Cells are independent: there is no inter-thread communication and no
-// shared memory; the coagulation correction tables are read through L1.
+// The step (calcsize -> water uptake -> amicphys) is a pipeline of kernels
+// (StepArgs) whose threads own a cell, a mode or a mode pair of a cell, or an
+// SOA loop; inputs, outputs and hand-off are structure-of-arrays fields, so
+// each load/store instruction of a warp touches 32 consecutive doubles. Cells
+// are independent; the two modes of a block of the front stage exchange a few
+// values through shared memory. The coagulation correction tables are read
+// through L1.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 
@@ -59,7 +61,7 @@ struct StepArgs {
   int *done;         // [ncell]: cells that pre_kernel<.., FUSE> finished
   int *order;        // [ncell]: cells in solver order, long loops from the
                      // front, short ones from the back
-  double *aux;       // [AUX_FIELDS][ncell], indexed by cell (size/mode kernels)
+  double *aux;       // [AUX_FIELDS][ncell], indexed by cell (front and mode kernels)
   unsigned *counters;
   int *npass;        // [ncell] or null: passes of each cell's loop (adjoint only)
   int mixed;         // the mode/pair stages ran in FP32 (MAM4B_MIXED, _FAST)
@@ -159,9 +161,9 @@ enum {
   H_SOAG0 = 62,    // SOA gas at the start of the loop (read by the adjoint)
   H_FIELDS = 63
 };
-// (The outgoing cloud-borne grid means are final once pre has set up the
-// subareas: the clear subarea does not change them. pre writes their
-// tendencies itself, store_cloudborne, so they are not handed off.)
+// (The outgoing cloud-borne grid means are final once the subareas are set up:
+// the clear subarea does not change them. front_out writes their tendencies, so
+// they are not handed off.)
 
 // Clear subarea, mam_amicphys_1subarea (mam4_amicphys.hpp:1127-1697), part 1:
 // optaa-2 production split and H2SO4 uptake rates from the per-particle
@@ -1083,20 +1085,15 @@ __device__ __forceinline__ void append_loop(const StepArgs &a, long long c, doub
 template <int SOA, class State>
 __device__ __forceinline__ bool soa_pass(State &st, bool fast);
 
-template <int SOA, class State>
-__device__ __forceinline__ bool soa_pass(State &st, bool fast);
-
 // Second half of a cell after its SOA loop: the rest of the clear subarea
 // (H2SO4 update, renaming, nucleation, coagulation with the coefficients of
 // pair_kernel, aging), recombination with the cloudy subarea's
 // contributions (ci, cg; partly cloudy cells), tendencies of the gases and
-// interstitial populations (the cloud-borne ones are written by the pre
-// stage). s holds the clear subarea with the loop's result, cm the values
-// saved before condensation.
-// src supplies the values read late (src.ci(p), cg(g), ai(p), h2so4(),
-// soag()): from registers in pre's fused path, from the hand-off and the
-// inputs in post_kernel, where reading them only when needed keeps them out
-// of registers during the suffix.
+// interstitial populations (the cloud-borne ones are written by front_out). s
+// holds the clear subarea with the loop's result, cm the values saved before
+// condensation. src supplies the values read late (src.ci(p), cg(g), ai(p),
+// h2so4(), soag()), from the hand-off and the inputs: reading them only when
+// needed keeps them out of registers during the suffix.
 template <bool DIAG, class Src>
 __device__ __forceinline__ void cell_finish(const StepArgs &a, const long long c, double temp,
                                             double pmid, double zm, double cld, double pblh,
@@ -2836,7 +2833,9 @@ __device__ __forceinline__ bool adj_soa_pass(SoaState &st, bool fast) {
 // pass kept in the four lanes' columns: row i of a lane its mode's SOA
 // before pass i, rows kAdjSoaStates + i / 2 of lanes 2 (i % 2) and 2 (i % 2)
 // + 1 g and tcur. The chain of a 1,000-pass loop, forward and reverse, is
-// what bounds a small batch.
+// what bounds a small batch. Where the line lies hardly matters: 32, 64 and 150
+// passes took 7.50, 7.43 and 7.30 ms on 4,096 x 72 cells, 2.92, 2.94 and 2.95
+// on 512 x 72.
 constexpr int kAdjLongPasses = 64;
 template <bool FAST>
 __device__ __forceinline__ void adj_long_loops(const AdjPipeArgs &p, unsigned nlong) {
@@ -3646,7 +3645,9 @@ static_assert(opt::kLwBandDoubles % 2 == 0 && opt::kSwBandDoubles % 2 == 0 &&
 // optics (listed ones with trop, whose warps are then full), then the cells
 // above the tropopause.
 constexpr int kBandBlock = 256;
-constexpr unsigned kBandCellBlocks = 512;  // blocks per band at most
+// blocks per band at most: 256, 512 and 1,024 took 0.974, 0.966 and 0.998 ms
+// longwave and 1.72, 1.69 and 1.69 shortwave on 16,384 x 72 cells
+constexpr unsigned kBandCellBlocks = 512;
 template <class Modal, class Above>
 __device__ __forceinline__ void band_cells(const OpticsArgs &a, bool all, const Modal &modal,
                                            const Above &above) {
@@ -4650,7 +4651,10 @@ cudaError_t ensure_solver_scratch(mam4b_ctx *ctx, size_t ncell) {
 // only start their longest loops early. FP64 step, 1..1,000 sub-steps per
 // cell, four lanes / one lane: 37 k cells 0.78 / 1.34 ms, 295 k cells 2.17 /
 // 2.40 ms, 590 k cells 3.70 / 3.60 ms, 2.4 M cells 13.2 / 10.7 ms. Loops
-// below 150 expected passes end before the long ones either way.
+// below 150 expected passes end before the long ones either way. The host
+// path asks for each of its chunks, which run several at a time; there the
+// copies hide the difference (65,536 x 72 cells, four lanes / one lane in every
+// chunk: 52.45 / 52.45 ms uneven, 53.67 / 53.64 uniform).
 void set_solver(StepArgs &a, int sms) {
   a.quads = a.ncell < 3500LL * sms;
   a.long_steps = a.quads ? 150.0 : 300.0;
@@ -4778,15 +4782,19 @@ void launch_pair(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s, bool 
   else
     pair_kernel<false><<<g, t.pair_block, 0, s>>>(a);
 }
+// Only the form that finishes cells has code for the register caps to shape;
+// the other needs 54 (MIXED 82).
 template <bool MIXED, bool FUSE>
 void launch_pre_t(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s) {
   const unsigned g = grid_for(a.ncell, t.pre_block, 1);
-  if (t.pre_regs == 128)
+  if (!FUSE || t.pre_regs == 128)
     pre_kernel<128, MIXED, FUSE><<<g, t.pre_block, 0, s>>>(a);
-  else if (t.pre_regs == 168)
-    pre_kernel<168, MIXED, FUSE><<<g, t.pre_block, 0, s>>>(a);
-  else
-    pre_kernel<255, MIXED, FUSE><<<g, t.pre_block, 0, s>>>(a);
+  else if constexpr (FUSE) {
+    if (t.pre_regs == 168)
+      pre_kernel<168, MIXED, FUSE><<<g, t.pre_block, 0, s>>>(a);
+    else
+      pre_kernel<255, MIXED, FUSE><<<g, t.pre_block, 0, s>>>(a);
+  }
 }
 // fuse: cells with short SOA loops finish in pre (a.inline_scale > 0)
 void launch_pre(const mam4b_tuning &t, const StepArgs &a, cudaStream_t s, bool mixed = false,
@@ -5476,12 +5484,10 @@ mam4b_status mam4b_autotune(mam4b_ctx *ctx, const double *in_slab, const double 
     t = d;
     t.pair_block = b;
     cand[2].push_back(t);
+    t = d;
+    t.pre_block = b;
+    cand[3].push_back(t);
     for (int r : {255, 168, 128}) {
-      t = d;
-      t.pre_block = b;
-      t.pre_regs = r;
-      if (valid_tuning(t))
-        cand[3].push_back(t);
       t = d;
       t.post_block = b;
       t.post_regs = r;
@@ -5515,9 +5521,7 @@ mam4b_status mam4b_autotune(mam4b_ctx *ctx, const double *in_slab, const double 
     t.size_regs = c0.size_regs;
     t.mode_block = cand[1][i % cand[1].size()].mode_block;
     t.pair_block = cand[2][i % cand[2].size()].pair_block;
-    const mam4b_tuning &c3 = cand[3][i % cand[3].size()];
-    t.pre_block = c3.pre_block;
-    t.pre_regs = c3.pre_regs;
+    t.pre_block = cand[3][i % cand[3].size()].pre_block;
     const mam4b_tuning &c4 = cand[4][i % cand[4].size()];
     t.soa_block = c4.soa_block;
     t.soa_regs = c4.soa_regs;
@@ -5567,7 +5571,6 @@ mam4b_status mam4b_autotune(mam4b_ctx *ctx, const double *in_slab, const double 
     b.mode_block = cand[1][arg[1]].mode_block;
     b.pair_block = cand[2][arg[2]].pair_block;
     b.pre_block = cand[3][arg[3]].pre_block;
-    b.pre_regs = cand[3][arg[3]].pre_regs;
     b.soa_block = cand[4][arg[4]].soa_block;
     b.soa_regs = cand[4][arg[4]].soa_regs;
     b.soa_blocks_per_sm = cand[4][arg[4]].soa_blocks_per_sm;
