@@ -1934,8 +1934,8 @@ __device__ __forceinline__ long long group_cells(bool wanted, bool first) {
 // them in the hand-off rows that the second fills (interstitial H_POP,
 // cloud-borne H_CI), SO4 after cloud chemistry and the gases in the rows that
 // pair_kernel fills later. In one thread per cell this took 254 registers
-// (7.7 warps per SM) and 1.40 ms for 8,192 x 72 cells, against 0.20, 0.35 and
-// 0.29 ms; the second is bound by the latency of its 100 loads a cell and of
+// (7.7 warps per SM) and 1.40 ms for 8,192 x 72 cells, against 0.20, 0.34 and
+// 0.25 ms; the second is bound by the latency of its 100 loads a cell and of
 // the pH's bisection (three blocks per SM hide more of it than two, 0.40 ms,
 // or four), the others by FP64 latency.
 __global__ void __launch_bounds__(128, 5) chem_size_kernel(const __grid_constant__ StepArgs a) {
@@ -3696,7 +3696,7 @@ __global__ void __launch_bounds__(kBandBlock, 3) optics_band_kernel(const __grid
 // coefficient and corner, linear search, species volumes and two divisions
 // again in every band) 920 instructions per mode and band: the shortwave
 // entry of 16,384 x 72 cells took 3.84 ms (this kernel 2.9) and takes 1.67,
-// the longwave one 2.78 and 0.95.
+// the longwave one 2.78 and 0.93.
 __global__ void __launch_bounds__(kBandBlock, 3) optics_sw_band_kernel(const __grid_constant__ OpticsArgs a) {
   __shared__ __align__(16) double s[opt::kSwBandDoubles];
   const int b = blockIdx.x;
