@@ -5383,7 +5383,7 @@ mam4b_status mam4b_step(mam4b_ctx *ctx, const mam4b_state_view *in, const mam4b_
     return set_err(ctx, MAM4B_ERR_NOT_SUPPORTED,
                    "mam4b_step: process diagnostics are FP64 only", cudaSuccess);
   // with process tendencies, in the pipeline's stages where their scratch can
-  // be had (1,024 x 72 cells: 0.27 ms against 0.78 ms start to end in one
+  // be had (1,024 x 72 cells: 0.28 ms against 0.78 ms start to end in one
   // thread per cell, which waits for instructions and spilled registers)
   if (diag && set_diag_scratch(ctx, a, s)) {
     e = launch_pipeline_t(ctx->tune, ctx->sms, a, s, precision, nullptr, nullptr, &ctx->launches,
